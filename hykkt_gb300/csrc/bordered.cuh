@@ -1,0 +1,1059 @@
+// Bordered layout of the factor and its solves (sm_103a, FP64 results).
+//
+// The columns of the permuted Hgamma near the roots of its elimination tree
+// form the border, the subtrees below them the blocks (at most kBlkRows rows
+// each with their border rows).  With A = [F B^T; B S], F block diagonal over
+// the blocks:
+//   per block   X = L^-1 of F = L L^T, E = B F^-1, and the update -E B^T
+//   border      X = L^-1, dense, of S - sum E B^T = L L^T
+//   solve       y_F = X b_F,  x_S = X^T (X (b_S - E b_F)),  x_F = X^T y_F - E^T x_S
+// so that a solve is a few dense phases whatever the depth of the tree (the
+// task-queue kernels pay 5-9 us per tree level and direction).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "kernels.cuh"
+
+namespace hykkt {
+
+// ---------------------------------------------------------------------------
+// Blocks: Cholesky of a block's front [F; B] over its own columns together
+// with the inverse of the factor, one CTA each, in place in the packed lower
+// triangle in shared memory.  Pivot p with v = A(:,p) / sqrt(a_pp) below it
+// and w = A(p,:) / sqrt(a_pp) left of it (row p of X = L^-1 so far):
+//   A_ij -= v_i v_j  (i >= j > p),   A_ij -= v_i w_j  (j < p)
+//   A_pj = w_j,  A_ip = -v_i / sqrt(a_pp)
+// so that F ends as X, B as -E and the border part as the Schur update.  A block's columns are sparse (they come from a subtree), so only
+// the nonzeros of v and w are visited.  Bounded by the pivots' latency.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int packed_lower(int i, int j) { return i * (i + 1) / 2 + j; }
+
+__global__ void __launch_bounds__(256) k_block_sweep(DevPlan d, DevBorder bd, int blk0) {
+  extern __shared__ double bsm[];
+  __shared__ int wcnt[8];
+  __shared__ double sroot;
+  const int blk = blk0 + blockIdx.x;
+  const int c0 = bd.blk_rp[blk], nt = bd.blk_rp[blk + 1] - c0;
+  const int R = bd.blk_rrp[blk + 1] - bd.blk_rrp[blk];
+  const int N = nt + R, tot = N * (N + 1) / 2;
+  double* A = bsm;
+  double* val = A + tot;                                    // nonzeros of the pivot's row and column
+  short* idx = reinterpret_cast<short*>(val + blockDim.x);  // their positions, ascending
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  for (int i = tid; i < tot; i += blockDim.x) A[i] = 0.0;
+  __syncthreads();
+  for (int e = bd.ent_rp[blk] + tid; e < bd.ent_rp[blk + 1]; e += blockDim.x) A[bd.ent_pos[e]] = d.lp_v[bd.ent_q[e]];
+  __syncthreads();
+  for (int p = 0; p < nt; ++p) {
+    // N <= blockDim.x: one entry of the pivot's row or column per thread
+    double v = 0.0;
+    if (tid < N && tid != p) v = tid > p ? A[packed_lower(tid, p)] : A[packed_lower(p, tid)];
+    const bool nz = v != 0.0;
+    const unsigned m = __ballot_sync(0xffffffffu, nz);
+    if (lane == 0) wcnt[warp] = __popc(m);
+    if (tid == 0) {
+      const double dp = A[packed_lower(p, p)];
+      note_pivot(d, bd.blk_col[c0 + p], dp);
+      sroot = rsqrt(dp);
+    }
+    __syncthreads();
+    int base = 0, nnz = 0;
+    for (int w = 0; w < nwarp; ++w) {
+      if (w < warp) base += wcnt[w];
+      nnz += wcnt[w];
+    }
+    const double rs = sroot;
+    if (nz) {
+      const int at = base + __popc(m & ((1u << lane) - 1));
+      val[at] = v * rs;
+      idx[at] = (short)tid;
+    }
+    __syncthreads();
+    for (int a = warp; a < nnz; a += nwarp) {
+      const int i = idx[a];
+      const double u = val[a];
+      if (i < p) {
+        if (lane == 0) A[packed_lower(p, i)] = u;
+        continue;
+      }
+      for (int b = lane; b <= a; b += 32) {
+        double* g = &A[packed_lower(i, idx[b])];
+        *g = fma(-u, val[b], *g);
+      }
+      if (lane == 0) A[packed_lower(i, p)] = -u * rs;
+    }
+    if (tid == 0) A[packed_lower(p, p)] = rs;
+    __syncthreads();
+  }
+  // [X; E] in panels of 64 rows and [-E^T X^T] in panels of 64 block columns,
+  // column after column of the panel, zeros past the last row
+  double* GE = bd.ge + bd.ge_off[blk];
+  double* ET = bd.et + bd.et_off[blk];
+  for (int e = tid; e < (N + 63) / 64 * 64 * nt; e += blockDim.x) {
+    const int i = e / (64 * nt) * 64 + e % 64, t = e / 64 % nt;
+    double a = 0.0;
+    if (i < nt) a = i >= t ? A[packed_lower(i, t)] : 0.0;
+    else if (i < N) a = -A[packed_lower(i, t)];
+    GE[e] = a;
+  }
+  for (int e = tid; e < (nt + 63) / 64 * 64 * N; e += blockDim.x) {
+    const int t = e / (64 * N) * 64 + e % 64, i = e / 64 % N;  // entry i: border rows, then own
+    double a = 0.0;
+    if (t < nt) a = i < R ? A[packed_lower(nt + i, t)] : i - R >= t ? A[packed_lower(i - R, t)] : 0.0;
+    ET[e] = a;
+  }
+  double* C = bd.cb + bd.c_off[blk];  // the border update, packed lower R x R
+  for (int i = warp; i < R; i += nwarp)
+    for (int j = lane; j <= i; j += 32) C[packed_lower(i, j)] = A[packed_lower(nt + i, nt + j)];
+}
+
+// The border's lower triangle: one thread per entry that has an original
+// value or block updates (block order: deterministic); zeroed before.
+__global__ void k_border_assemble(DevPlan d, DevBorder bd) {
+  const int stride = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int t = tid; t < bd.nasm; t += stride) {
+    double a = bd.asm_src[t] >= 0 ? d.lp_v[bd.asm_src[t]] : 0.0;
+    for (int p = bd.asm_rp[t]; p < bd.asm_rp[t + 1]; ++p) a += bd.cb[bd.asm_pos[p]];
+    bd.W[(int64_t)bd.asm_col[t] * bd.ld + bd.asm_row[t]] = a;
+  }
+  for (int j = bd.k + tid; j < bd.npan * kBorderPanel; j += stride) bd.W[(int64_t)j * bd.ld + j] = 1.0;  // padding
+}
+
+// ---------------------------------------------------------------------------
+// Border: Cholesky and the inverse of the factor in one sweep, 32 columns at
+// a time, in place: after panel p the rows up to it hold X = L^-1, the rows
+// below the partial products of X left of the panel and the Schur complement
+// right of it.  With L L^T the panel's diagonal block, per panel:
+//   k_border_panel   Y = V L^-T for the rows below (V the panel's columns) and
+//                    Y = L^-1 V for the columns left of it (V its rows of X),
+//                    Y in digits for the update; in place X_p = Y to the left,
+//                    L^-1 on the diagonal, -Y L^-1 below
+//   k_border_update  A -= Y Y^T on the rows below the panel, all columns
+// (An explicit W = X^T X would save a phase of every solve, but its products
+// cancel: the first residual of a 1,000-bus solve rose from 2e-6 to 5e-4.)
+// The update is the cost (2/3 k^3 flops in all).  FP64 runs at 1.25 TFLOP/s on
+// this chip and the bf16 tensor cores at 1,900, so the products are made of
+// exact bf16 pieces: every row of Y is scaled by its power of two and cut
+// into seven signed 8-bit digits (55 bits), digit products are integers that
+// FP32 accumulates without rounding (at most 7 * 32 * 2^14 < 2^24), and the
+// digit products of equal weight share one accumulator (Ootomo, Ozaki and
+// Yokota, "DGEMM on integer matrix multiplication unit", 2024, here on
+// tcgen05 with bf16 operands).  Weights below 2^-62 of the largest product
+// are left out; a 32-term FP64 FMA chain rounds at 2^-53 each.
+// ---------------------------------------------------------------------------
+constexpr int kDigits = 7;
+constexpr int kRowBlock = 128;                                   // rows of a digit block and of an update tile
+constexpr int kPlaneBytes = kRowBlock * kBorderPanel * 2;         // one digit of one row block
+constexpr int kDigitBlockBytes = kDigits * kPlaneBytes;
+constexpr int kTileCols = 32;                                     // columns of an update tile
+constexpr int kAccs = 8;                                          // digit weights kept
+constexpr int kTmemCols = kAccs * kTileCols;
+constexpr int kBPlaneBytes = kTileCols * kBorderPanel * 2;
+// two CTAs per SM (their accumulators fill the 512 tensor-memory columns):
+// more than a third of the SM's shared memory keeps a third one out
+constexpr int kUpdateSmem = 78 * 1024;
+static_assert(kDigitBlockBytes + kDigits * kBPlaneBytes + 1024 <= kUpdateSmem, "update tiles must fit");
+constexpr int kExpZero = -100000, kExpNan = 1000000;  // row exponents of rows that are zero / not finite
+constexpr unsigned kMbarLimit = 1u << 22;
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+
+// Bounded wait on an mbarrier phase; false (and the solve's timeout flag) when
+// the limit runs out.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, DevScalars* sc) {
+  for (unsigned it = 0; it < kMbarLimit; ++it)
+    if (mbar_test(bar, parity)) return true;
+  atomicOr(&sc->solve_flags, 1);
+  return false;
+}
+
+// Test hook (dbg_unsatisfiable, 0 in use): asks for a phase that never
+// completes, with the plan's poll limit, as the task-queue waits do.
+__device__ __forceinline__ void mbar_wait_hook(uint32_t bar, uint32_t parity, const DevPlan& d) {
+  volatile const int* flags = &d.sc->solve_flags;
+  for (unsigned it = 0; !mbar_test(bar, parity); ++it) {
+    if (it > d.spin_limit || (*flags & 1)) {
+      atomicOr(&d.sc->solve_flags, 1);
+      break;
+    }
+    __nanosleep(64);
+  }
+}
+
+// K-major shared-memory operand without swizzle: 8-row x 16-byte core
+// matrices of 128 bytes, 128 bytes apart along K, 512 along the rows.
+__device__ __forceinline__ uint64_t operand_desc(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) | (1ull << 46);
+}
+
+// power of two 2^e (0 below the normal range; NaN for the not-finite mark)
+__device__ __forceinline__ double pow2_or_nan(int e) {
+  if (e > 1023) return __longlong_as_double(0x7ff8000000000000ll);
+  return e < -1022 ? 0.0 : __longlong_as_double((long long)(e + 1023) << 52);
+}
+
+// L D L^T of a 32 x 32 diagonal block (lower triangle in A, row stride 33) by
+// 256 threads: M = L^-1 (unit lower), the reciprocals of D and of its roots.
+// Gauss elimination applied to [A I], two barriers per pivot.  It runs in the
+// update kernel's first tile (the one that completes the block), beside the
+// other tiles, so that the panel kernel starts with M ready.
+__device__ void pivot_block(DevPlan& d, const DevBorder& bd, int panel, double* A, double* M) {
+  constexpr int n = kBorderPanel, ld = n + 1;
+  __shared__ double sinv[n];
+  const int tid = threadIdx.x;
+  for (int e = tid; e < n * n; e += 256) M[(e / n) * ld + e % n] = e / n == e % n ? 1.0 : 0.0;
+  __syncthreads();
+  for (int k = 0; k < n; ++k) {
+    if (tid == 0) {
+      const double p = A[k * ld + k];
+      const int col = panel * n + k;
+      if (col < bd.k) note_pivot(d, bd.bcol[col], p);
+      sinv[k] = 1.0 / p;
+    }
+    __syncthreads();
+    const double inv = sinv[k];
+    // row i > k: columns j in (k, i] of A and j <= k of M; eight threads per row
+    const int i = tid >> 3, part = tid & 7;
+    if (i > k) {
+      const double l = A[i * ld + k] * inv;
+      for (int j = part; j <= i; j += 8) {
+        if (j > k) A[i * ld + j] = fma(-l, A[j * ld + k], A[i * ld + j]);
+        else M[i * ld + j] = fma(-l, M[k * ld + j], M[i * ld + j]);
+      }
+    }
+    __syncthreads();
+  }
+  double* out = bd.piv;
+  for (int e = tid; e < n * n; e += 256) out[e] = M[(e / n) * ld + e % n];
+  if (tid < n) {
+    out[n * n + tid] = sinv[tid];
+    out[n * n + n + tid] = sqrt(sinv[tid]);
+  }
+}
+
+__global__ void __launch_bounds__(256) k_border_pivot0(DevPlan d, DevBorder bd) {
+  constexpr int n = kBorderPanel, ld = n + 1;
+  __shared__ double A[n * ld], M[n * ld];
+  for (int e = threadIdx.x; e < n * n; e += 256) A[(e % n) * ld + e / n] = bd.W[(int64_t)(e / n) * bd.ld + e % n];
+  __syncthreads();
+  pivot_block(d, bd, 0, A, M);
+}
+
+// One CTA per group of eight rows, a warp for two of them: with lane t the
+// dot products of row a's index t and of row b's index 31 - t have 31 terms
+// together, so the triangular products waste no lanes.  FP64-bound (about
+// 1,000 FMA a row); eight rows a CTA spread a small border over the SMs.
+__global__ void __launch_bounds__(128) k_border_panel(DevPlan d, DevBorder bd, int p) {
+  constexpr int n = kBorderPanel, ld = n + 1;
+  __shared__ double M[n * ld], dinv[n], rs[n];
+  __shared__ double V[8][n + 1], Z[8][n + 1];
+  __shared__ __align__(16) uint16_t stage[kDigits * 8 * n];
+  __shared__ int ex[8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r0 = blockIdx.x * 8, c0 = p * n;
+  for (int e = tid; e < n * n; e += 128) M[(e / n) * ld + e % n] = bd.piv[e];
+  if (tid < n) {
+    dinv[tid] = bd.piv[n * n + tid];
+    rs[tid] = bd.piv[n * n + n + tid];
+  }
+  const bool below = r0 >= c0 + n, own = !below && r0 >= c0;
+  double* W = bd.W;
+  if (below) {
+    for (int e = tid; e < 8 * n; e += 128) V[e & 7][e >> 3] = W[(int64_t)(c0 + (e >> 3)) * bd.ld + r0 + (e & 7)];
+  } else if (!own) {
+    for (int e = tid; e < 8 * n; e += 128) V[e >> 5][e & 31] = W[(int64_t)(r0 + (e >> 5)) * bd.ld + c0 + (e & 31)];
+  }
+  __syncthreads();
+  if (own) {
+    // the panel's own rows of X: D^-1/2 M; their digits are zero
+    for (int e = tid; e < 8 * n; e += 128) {
+      const int i = r0 - c0 + (e & 7), j = e >> 3;
+      V[e & 7][j] = rs[i] * M[i * ld + j];
+    }
+    for (int e = tid; e < kDigits * 8 * n / 2; e += 128) reinterpret_cast<uint32_t*>(stage)[e] = 0u;
+    if (tid < 8) ex[tid] = kExpZero;
+  } else {
+    const int ra = 2 * warp, rb = ra + 1, t = lane, tb = n - 1 - lane;
+    double ya = V[ra][t], yb = V[rb][tb];
+#pragma unroll 4
+    for (int s = 0; s < n - 1; ++s) {
+      if (s < t) ya = fma(M[t * ld + s], V[ra][s], ya);
+      else yb = fma(M[tb * ld + s - t], V[rb][s - t], yb);
+    }
+    Z[ra][t] = ya * dinv[t];
+    Z[rb][tb] = yb * dinv[tb];
+    ya *= rs[t];
+    yb *= rs[tb];
+    // digits of the two rows of Y
+    double y2[2] = {ya, yb};
+    const int row2[2] = {ra, rb}, t2[2] = {t, tb};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const double a = fabs(y2[h]);
+      // exponent field of the largest entry (NaN and infinity: 2047)
+      int e = (int)((unsigned long long)__double_as_longlong(a) >> 52) & 0x7ff;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+      const bool bad = e == 0x7ff, tiny = e < 64;  // |y| < 2^(e - 1022)
+      long long m = 0;
+      if (!bad && !tiny) m = __double2ll_rn(y2[h] * pow2_or_nan(55 - (e - 1022)));
+      if (lane == 0) ex[row2[h]] = bad ? kExpNan : tiny ? kExpZero : e - 1022;
+      uint16_t* st = stage + (t2[h] >> 3) * 64 + row2[h] * 8 + (t2[h] & 7);
+#pragma unroll
+      for (int q = kDigits - 1; q >= 0; --q) {
+        int dg = q ? (int)(signed char)(m & 0xff) : (int)m;
+        m = (m - dg) >> 8;
+        st[q * 8 * n] = (uint16_t)(__float_as_uint((float)dg) >> 16);  // an integer of at most 8 bits: exact in bf16
+      }
+    }
+    __syncwarp();
+    if (below) {
+      // Y L^-1 = M^T D^-1 M v: z_s + sum_{t > s} M[t][s] z_t
+      ya = Z[ra][t];
+      yb = Z[rb][tb];
+#pragma unroll 4
+      for (int s = 1; s < n; ++s) {
+        if (s > t) ya = fma(M[s * ld + t], Z[ra][s], ya);
+        else yb = fma(M[(tb + s) * ld + tb], Z[rb][tb + s], yb);
+      }
+      ya = -ya;
+      yb = -yb;
+    }
+    V[ra][t] = ya;
+    V[rb][tb] = yb;
+  }
+  __syncthreads();
+  if (below || own) {
+    for (int e = tid; e < 8 * n; e += 128) W[(int64_t)(c0 + (e >> 3)) * bd.ld + r0 + (e & 7)] = V[e & 7][e >> 3];
+  } else {
+    for (int e = tid; e < 8 * n; e += 128) W[(int64_t)(r0 + (e >> 5)) * bd.ld + c0 + (e & 31)] = V[e >> 5][e & 31];
+  }
+  uint8_t* dst = bd.dig + (int64_t)(r0 / kRowBlock) * kDigitBlockBytes + (r0 % kRowBlock) / 8 * 512;
+  for (int e = tid; e < kDigits * 32; e += 128)
+    *reinterpret_cast<uint4*>(dst + (e >> 5) * kPlaneBytes + (e & 31) * 16) =
+        *reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(stage) + e * 16);
+  if (tid < 8) bd.ey[r0 + tid] = ex[tid];
+}
+
+// A -= Y Y^T on one 128 x 32 tile of the rows below the panel.  Bounded by the
+// epilogue's FP64 work (three operations an element; the 34 digit products
+// take a quarter of that on the tensor cores) and by the read and write of
+// A; two CTAs an SM overlap one's loads and products with the other's
+// epilogue.
+__global__ void __launch_bounds__(256, 2) k_border_update(DevPlan d, DevBorder bd, int p) {
+  extern __shared__ __align__(1024) uint8_t usm[];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ uint32_t tmem_at;
+  __shared__ int ecol[kTileCols];
+  const int pn = p + 1;  // the next panel: its diagonal tile comes first, then its pivot block
+  const int t_0 = 2 * (pn / 4) * (pn / 4 + 1), t_next = t_0 + pn;  // tiles of the row blocks above: none
+  int t = t_0 + (int)blockIdx.x;
+  t = t == t_0 ? t_next : t == t_next ? t_0 : t;
+  int rb = (int)((sqrtf(1.0f + 2.0f * (float)t) - 1.0f) * 0.5f);
+  while (2 * rb * (rb + 1) > t) --rb;
+  while (2 * (rb + 1) * (rb + 2) <= t) ++rb;
+  const int cb = t - 2 * rb * (rb + 1);
+  if (cb == p) return;  // the panel itself
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t sA = smem_addr(usm), sB = sA + kDigitBlockBytes;
+  const uint32_t bar_load = smem_addr(&bars[0]), bar_mma = smem_addr(&bars[1]);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_at)),
+                 "r"(kTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 32) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_load));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_mma));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_load),
+                 "r"(kDigitBlockBytes + kDigits * kBPlaneBytes) : "memory");
+    const uint8_t* ga = bd.dig + (int64_t)rb * kDigitBlockBytes;
+    const uint8_t* gb = bd.dig + (int64_t)(cb >> 2) * kDigitBlockBytes + (cb & 3) * kBPlaneBytes;
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sA),
+                 "l"(ga), "r"(kDigitBlockBytes), "r"(bar_load) : "memory");
+#pragma unroll
+    for (int q = 0; q < kDigits; ++q)
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       sB + q * kBPlaneBytes),
+                   "l"(gb + q * kPlaneBytes), "r"(kBPlaneBytes), "r"(bar_load) : "memory");
+  }
+  if (tid >= 64 && tid < 64 + kTileCols) ecol[tid - 64] = bd.ey[cb * kTileCols + tid - 64];
+  // this thread's sixteen elements of A, on their way while the digits load
+  const int quad = warp & 3, half = warp >> 2;
+  const int row = rb * kRowBlock + quad * 32 + lane;
+  double* g = bd.W + (int64_t)(cb * kTileCols + half * 16) * bd.ld + row;
+  double a[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) a[j] = g[(int64_t)j * bd.ld];
+  const int er = row < pn * kBorderPanel ? kExpZero : bd.ey[row] - 38;  // rows up to the panel are done
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_at;
+  if (tid == 0) {
+    bool ok = mbar_wait(bar_load, 0, d.sc);
+    if (!ok) ok = mbar_wait(bar_load, 0, d.sc);  // the copies in flight: once more, with a limit
+    if (d.dbg_unsatisfiable) mbar_wait_hook(bar_load, 1, d);
+    // D f32, A and B bf16, K-major both, M 128, N 32
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileCols / 8) << 17) | ((uint32_t)(kRowBlock / 16) << 24);
+#pragma unroll 1
+    for (int kk = 0; kk < 2; ++kk)
+#pragma unroll 1
+      for (int i = 0; i < kDigits; ++i)
+#pragma unroll 1
+        for (int j = 0; j < kDigits && i + j < kAccs; ++j) {
+          const uint64_t da = operand_desc(sA + i * kPlaneBytes + kk * 256);
+          const uint64_t db = operand_desc(sB + j * kBPlaneBytes + kk * 256);
+          // first product of this weight: (0, w), or (1, 6) for weight 7
+          const uint32_t acc = kk > 0 || i > (i + j < kDigits ? 0 : i + j - (kDigits - 1));
+          asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(
+                           tmem + (uint32_t)((i + j) * kTileCols)),
+                       "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
+        }
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_mma) : "memory");
+    if (!mbar_wait(bar_mma, 0, d.sc)) mbar_wait(bar_mma, 0, d.sc);
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // Per element the eight exact sums a_w of weight 2^(er + ec - 14 - 8 w) form
+  // hi 2^32 + lo with integers; as doubles through the bits of 1.5 * 2^52 + i,
+  // t = hi + lo 2^-32 is rounded once, and once more when it is subtracted.
+  const double kBiasHi = 6755399441055744.0 + 1572864.0;  // 1.5 * 2^52 and lo's bias 1.5 * 2^52 * 2^-32
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t r[kAccs][8];
+#pragma unroll
+    for (int w = 0; w < kAccs; ++w) {
+      const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(w * kTileCols + half * 16 + h * 8);
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(r[w][0]), "=r"(r[w][1]), "=r"(r[w][2]), "=r"(r[w][3]), "=r"(r[w][4]), "=r"(r[w][5]),
+                     "=r"(r[w][6]), "=r"(r[w][7])
+                   : "r"(ta));
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      int s[kAccs];
+#pragma unroll
+      for (int w = 0; w < kAccs; ++w)  // exact: |sum| <= 7 * 2^19 < 2^22
+        s[w] = __float_as_int(__uint_as_float(r[w][j]) + 12582912.0f) - 0x4B400000;
+      const long long hi = (long long)(s[0] * 256 + s[1]) * 65536 + (s[2] * 256 + s[3]);
+      const long long lo = (long long)(s[4] * 256 + s[5]) * 65536 + (s[6] * 256 + s[7]);
+      const double dh = __longlong_as_double(0x4338000000000000ll + hi) - kBiasHi;
+      const double t2 = fma(__longlong_as_double(0x4338000000000000ll + lo), 0x1p-32, dh);
+      const double sc = pow2_or_nan(er + ecol[half * 16 + h * 8 + j]);
+      a[h * 8 + j] = fma(-sc, t2, a[h * 8 + j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) g[(int64_t)j * bd.ld] = a[j];
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+  if (blockIdx.x == 0 && pn < bd.npan) {
+    // the shared memory of the operands is free: the next panel's pivot block
+    double* A = reinterpret_cast<double*>(usm);
+    double* M = A + kBorderPanel * (kBorderPanel + 1);
+    const double* src = bd.W + (int64_t)pn * kBorderPanel * bd.ld + pn * kBorderPanel;
+    for (int e = tid; e < kBorderPanel * kBorderPanel; e += 256)
+      A[(e % kBorderPanel) * (kBorderPanel + 1) + e / kBorderPanel] = src[(int64_t)(e / kBorderPanel) * bd.ld + e % kBorderPanel];
+    __syncthreads();
+    pivot_block(d, bd, pn, A, M);
+  }
+}
+
+// Row panels of X and of X^T for the solves' products, one contiguous block
+// per rb rows (column after column of the panel, zeros outside the triangle):
+// in the column-major border itself a task's pieces lie a column stride apart,
+// which ran the 10,000-bus products at a fifth of the streaming rate.  One CTA
+// per 64 x 64 tile of the lower triangle.
+__host__ __device__ inline int64_t panel_lo(int64_t b, int rb) { return (int64_t)rb * rb * (b * (b + 1) / 2); }
+// X^T panels cover the columns [rb b, rb nrb): the offset from the first
+__host__ __device__ inline int64_t panel_up(int64_t b, int64_t nrb, int rb) {
+  return (int64_t)rb * rb * (b * nrb - b * (b - 1) / 2);
+}
+
+__global__ void __launch_bounds__(256) k_border_pack(DevBorder bd) {
+  __shared__ double tile[64][65];
+  int ti = (int)((sqrtf(1.0f + 8.0f * (float)blockIdx.x) - 1.0f) * 0.5f);
+  while (ti * (ti + 1) / 2 > (int)blockIdx.x) --ti;
+  while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.x) ++ti;
+  const int tj = blockIdx.x - ti * (ti + 1) / 2;
+  const int i0 = ti * 64, j0 = tj * 64, rb = bd.rb, nrb = bd.nrb;
+  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
+    const int i = e & 63, j = e >> 6;
+    tile[j][i] = i0 + i >= j0 + j ? bd.W[(int64_t)(j0 + j) * bd.ld + i0 + i] : 0.0;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
+    // rows of X: row block (i0 + i) / rb, column j0 + j
+    const int r = e % rb, j = (e / rb) & 63, g = e / rb / 64, b = i0 / rb + g;
+    if (b < nrb && j0 + j < (b + 1) * rb) bd.xlo[panel_lo(b, rb) + (int64_t)(j0 + j) * rb + r] = tile[j][g * rb + r];
+  }
+  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
+    // rows of X^T: row block (j0 + c) / rb, column i0 + i
+    const int r = e % rb, i = (e / rb) & 63, g = e / rb / 64, b = j0 / rb + g;
+    if (b < nrb && i0 + i >= b * rb && i0 + i < nrb * rb)
+      bd.xup[panel_up(b, nrb, rb) + (int64_t)(i0 + i - b * rb) * rb + r] = tile[g * rb + r][i];
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Solves and the CG loop: one launch each, its CTAs claiming tasks of dense
+// phases from a counter in phase order.
+//   0  blocks:  y_F = X b_F, u = E b_F;       CG: the vector update as well
+//   1  border right-hand side  bt = b_S - sum u   (in phase 0 without blocks)
+//   2  by = X bt               3  x_S = X^T by
+//   4  blocks:  x_F = X^T y_F - E^T x_S
+//   5  CG: w = Jc_p x and the recurrence's scalars
+// A task waits (bounded) until the tasks of the phase it reads from are done;
+// they were claimed before it by CTAs that are running, so the scheme cannot
+// deadlock whatever the number of resident CTAs.  What a task reads that the
+// launch does not change (its panel, its block, indices) it loads before it
+// waits: a phase then costs little more than the round trips of its signal and
+// of the vector.  Data written in the same launch is read with ld.global.cg.
+// Every sum is taken in a fixed order: results do not depend on the
+// scheduling.  The CG loop in one launch replaces five launches per iteration.
+// ---------------------------------------------------------------------------
+constexpr int kCgRows = 256;  // rows of a vector task
+constexpr int kRowTask = 64;  // columns or constraints of a sparse task, four threads each
+
+struct BorderRhs {
+  const double* b;  // right-hand side, or null: Jc_p^T r of the CG's updated residual
+  const double *r, *w, *s;
+  double alpha, beta;
+};
+
+// r - alpha (w + beta s): the residual after this iteration's update
+__device__ __forceinline__ double cg_updated(const BorderRhs& q, int k) {
+  return fma(-q.alpha, fma(q.beta, __ldcg(&q.s[k]), __ldcg(&q.w[k])), __ldcg(&q.r[k]));
+}
+
+// Part of one row of a sparse product: L threads share a row (its entries
+// interleaved), each one's first eight indices and values are loaded ahead of
+// the wait for the vector.  (Hub buses have rows of 60 entries and more: one
+// thread per row made them the phase's length.)
+struct SparseRow {
+  int p, e, L;
+  int c[8];
+  double a[8];
+};
+template <class VIdx>
+__device__ __forceinline__ void load_row(SparseRow& r, int p, int e, int L, int sub, const int* __restrict__ ci, const double* __restrict__ v, VIdx vidx) {
+  r.p = p + sub;
+  r.e = e;
+  r.L = L;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const bool in = r.p + j * L < e;
+    r.c[j] = in ? ci[r.p + j * L] : 0;
+    r.a[j] = in ? v[vidx(r.p + j * L)] : 0.0;
+  }
+}
+template <class VIdx, class X>
+__device__ __forceinline__ double row_dot(SparseRow& r, const int* __restrict__ ci, const double* __restrict__ v, VIdx vidx, X x) {
+  double acc = 0.0;
+  for (;;) {
+    double t[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) t[j] = r.p + j * r.L < r.e ? x(r.c[j]) : 0.0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (r.p + j * r.L < r.e) acc = fma(r.a[j], t[j], acc);
+    const int p = r.p + 8 * r.L;
+    if (p >= r.e) break;
+    load_row(r, p, r.e, r.L, 0, ci, v, vidx);
+  }
+  return acc;
+}
+// the L threads' parts (neighbouring lanes), L a power of two up to 4
+__device__ __forceinline__ double join_row(double s, int L) {
+  if (L > 1) s = dadd(s, __shfl_xor_sync(0xffffffffu, s, 1));
+  if (L > 2) s = dadd(s, __shfl_xor_sync(0xffffffffu, s, 2));
+  return s;
+}
+
+// right-hand side of a permuted column in the CG: the column's row of Jc_p^T
+__device__ __forceinline__ void load_rhs_row(const DevPlan& d, SparseRow& r, int col, int L, int sub) {
+  const int* src = d.jctp_src;
+  load_row(r, d.jctp_rp[col], d.jctp_rp[col + 1], L, sub, d.jctp_ci, d.jc_s, [src](int p) { return src[p]; });
+}
+__device__ __forceinline__ double rhs_row_dot(const DevPlan& d, SparseRow& r, const BorderRhs& q) {
+  const int* src = d.jctp_src;
+  return row_dot(r, d.jctp_ci, d.jc_s, [src](int p) { return src[p]; }, [&](int k) { return cg_updated(q, k); });
+}
+
+// every fourth of the blocks' contributions to border column j
+__device__ __forceinline__ double border_updates(const DevBorder& bd, int j, int sub) {
+  double s = 0.0;
+  const int e = bd.ug_rp[j + 1];
+  for (int p = bd.ug_rp[j] + sub; p < e; p += 16) {
+    double t[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = p + 4 * i < e ? __ldcg(&bd.u[bd.ug_pos[p + 4 * i]]) : 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s = dadd(s, t[i]);
+  }
+  return s;
+}
+
+// Products of a dense row panel, column after column of its RB rows, with a
+// vector in shared memory: 256 / RB threads a row over interleaved columns.
+// The panel streams through kStages shared-memory chunks by bulk copies, the
+// first of them issued before the task waits for its vector.
+constexpr int kGemvSeg = 2048, kChunk = 2048, kStages = 3;  // most columns of a panel, entries of a chunk
+constexpr int kRed = 256;                                   // doubles before the vector
+constexpr int kSolveSmem = (kRed + kGemvSeg + kStages * kChunk) * 8;
+
+// state of the CTA's chunk ring: chunks issued and consumed since the launch
+struct Ring {
+  uint32_t bar;  // kStages mbarriers
+  unsigned put, got;
+};
+
+__device__ __forceinline__ void ring_put(Ring& g, double* chunks, const double* src, int n) {
+  const int st = g.put % kStages;
+  ++g.put;
+  if (threadIdx.x == 0) {
+    const uint32_t bar = g.bar + 8 * st;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n * 8) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_addr(chunks + st * kChunk)),
+                 "l"(src), "r"(n * 8), "r"(bar) : "memory");
+  }
+}
+
+// every thread waits for the oldest chunk (bounded)
+__device__ __forceinline__ int ring_get(Ring& g, DevScalars* sc) {
+  const int st = g.got % kStages;
+  mbar_wait(g.bar + 8 * st, (g.got / kStages) & 1, sc);
+  ++g.got;
+  return st;
+}
+
+struct Panel {
+  const double* M;
+  int n;  // entries: columns * RB
+};
+__device__ __forceinline__ void panel_start(Ring& g, const Panel& p, double* sm) {
+  double* ch = sm + kRed + kGemvSeg;
+  for (int c = 0; c < kStages && c * kChunk < p.n; ++c) ring_put(g, ch, p.M + c * kChunk, min(kChunk, p.n - c * kChunk));
+}
+// the copies in flight of a task that gives up
+__device__ __forceinline__ void panel_drain(Ring& g, DevScalars* sc) {
+  while (g.got < g.put) ring_get(g, sc);
+}
+// the product of row threadIdx.x in threads below RB; v = sm + kRed is complete
+template <int RB>
+__device__ __forceinline__ double panel_product(Ring& g, const Panel& p, double* sm, DevScalars* sc) {
+  constexpr int P = 256 / RB, kCols = kChunk / RB;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double* v = sm + kRed + threadIdx.x / RB;
+  double* ch = sm + kRed + kGemvSeg;
+  double a[2] = {0.0, 0.0};
+  int left = p.n / RB - threadIdx.x / RB;
+  for (int c = 0; c * kChunk < p.n; ++c, v += kCols, left -= kCols) {
+    const double* m = ch + ring_get(g, sc) * kChunk + threadIdx.x;
+    if (left > 7 * P) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a[q & 1] = fma(m[q * 256], v[q * P], a[q & 1]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q * P < left) a[q & 1] = fma(m[q * 256], v[q * P], a[q & 1]);
+    }
+    __syncthreads();
+    const int nx = (c + kStages) * kChunk;
+    if (nx < p.n) ring_put(g, ch, p.M + nx, min(kChunk, p.n - nx));
+  }
+  double s = dadd(a[0], a[1]);
+  constexpr int kParts = RB < 32 ? 8 : P;  // partial sums per row left after the shuffles
+#pragma unroll
+  for (int o = RB; o < 32; o <<= 1) s = dadd(s, __shfl_xor_sync(0xffffffffu, s, o));
+  if (RB >= 32) sm[threadIdx.x] = s;
+  else if (lane < RB) sm[warp * RB + lane] = s;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x < RB) {
+    double w[kParts];
+#pragma unroll
+    for (int q = 0; q < kParts; ++q) w[q] = sm[q * RB + threadIdx.x];
+#pragma unroll
+    for (int o = 1; o < kParts; o <<= 1)
+#pragma unroll
+      for (int q = 0; q < kParts; q += 2 * o) w[q] = dadd(w[q], w[q + o]);
+    t = w[0];
+  }
+  return t;
+}
+
+// by = X bt (up 0) or x_S = X^T by (up 1) for up to kGemvSeg columns of a
+// panel.  A longer panel's tasks store their sums, the last one adds them in
+// column order.  Bounded by FP64 issue (one multiply-add per entry, 2 per clock
+// and SM), by HBM where the panels exceed the L2.  Four rows a panel keep a
+// small border's tasks short, eight halve the vector reads of a large one.
+template <int RB, class Wait>
+__device__ __forceinline__ bool border_gemv(const DevPlan& d, const DevBorder& bd, Ring& g, int task, bool up, double* x, double* sm, Wait wait) {
+  __shared__ bool fin;
+  // tasks by column segment, in a segment the panels that reach it, longest first
+  int sg = 0, b = task;
+  for (int c = bd.nrb; b >= c; c = bd.nrb - (sg * kGemvSeg) / RB) {
+    b -= c;
+    ++sg;
+  }
+  if (!up) b = bd.nrb - 1 - b;
+  const int len = up ? bd.k - b * RB : min(bd.k, (b + 1) * RB);
+  const int j0 = sg * kGemvSeg, n = min(kGemvSeg, len - j0), segs = (len + kGemvSeg - 1) / kGemvSeg;
+  const Panel p{(up ? bd.xup + panel_up(b, bd.nrb, RB) : bd.xlo + panel_lo(b, RB)) + (int64_t)j0 * RB, n * RB};
+  panel_start(g, p, sm);
+  if (!wait()) {
+    panel_drain(g, d.sc);
+    return false;
+  }
+  const double* src = (up ? bd.by + b * RB : bd.bt) + j0;
+  double* v = sm + kRed;
+#pragma unroll
+  for (int h = 0; h < kGemvSeg / 256; h += 4) {
+    double t[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) t[q] = threadIdx.x + (h + q) * 256 < n ? __ldcg(&src[threadIdx.x + (h + q) * 256]) : 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[threadIdx.x + (h + q) * 256] = t[q];
+    if ((h + 4) * 256 >= n) break;
+  }
+  __syncthreads();
+  double t = panel_product<RB>(g, p, sm, d.sc);
+  const int row = b * RB + threadIdx.x;
+  if (segs > 1) {
+    double* slot = bd.part + (int64_t)b * bd.nseg * RB;
+    if (threadIdx.x < RB) __stcg(&slot[sg * RB + threadIdx.x], t);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      fin = atomicAdd(&bd.rowcnt[b], 1) == segs - 1;
+      __threadfence();
+    }
+    __syncthreads();
+    if (!fin) return true;
+    if (threadIdx.x < RB) {
+      t = __ldcg(&slot[threadIdx.x]);
+      for (int q = 1; q < segs; ++q) t = dadd(t, __ldcg(&slot[q * RB + threadIdx.x]));
+    }
+    if (threadIdx.x == 0) bd.rowcnt[b] = 0;  // for the next product
+  }
+  if (threadIdx.x < RB && row < bd.k) {
+    if (up) x[bd.bcol[row]] = t;
+    else bd.by[row] = t;
+  }
+  return true;
+}
+
+// Dot product of row `lane` of a warp's block panel (64 rows a column).
+__device__ __forceinline__ double warp_rows(const double* __restrict__ M, int K, const double* v) {
+  double a[2] = {0.0, 0.0};
+  for (int t = 0; t < K; t += 8) {
+    double m[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m[j] = t + j < K ? M[(t + j) * 64] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (t + j < K) a[j & 1] = fma(m[j], v[t + j], a[j & 1]);
+  }
+  return dadd(a[0], a[1]);
+}
+
+// y_F = X b_F, u = E b_F: 64 rows of a block of more than 32 rows per CTA, or
+// eight smaller blocks, one per warp.  (A block's rows on several CTAs: one
+// SM's FP64 rate would make a whole large block 20-40 us.)
+template <bool kCg, class Wait>
+__device__ __forceinline__ bool block_fwd(const DevPlan& d, const DevBorder& bd, const BorderRhs& q, Ring& g, int task, double* sm, Wait wait) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool big = task < bd.nfp;
+  const int blk = big ? bd.fp_blk[task] : bd.nbig + (task - bd.nfp) * 8 + warp;
+  const bool have = blk < bd.nblk;
+  const int c0 = have ? bd.blk_rp[blk] : 0, nt = have ? bd.blk_rp[blk + 1] - c0 : 0;
+  const int N = have ? nt + bd.blk_rrp[blk + 1] - bd.blk_rrp[blk] : 0;
+  const int r0 = big ? 64 * (task - bd.fp_first[blk]) : 0;
+  // right-hand side: L threads per column (a warp's block: one)
+  const int L = !big || nt > 128 ? 1 : nt > 64 ? 2 : 4;
+  const int i = big ? (int)threadIdx.x / L : lane, sub = big ? threadIdx.x % L : 0;
+  const int col = i < nt ? bd.blk_col[c0 + i] : 0;
+  const Panel p{bd.ge + (have ? bd.ge_off[blk] + (int64_t)r0 * nt : 0), 64 * nt};
+  SparseRow row;
+  row.p = row.e = 0;
+  row.L = 1;
+  if (kCg && i < nt) load_rhs_row(d, row, col, L, sub);
+  if (big) panel_start(g, p, sm);
+  else prefetch_bytes(p.M, (int64_t)64 * nt * 8, lane, 32);
+  if (!wait()) {
+    panel_drain(g, d.sc);
+    return false;
+  }
+  const double w = kCg ? join_row(rhs_row_dot(d, row, q), L) : i < nt ? q.b[col] : 0.0;
+  double* v = big ? sm + kRed : sm + warp * 32;
+  if (i < nt && sub == 0) v[i] = w;
+  if (big) __syncthreads();
+  else __syncwarp();
+  const double t = big ? panel_product<64>(g, p, sm, d.sc) : warp_rows(p.M + lane, nt, v);
+  const int r = big ? (int)threadIdx.x : lane;
+  if ((!big || r < 64) && r0 + r < N) {
+    if (r0 + r < nt) bd.y[c0 + r0 + r] = t;
+    else bd.u[bd.u_off[blk] + r0 + r - nt] = t;
+  }
+  return true;
+}
+
+// x_F = X^T y_F - E^T x_S: the same for 64 columns of a block
+template <class Wait>
+__device__ __forceinline__ bool block_bwd(const DevPlan& d, const DevBorder& bd, Ring& g, int task, double* x, double* sm, Wait wait) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool big = task < bd.nbp;
+  const int blk = big ? bd.bp_blk[task] : bd.nbig + (task - bd.nbp) * 8 + warp;
+  const bool have = blk < bd.nblk;
+  const int c0 = have ? bd.blk_rp[blk] : 0, nt = have ? bd.blk_rp[blk + 1] - c0 : 0;
+  const int b0 = have ? bd.blk_rrp[blk] : 0, R = have ? bd.blk_rrp[blk + 1] - b0 : 0, N = nt + R;
+  const int t0 = big ? 64 * (task - bd.bp_first[blk]) : 0;
+  const int i = big ? (int)threadIdx.x : lane;
+  const int brow = i < R ? bd.bcol[bd.blk_row[b0 + i]] : 0;
+  const Panel p{bd.et + (have ? bd.et_off[blk] + (int64_t)t0 * N : 0), 64 * N};
+  if (big) panel_start(g, p, sm);
+  else prefetch_bytes(p.M, (int64_t)64 * N * 8, lane, 32);
+  const int r = t0 + (big ? (int)threadIdx.x & 63 : lane);
+  const int col = r < nt ? bd.blk_col[c0 + r] : 0;
+  if (!wait()) {
+    panel_drain(g, d.sc);
+    return false;
+  }
+  double* v = big ? sm + kRed : sm + warp * 32;
+  if (i < N) v[i] = i < R ? __ldcg(&x[brow]) : __ldcg(&bd.y[c0 + i - R]);
+  if (big) __syncthreads();
+  else __syncwarp();
+  const double t = big ? panel_product<64>(g, p, sm, d.sc) : warp_rows(p.M + lane, N, v);
+  if ((!big || threadIdx.x < 64) && r < nt) x[col] = t;
+  return true;
+}
+
+// Task table of one launch: phases in order, the phase each one waits for,
+// counters [head, ready, done, phase counts].
+struct BorderTasks {
+  int n[6], off[7], dep[6];
+  int n_upd;  // CG: vector update tasks of phase 0
+  int n_fwd;  // block tasks of phase 0
+};
+// each on a 128-byte line of its own: hundreds of CTAs poll them
+constexpr int kCtlReady = 16, kCtlDone = 32, kCtlCount = 48, kCtlStep = 16, kCtlWords = 48 + 6 * 16;
+typedef unsigned long long count_t;  // tasks of all iterations of a CG run
+__device__ __forceinline__ count_t load_acquire(const count_t* p) {
+  count_t v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// thread 0: waits until *p >= need; false when the CG has stopped or the wait
+// gave up (wait_ge in kernels.cuh: the same limit, flag and test hook)
+__device__ __forceinline__ bool border_wait(const count_t* p, count_t need, const count_t* done, const DevPlan& d) {
+  need += d.dbg_unsatisfiable;
+  if (need > 0) {
+    volatile const int* flags = &d.sc->solve_flags;
+    for (unsigned it = 0; load_acquire(p) < need; ++it) {
+      if ((it & 7) == 7 && *(volatile const count_t*)done) return false;
+      if (it > d.spin_limit || ((it & 15) == 15 && (*flags & 1))) {
+        atomicOr(&d.sc->solve_flags, 1);
+        return false;
+      }
+    }
+  }
+  return !*(volatile const count_t*)done;  // set before the count that a stopped CG publishes
+}
+
+template <bool kCg>
+__global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd, BorderTasks tk, const double* b, double* x, int use_stop) {
+  extern __shared__ double sm[];
+  __shared__ double red[2 * 32];
+  __shared__ int s_it, s_t, go, last;
+  __shared__ double sc2[2];
+  if ((kCg || use_stop) && *(volatile const int*)&d.sc->stop) return;
+  count_t* head = bd.ctl;
+  count_t* ready = bd.ctl + kCtlReady;
+  count_t* done = bd.ctl + kCtlDone;
+  count_t* cnt = bd.ctl + kCtlCount;
+  DevScalars* S = d.sc;
+  const int T = tk.off[6];
+  __shared__ __align__(8) uint64_t bars[kStages];
+  Ring ring{smem_addr(bars), 0, 0};
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ring.bar + 8 * i));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  count_t base = 0, seen = 0;  // thread 0: the first task of iteration s_it; phases known to be done (6 per iteration)
+  if (threadIdx.x == 0) s_it = 0;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const count_t next = atomicAdd(head, count_t(1));
+      for (; next - base >= (count_t)T; base += T) ++s_it;
+      s_t = (int)(next - base);
+    }
+    __syncthreads();
+    const int it = s_it, t = s_t;
+    if (!kCg && it > 0) return;
+    trace_mark(d, t, 0);
+    trace_mark(d, t, 3);
+    int ph = 0;
+    while (t >= tk.off[ph + 1]) ++ph;
+    const int task = t - tk.off[ph];
+    double* rin = it & 1 ? bd.r2 : d.cg_r;
+    double* rout = it & 1 ? d.cg_r : bd.r2;
+    double* sin = it & 1 ? bd.s2 : d.cg_s;
+    double* sout = it & 1 ? d.cg_s : bd.s2;
+    BorderRhs q{b, rin, d.cg_w, sin, 0.0, 0.0};
+    // the CTA waits for the previous iteration's scalars (kCg), or for a phase
+    auto wait_for = [&](const count_t* p, count_t need, bool scal) {
+      if (threadIdx.x == 0) {
+        const count_t mark = (count_t)it * 6 + (scal ? 0 : ph);
+        const bool ok = mark < seen || border_wait(p, need, done, d);
+        seen = mark + 1;
+        go = ok;
+        if (!ok && kCg && (*(volatile int*)&S->solve_flags & 1)) {
+          *(volatile int*)&S->stop = 3;
+          *(volatile count_t*)done = 1;
+        }
+        if (kCg && scal) {
+          sc2[0] = *(volatile double*)&S->alpha;
+          sc2[1] = *(volatile double*)&S->beta;
+        }
+      }
+      __syncthreads();
+      if (kCg && scal) {
+        q.alpha = sc2[0];
+        q.beta = sc2[1];
+      }
+      trace_mark(d, t, 1);
+      return go != 0;
+    };
+    auto wait_ready = [&]() { return wait_for(ready, (count_t)it, true); };
+    auto wait_phase = [&]() { return wait_for(&cnt[tk.dep[ph] * kCtlStep], (count_t)(it + 1) * tk.n[tk.dep[ph]], false); };
+    bool scalars = false;
+    if (ph == 0 && task < tk.n_fwd) {
+      if (!block_fwd<kCg>(d, bd, q, ring, task, sm, wait_ready)) return;
+    } else if (ph == 0 && task < tk.n_fwd + tk.n_upd) {
+      // p = r + beta p; s = w + beta s; x += alpha p; r -= alpha s; r.r
+      if (!wait_ready()) return;
+      const int c = task - tk.n_fwd, k = c * kCgRows + threadIdx.x;
+      double part[1] = {0.0};
+      if (k < d.m_c) {
+        const double r = __ldcg(&rin[k]), s0 = __ldcg(&sin[k]), w = __ldcg(&d.cg_w[k]), p0 = __ldcg(&d.cg_p[k]), x0 = __ldcg(&d.cg_x[k]);
+        const double sv = fma(q.beta, s0, w), p = fma(q.beta, p0, r), rn = fma(-q.alpha, sv, r);
+        d.cg_p[k] = p;
+        sout[k] = sv;
+        d.cg_x[k] = fma(q.alpha, p, x0);
+        rout[k] = rn;
+        part[0] = rn * rn;
+      }
+      block_reduce_sum<1>(part, red);
+      if (threadIdx.x == 0) bd.rrp[c] = part[0];
+    } else if (ph <= 1) {
+      // bt = b_S - sum u (in phase 0 there are no blocks)
+      const int j = (ph ? task : task - tk.n_fwd - tk.n_upd) * kRowTask + (threadIdx.x >> 2), sub = threadIdx.x & 3;
+      const int col = j < bd.k ? bd.bcol[j] : 0;
+      SparseRow row;
+      row.p = row.e = 0;
+      row.L = 4;
+      if (kCg && j < bd.k) load_rhs_row(d, row, col, 4, sub);
+      if (!wait_ready()) return;
+      double v = kCg ? rhs_row_dot(d, row, q) : j < bd.k && sub == 0 ? b[col] : 0.0;
+      if (ph == 1) {
+        __syncthreads();  // go is read before it is written again
+        if (!wait_phase()) return;
+        if (j < bd.k) v = dsub(v, border_updates(bd, j, sub));
+      }
+      v = join_row(v, 4);
+      if (j < bd.k && sub == 0) bd.bt[j] = v;
+    } else if (ph <= 3) {
+      if (!(bd.rb == 4 ? border_gemv<4>(d, bd, ring, task, ph == 3, x, sm, wait_phase)
+                       : border_gemv<8>(d, bd, ring, task, ph == 3, x, sm, wait_phase)))
+        return;
+    } else if (ph == 4) {
+      if (!block_bwd(d, bd, ring, task, x, sm, wait_phase)) return;
+    } else {
+      // w = Jc_p x, delta = w.r
+      const int k = task * kRowTask + (threadIdx.x >> 2), sub = threadIdx.x & 3;
+      SparseRow row;
+      row.p = row.e = 0;
+      row.L = 4;
+      auto vi = [](int p) { return p; };
+      if (k < d.m_c) load_row(row, d.jc_rp[k], d.jc_rp[k + 1], 4, sub, d.jcp_ci, d.jc_s, vi);
+      if (!wait_phase()) return;
+      double part[1] = {0.0};
+      const double r = k < d.m_c ? __ldcg(&rout[k]) : 0.0;
+      const double acc = join_row(row_dot(row, d.jcp_ci, d.jc_s, vi, [&](int c) { return __ldcg(&x[c]); }), 4);
+      if (k < d.m_c && sub == 0) {
+        d.cg_w[k] = acc;
+        part[0] = acc * r;
+      }
+      block_reduce_sum<1>(part, red);
+      if (threadIdx.x == 0) bd.dlp[task] = part[0];
+      scalars = true;
+    }
+    // done: the CTA's writes, then the count
+    __syncthreads();
+    trace_mark(d, t, 2);
+    if (!scalars) {
+      if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&cnt[ph * kCtlStep]) : "memory");
+      continue;
+    }
+    if (threadIdx.x == 0) {
+      count_t old;
+      asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], 1;" : "=l"(old) : "l"(&cnt[ph * kCtlStep]) : "memory");
+      last = old == (count_t)(it + 1) * tk.n[5] - 1;
+    }
+    __syncthreads();
+    if (!last) continue;
+    // the last constraint task: both sums in task order, the recurrence and the
+    // stopping tests (k_spmv_jcp, k_cg_update)
+    double v[2] = {0.0, 0.0};
+    for (int i = threadIdx.x; i < tk.n_upd; i += 256) v[0] = dadd(v[0], __ldcg(&bd.rrp[i]));
+    for (int i = threadIdx.x; i < tk.n[5]; i += 256) v[1] = dadd(v[1], __ldcg(&bd.dlp[i]));
+    block_reduce_sum<2>(v, red);
+    if (threadIdx.x == 0) {
+      S->gam1 = v[0];
+      S->it += 1;
+      S->it_total += 1;
+      S->cg_err = sqrt(v[0]);
+      const double thr = S->rtol_cur > 0.0 ? S->rtol_cur * sqrt(S->gam0) : d.cg_tol;
+      int stop = 0;
+      if (S->cg_err < thr) stop = 1;
+      S->cond_calls += 1;
+      if (!stop && (S->it >= d.cg_itmax || S->cond_calls >= d.cg_itmax)) {
+        stop = 2;
+        S->stop_main += 1;
+      }
+      S->delta = v[1];
+      if (!stop) {
+        const double gam = v[0], beta = gam / S->gam;
+        S->beta = beta;
+        S->gam = gam;
+        S->alpha = gam / (v[1] - beta * gam / S->alpha);
+      } else {
+        S->stop = stop;
+        *(volatile count_t*)done = 1;
+      }
+      asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(ready), "l"((count_t)(it + 1)) : "memory");
+    }
+  }
+}
+
+}  // namespace hykkt

@@ -132,6 +132,17 @@ void apply_solve_piece(SymbolicOptions& o, int solve_piece) {
   o.solve_piece = solve_piece;
   if (!std::getenv("HYKKT_SOLVE_WARP_SUBTREE")) o.warp_subtree = 0;
 }
+
+// Pieces of kMinBorderPiece columns or more are asked for to save inversion
+// work on the widest supernodes, which the bordered layout does not have;
+// narrower ones ask for the task-queue layout itself.  HYKKT_BORDERED=0 keeps
+// every plan on the task queues.
+constexpr int kMinBorderPiece = 512;
+bool border_allowed(int solve_piece) {
+  const char* e = std::getenv("HYKKT_BORDERED");
+  if (e && e[0] == '0') return false;
+  return solve_piece <= 0 || solve_piece >= kMinBorderPiece;
+}
 }  // namespace
 
 extern "C" const char* hykkt_last_error(void) { return g_err.c_str(); }
@@ -173,6 +184,7 @@ static int plan_create(hykkt_plan_t* plan, int n_x, int m_c, int m_d, const int*
     CsrPattern Jd = make_pattern(m_d, n_x, jd_rowptr, jd_colidx, nnz_jd);
     SymbolicOptions opt = default_options(ordering);
     apply_solve_piece(opt, solve_piece);
+    opt.bordered = border_allowed(solve_piece);
     Symbolic S = build_symbolic(H, Ds, Jc, Jd, opt, perm);
     auto p = std::make_unique<hykkt_plan_s>();
     p->eng = std::make_unique<Engine>(std::move(S), gamma, opt, deferred);
@@ -328,6 +340,7 @@ SymbolicOptions options_for(const SymbolicOptions& base, const TuneChoice& c) {
   o.solve_piece = c.solve_piece > 0 ? c.solve_piece : (1 << 30);
   o.warp_subtree = c.warp_subtree;
   o.chunk_fma = c.chunk_fma;
+  o.bordered = border_allowed(c.solve_piece);
   return o;
 }
 
@@ -733,6 +746,22 @@ const std::vector<int>* sym_array(const Symbolic& S, std::vector<int>& L_cp, std
   if (w == "perm") return &S.perm;
   if (w == "etree") return &S.parent;
   if (w == "colcount") return &S.colcount;
+  // bordered layout (empty for a plan of the task-queue layout)
+  if (w == "bd_col") return &S.border.bcol;
+  if (w == "bd_blk_rp") return &S.border.blk_rp;
+  if (w == "bd_blk_col") return &S.border.blk_col;
+  if (w == "bd_blk_rrp") return &S.border.blk_rrp;
+  if (w == "bd_blk_row") return &S.border.blk_row;
+  if (w == "bd_ent_rp") return &S.border.ent_rp;
+  if (w == "bd_ent_q") return &S.border.ent_q;
+  if (w == "bd_ent_pos") return &S.border.ent_pos;
+  if (w == "bd_asm_row") return &S.border.asm_row;
+  if (w == "bd_asm_col") return &S.border.asm_col;
+  if (w == "bd_asm_src") return &S.border.asm_src;
+  if (w == "bd_asm_rp") return &S.border.asm_rp;
+  if (w == "bd_asm_pos") return &S.border.asm_pos;
+  if (w == "bd_ug_rp") return &S.border.ug_rp;
+  if (w == "bd_ug_pos") return &S.border.ug_pos;
   if (w == "ht_rp") return &S.Ht.rp;
   if (w == "ht_ci") return &S.Ht.ci;
   if (w == "hg_rp") return &S.Hg.rp;
@@ -839,6 +868,9 @@ extern "C" int hykkt_symbolic_create_ex(hykkt_symbolic_t* sym, int n_x, int m_c,
     CsrPattern Jd = make_pattern(m_d, n_x, jd_rowptr, jd_colidx, nnz_jd);
     SymbolicOptions opt = default_options(ordering);
     apply_solve_piece(opt, solve_piece);
+    // the task-queue layout, or what a plan takes with HYKKT_BORDERED=1
+    const char* e = std::getenv("HYKKT_BORDERED");
+    opt.bordered = e && e[0] == '1' && border_allowed(solve_piece);
     auto h = std::make_unique<hykkt_symbolic_s>();
     h->S = build_symbolic(H, Ds, Jc, Jd, opt, perm);
     *sym = h.release();
@@ -1099,8 +1131,10 @@ extern "C" int hykkt_solver_execute(hykkt_solver_t s) {
       CsrPattern Ds = make_pattern(s->Ds.n, s->Ds.m, s->Ds.rp, s->Ds.ci, s->Ds.nnz);
       CsrPattern Jc = make_pattern(s->Jc.n, s->Jc.m, s->Jc.rp, s->Jc.ci, s->Jc.nnz);
       CsrPattern Jd = make_pattern(s->Jd.n, s->Jd.m, s->Jd.rp, s->Jd.ci, s->Jd.nnz);
-      Symbolic S = build_symbolic(H, Ds, Jc, Jd, default_options(s->ordering), nullptr);
-      s->eng = std::make_unique<Engine>(std::move(S), s->gamma, default_options(s->ordering));
+      SymbolicOptions opt = default_options(s->ordering);
+      opt.bordered = border_allowed(0);
+      Symbolic S = build_symbolic(H, Ds, Jc, Jd, opt, nullptr);
+      s->eng = std::make_unique<Engine>(std::move(S), s->gamma, opt);
       s->eng->set_accuracy(s->cg_itmax, s->cg_rtol, s->refine_max, s->refine_target);
       s->snapshot(s->snap);
     } else {
@@ -1268,7 +1302,9 @@ extern "C" int hykkt_chol_create(hykkt_chol_t* c, int n, int nnz, const int* row
     Ds.rp.assign(1, 0);
     Jd.n = 0; Jd.m = n; Jd.rp.assign(1, 0);
     Jc.n = 0; Jc.m = n; Jc.rp.assign(1, 0);
-    Symbolic S = build_symbolic(A, Ds, Jc, Jd, default_options(ordering), nullptr);
+    SymbolicOptions opt = default_options(ordering);
+    opt.bordered = border_allowed(0);
+    Symbolic S = build_symbolic(A, Ds, Jc, Jd, opt, nullptr);
     auto h = std::make_unique<hykkt_chol_s>();
     h->n = n;
     h->nnz = nnz;
@@ -1285,7 +1321,7 @@ extern "C" int hykkt_chol_create(hykkt_chol_t* c, int n, int nnz, const int* row
         if (it == end || *it != a) throw std::runtime_error("chol: entry not in pattern");
         h->entry_to_lp[p] = (int)(it - S.lp_row.data());
       }
-    h->eng = std::make_unique<Engine>(std::move(S), 0.0, default_options(ordering));
+    h->eng = std::make_unique<Engine>(std::move(S), 0.0, opt);
     HYKKT_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     *c = h.release();
     return HYKKT_OK;

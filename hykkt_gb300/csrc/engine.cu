@@ -14,11 +14,15 @@
 #include <stdexcept>
 #include <vector>
 
+#include "bordered.cuh"
 #include "kernels.cuh"
 
 namespace hykkt {
 
 void raise_front_small_smem(int bytes);
+
+// shared memory of k_block_sweep for fronts of n rows
+static int block_smem(int n) { return (n * (n + 1) / 2 + 256) * 8 + 256 * 2; }
 
 std::mutex& cuda_setup_mutex() {
   static std::mutex m;
@@ -89,7 +93,7 @@ Engine::Engine(Symbolic&& S, double gamma, const SymbolicOptions& opt, bool defe
     : S_(std::move(S)), opt_(opt), gamma_(gamma) {
   // Front arena in level order: small fronts then large fronts of each level,
   // so the large fronts of one level form one contiguous range (one memset).
-  {
+  if (!S_.border.on) {
     int64_t off = 0;
     std::vector<int64_t> noff(S_.nsn + 1, 0);
     for (int l = 0; l < S_.nlevels; ++l) {
@@ -167,6 +171,7 @@ void Engine::release_device() {
     dp = DevPlan{};
     copy_settings(keep, dp);
     sched_ = SolveSched{};
+    bord_ = DevBorder{};
     resident_ = false;
   }
   free_storage(mine);
@@ -319,6 +324,11 @@ void Engine::upload_all() {
   d.perm = dev_upload(A, B, S.perm); d.rev_perm = dev_upload(A, B, S.rev_perm);
   d.jcp_ci = dev_upload(A, B, S.jcp_ci);
   d.jctp_rp = dev_upload(A, B, S.jctp_rp); d.jctp_ci = dev_upload(A, B, S.jctp_ci); d.jctp_src = dev_upload(A, B, S.jctp_src);
+  if (S.border.on) {
+    dp = d;
+    upload_border();
+    d = dp;
+  } else {
   d.nsn = S.nsn;
   d.sn_first = dev_upload(A, B, S.sn_first); d.sn_nrows = dev_upload(A, B, S.sn_nrows);
   d.sn_rp = dev_upload(A, B, S.sn_rp); d.sn_rows = dev_upload(A, B, S.sn_rows);
@@ -496,6 +506,8 @@ void Engine::upload_all() {
     d_pack_b_ = dev_upload(A, B, pack_b);
   }
 
+  }  // task-queue layout
+
   // ---- vectors ---------------------------------------------------------------
   d.rxp = dev_alloc<double>(A, B, S.n_x);
   d.hrxp = dev_alloc<double>(A, B, S.n_x);
@@ -525,7 +537,11 @@ void Engine::upload_all() {
   dp = d;
 
   HYKKT_CUDA(cudaFuncSetAttribute(k_piece_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem));
-  raise_front_small_smem(max_small_smem_);
+  HYKKT_CUDA(cudaFuncSetAttribute(k_block_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, block_smem(kBlkRows)));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_update, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
+  if (!S.border.on) raise_front_small_smem(max_small_smem_);
 
   // pinned staging for host inputs / outputs (kept while device storage is released)
   if (g_count_only || pin_in_) return;
@@ -534,6 +550,79 @@ void Engine::upload_all() {
   pin_out_n_ = (int64_t)S.n_x + 2LL * S.m_d + S.m_c + 16;
   HYKKT_CUDA(cudaMallocHost(&pin_out_, pin_out_n_ * sizeof(double)));
   HYKKT_CUDA(cudaMallocHost(&pin_sc_, sizeof(DevScalars)));
+}
+
+// Device storage and lists of the bordered layout.
+void Engine::upload_border() {
+  const Bordered& S = S_.border;
+  auto& A = allocs_;
+  int64_t& B = dev_bytes_;
+  DevBorder b{};
+  b.k = S.k;
+  b.ld = cdiv(S.k, kRowBlock) * kRowBlock;
+  b.npan = cdiv(S.k, kBorderPanel);
+  b.nblk = S.nblk;
+  b.nbig = S.nbig;
+  b.nasm = (int)S.asm_row.size();
+  b.bcol = dev_upload(A, B, S.bcol);
+  b.blk_rp = dev_upload(A, B, S.blk_rp); b.blk_col = dev_upload(A, B, S.blk_col);
+  b.blk_rrp = dev_upload(A, B, S.blk_rrp); b.blk_row = dev_upload(A, B, S.blk_row);
+  b.ge_off = dev_upload(A, B, S.ge_off); b.et_off = dev_upload(A, B, S.et_off); b.c_off = dev_upload(A, B, S.c_off);
+  b.ent_rp = dev_upload(A, B, S.ent_rp); b.ent_q = dev_upload(A, B, S.ent_q); b.ent_pos = dev_upload(A, B, S.ent_pos);
+  b.asm_row = dev_upload(A, B, S.asm_row); b.asm_col = dev_upload(A, B, S.asm_col);
+  b.asm_src = dev_upload(A, B, S.asm_src); b.asm_rp = dev_upload(A, B, S.asm_rp); b.asm_pos = dev_upload(A, B, S.asm_pos);
+  b.u_off = dev_upload(A, B, S.u_off); b.ug_rp = dev_upload(A, B, S.ug_rp); b.ug_pos = dev_upload(A, B, S.ug_pos);
+  b.ge = dev_alloc<double>(A, B, S.ge_off[S.nblk]);
+  b.et = dev_alloc<double>(A, B, S.et_off[S.nblk]);
+  b.cb = dev_alloc<double>(A, B, S.c_off[S.nblk]);
+  b.W = dev_alloc<double>(A, B, (int64_t)b.ld * b.ld);
+  // products of the solves: with four rows a panel a border of up to 1,536
+  // columns runs in one wave of short tasks; above, eight
+  b.rb = S.k <= 1536 ? 4 : 8;
+  b.nrb = cdiv(S.k, b.rb);
+  b.nseg = cdiv(S.k, kGemvSeg);
+  for (int q = 0; q < b.nseg; ++q) b.n_lo += b.nrb - q * kGemvSeg / b.rb;
+  b.n_up = b.n_lo;
+  b.part = dev_alloc<double>(A, B, (int64_t)b.nrb * b.nseg * b.rb);
+  b.rowcnt = dev_alloc<int>(A, B, b.nrb);
+  b.xlo = dev_alloc<double>(A, B, panel_lo(b.nrb, b.rb));
+  b.xup = dev_alloc<double>(A, B, panel_up(b.nrb, b.nrb, b.rb));
+  b.dig = dev_alloc<uint8_t>(A, B, (int64_t)b.ld / kRowBlock * kDigitBlockBytes);
+  b.ey = dev_alloc<int>(A, B, b.ld);
+  b.piv = dev_alloc<double>(A, B, kBorderPanel * (kBorderPanel + 2));
+  b.u = dev_alloc<double>(A, B, S.u_off[S.nblk]);
+  b.y = dev_alloc<double>(A, B, (int64_t)S.blk_col.size());
+  std::vector<int> fpb, fpf, bpb, bpf;
+  for (int i = 0; i < S.nbig; ++i) {
+    const int nt = S.blk_rp[i + 1] - S.blk_rp[i], R = S.blk_rrp[i + 1] - S.blk_rrp[i];
+    fpf.push_back((int)fpb.size());
+    bpf.push_back((int)bpb.size());
+    fpb.insert(fpb.end(), cdiv(nt + R, 64), i);
+    bpb.insert(bpb.end(), cdiv(nt, 64), i);
+  }
+  b.nfp = (int)fpb.size();
+  b.nbp = (int)bpb.size();
+  b.fp_blk = dev_upload(A, B, fpb); b.fp_first = dev_upload(A, B, fpf);
+  b.bp_blk = dev_upload(A, B, bpb); b.bp_first = dev_upload(A, B, bpf);
+  b.bt = dev_alloc<double>(A, B, b.ld);
+  b.by = dev_alloc<double>(A, B, b.ld);
+  const int nm = cdiv(S_.m_c, kCgRows);
+  b.r2 = dev_alloc<double>(A, B, S_.m_c);
+  b.s2 = dev_alloc<double>(A, B, S_.m_c);
+  b.rrp = dev_alloc<double>(A, B, nm);
+  b.dlp = dev_alloc<double>(A, B, cdiv(S_.m_c, kRowTask));
+  b.ctl = dev_alloc<unsigned long long>(A, B, kCtlWords);
+  // blocks by front size, so that small fronts share an SM
+  blk_class_.assign(1, 0);
+  int i = 0;
+  for (int most : {128, 64, 0}) {
+    while (i < S.nblk && S.blk_rp[i + 1] - S.blk_rp[i] + S.blk_rrp[i + 1] - S.blk_rrp[i] > most) ++i;
+    blk_class_.push_back(i);
+  }
+  int dev = 0;
+  HYKKT_CUDA(cudaGetDevice(&dev));
+  HYKKT_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
+  bord_ = b;
 }
 
 // A kernel's dynamic shared-memory limit is one value per device for the
@@ -642,7 +731,72 @@ void Engine::record_numeric(cudaStream_t st) {
   }
 }
 
+// Bordered layout: the blocks' sweeps, the border's assembly and its sweep by
+// panels, one panel and one update launch each (the update's first tile
+// prepares the next panel's pivot block).
+void Engine::record_border_factor(cudaStream_t st) {
+  const Bordered& S = S_.border;
+  const DevPlan& d = dp;
+  const DevBorder& b = bord_;
+  for (size_t c = 0; c + 1 < blk_class_.size(); ++c) {
+    const int b0 = blk_class_[c], nb = blk_class_[c + 1] - b0;
+    if (!nb) continue;
+    const int N = S.blk_rp[b0 + 1] - S.blk_rp[b0] + S.blk_rrp[b0 + 1] - S.blk_rrp[b0];
+    LAUNCH(k_block_sweep, nb, N > 128 ? 256 : N > 64 ? 128 : 64, block_smem(N), st, d, b, b0);
+  }
+  HYKKT_CUDA(cudaMemsetAsync(b.W, 0, (size_t)b.ld * b.ld * sizeof(double), st));
+  LAUNCH(k_border_assemble, std::max(1, std::min(cdiv(b.nasm, kBlock), 152 * 16)), kBlock, 0, st, d, b);
+  LAUNCH(k_border_pivot0, 1, 256, 0, st, d, b);
+  const int nrb = cdiv(b.k, kRowBlock);
+  const int tiles = 2 * (nrb - 1) * nrb + std::min(4 * nrb, b.npan);
+  for (int p = 0; p < b.npan; ++p) {
+    LAUNCH(k_border_panel, b.ld / 8, 128, 0, st, d, b, p);
+    const int rb = (p + 1) / 4;  // row blocks below the panel
+    if (p + 1 < b.npan) LAUNCH(k_border_update, tiles - 2 * rb * (rb + 1), 256, kUpdateSmem, st, d, b, p);
+  }
+  const int nt = cdiv(b.k, 64);
+  LAUNCH(k_border_pack, nt * (nt + 1) / 2, 256, 0, st, b);
+  if (prof_) {
+    const double k = b.k;
+    prof_work("k_border_update", 2.0 / 3.0 * k * k * k, 16.0 / 3.0 * k * (k + 1) * b.npan);
+  }
+}
+
+// x = Hgamma^-1 b, or (cg) the whole CG loop from its start vectors.
+void Engine::record_border_solve(cudaStream_t st, const double* rhs, double* x, int use_stop, bool cg) {
+  const DevPlan& d = dp;
+  const DevBorder& b = bord_;
+  BorderTasks t{};
+  t.n_fwd = b.nfp + cdiv(b.nblk - b.nbig, 8);
+  t.n_upd = cg ? cdiv(d.m_c, kCgRows) : 0;
+  const int rhs_tasks = cdiv(b.k, kRowTask);
+  t.n[0] = t.n_fwd + t.n_upd + (t.n_fwd ? 0 : rhs_tasks);
+  t.n[1] = t.n_fwd ? rhs_tasks : 0;
+  t.n[2] = b.n_lo;
+  t.n[3] = b.n_up;
+  t.n[4] = b.nbp + cdiv(b.nblk - b.nbig, 8);
+  t.n[5] = cg ? cdiv(d.m_c, kRowTask) : 0;
+  for (int q = 0, last = 0; q < 6; ++q) {
+    t.off[q + 1] = t.off[q] + t.n[q];
+    t.dep[q] = last;
+    if (t.n[q]) last = q;
+  }
+  HYKKT_CUDA(cudaMemsetAsync(b.ctl, 0, kCtlWords * sizeof(unsigned long long), st));
+  // three CTAs per SM; with CTAs for all tasks (and, in the loop, the next
+  // iteration's) each one waits for its phase with its data at hand
+  const int grid = std::min(cg ? 2 * t.off[6] : t.off[6], std::max(16, sms_ * 3 / share_));
+  if (cg) {
+    LAUNCH(k_border_solve<true>, grid, 256, kSolveSmem, st, d, b, t, rhs, x, use_stop);
+  } else {
+    LAUNCH(k_border_solve<false>, grid, 256, kSolveSmem, st, d, b, t, rhs, x, use_stop);
+  }
+}
+
 void Engine::record_factor(cudaStream_t st) {
+  if (S_.border.on) {
+    record_border_factor(st);
+    return;
+  }
   const Symbolic& S = S_;
   const DevPlan& d = dp;
   int step = 0;
@@ -732,6 +886,10 @@ void Engine::record_factor(cudaStream_t st) {
 // `reset` clears both first (a pair that does not follow a pair of the same
 // loop body).
 void Engine::record_trisolve(cudaStream_t st, const double* b, double* x, int use_stop, bool reset) {
+  if (S_.border.on) {
+    record_border_solve(st, b, x, use_stop, false);
+    return;
+  }
   const Symbolic& S = S_;
   const DevPlan& d = dp;
   if (reset) HYKKT_CUDA(cudaMemsetAsync(sched_.cnt, 0, cnt_ints_ * sizeof(int), st));
@@ -886,9 +1044,14 @@ void Engine::capture_graph() {
   int before = kernels_per_solve_;
   auto cg_body = [this](cudaStream_t s, cudaGraphConditionalHandle h) { record_cg_body(s, h, true); };
   auto cg_arm = [this](cudaStream_t s, cudaGraphConditionalHandle h) { LAUNCH(k_cond_arm, 1, 1, 0, s, h); };
-  capture_while(st, body_stream_, 0, cg_arm, cg_body);
-  kernels_per_iter_ = kernels_per_solve_ - before - 1;  // the arming kernel runs once
-  kernels_per_solve_ = before + 1;
+  if (S_.border.on) {
+    record_border_solve(st, nullptr, dp.cg_z, 1, true);  // the loop is one launch
+    kernels_per_iter_ = 0;
+  } else {
+    capture_while(st, body_stream_, 0, cg_arm, cg_body);
+    kernels_per_iter_ = kernels_per_solve_ - before - 1;  // the arming kernel runs once
+    kernels_per_solve_ = before + 1;
+  }
   record_post(st, 0);
   if (dp.refine_max > 0) {
     // iterative refinement on the full KKT system, reusing the factorization
@@ -898,7 +1061,8 @@ void Engine::capture_graph() {
     auto body = [this, cg_body, cg_arm](cudaStream_t s, cudaGraphConditionalHandle h) {
       record_correction_rhs(s);
       record_cg_pre(s, 1);
-      capture_while(s, body_stream2_, 0, cg_arm, cg_body);
+      if (S_.border.on) record_border_solve(s, nullptr, dp.cg_z, 1, true);
+      else capture_while(s, body_stream2_, 0, cg_arm, cg_body);
       record_post(s, 1);
       LAUNCH(k_refine_cond, 1, 1, 0, s, dp, h);
     };
@@ -912,6 +1076,10 @@ void Engine::capture_graph() {
 
 // Host-driven CG loop of the uncaptured path.
 void Engine::direct_cg_loop(cudaStream_t st) {
+  if (S_.border.on) {
+    record_border_solve(st, nullptr, dp.cg_z, 1, true);
+    return;
+  }
   bool done = false;
   for (int it = 0; it < dp.cg_itmax; ++it) {
     record_cg_body(st, 0, false);
@@ -970,6 +1138,7 @@ int Engine::run_direct(cudaStream_t st, int upto, float* stage_ms) {
 // part of them (at least 16 CTAs) when `share` plans solve at once, so that
 // the plans' solve kernels can be resident together.
 void Engine::size_solve_grids() {
+  if (S_.border.on) return;  // ordinary launches, no persistent kernels
   const int f = std::max(16, sms_ * occ_f_ / share_), b = std::max(16, sms_ * occ_b_ / share_);
   grid_f_ = std::max(1, std::min(sched_.ntasks_f, f));
   grid_b_ = std::max(1, std::min(sched_.ntasks_b, b));
@@ -1145,6 +1314,8 @@ float Engine::time_trisolve_group(const std::vector<Engine*>& es, int nrep, int 
   const int n = (int)es.size();
   if (n == 0) return 0.0f;
   for (Engine* e : es)
+    if (e->S_.border.on) throw std::invalid_argument("group solve timing needs plans of the task-queue layout");
+  for (Engine* e : es)
     if (e->sched_.ntasks_f != es[0]->sched_.ntasks_f || e->sched_.ntasks_b != es[0]->sched_.ntasks_b)
       throw std::invalid_argument("plans of different patterns");
   std::vector<DevPlan> hd(n);
@@ -1232,7 +1403,8 @@ void Engine::trace_trisolve(cudaStream_t st, std::vector<unsigned long long>& ou
   (void)st, (void)out;
   throw std::invalid_argument("the solve timeline is in measurement builds only (HYKKT_MEASURE=1)");
 #else
-  const int64_t n = 4LL * (sched_.ntasks_f + sched_.ntasks_b);
+  const int n_blk = bord_.nfp + bord_.nbp + 2 * cdiv(bord_.nblk - bord_.nbig, 8);
+  const int64_t n = S_.border.on ? 4LL * (n_blk + cdiv(bord_.k, kRowTask) + bord_.n_lo + bord_.n_up) : 4LL * (sched_.ntasks_f + sched_.ntasks_b);
   unsigned long long* buf = nullptr;
   HYKKT_CUDA(cudaMallocAsync(&buf, std::max<int64_t>(n, 1) * sizeof(unsigned long long), st));
   HYKKT_CUDA(cudaMemsetAsync(buf, 0, std::max<int64_t>(n, 1) * sizeof(unsigned long long), st));
@@ -1276,7 +1448,7 @@ int Engine::factor_values(const double* lower_vals_host, cudaStream_t st) {
   HYKKT_CUDA(cudaMemcpyAsync(pin_sc_, dp.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, st));
   HYKKT_CUDA(cudaStreamSynchronize(st));
   last_sc_ = *pin_sc_;
-  last_status_ = last_sc_.pivot_col != INT_MAX ? ST_NOT_SPD : ST_OK;
+  last_status_ = last_sc_.solve_flags & 1 ? ST_TIMEOUT : last_sc_.pivot_col != INT_MAX ? ST_NOT_SPD : ST_OK;
   return last_status_;
 }
 

@@ -169,6 +169,35 @@ struct SolveSched {
   int* cnt;  // [head_f, head_b, diag_cnt, g_done, inv_done, bg_cnt (nchunks), bd_cnt, red_done, invt_done, panel_f, panel_b]
 };
 
+// Device view of the bordered layout (Bordered in symbolic.hpp, bordered.cuh).
+struct DevBorder {
+  int k, ld, npan;  // ld: k rounded up to 128, npan: 32-column panels
+  int nblk, nbig, nasm;
+  const int* bcol;
+  const int *blk_rp, *blk_col, *blk_rrp, *blk_row;
+  const int64_t *ge_off, *et_off, *c_off;
+  const int *ent_rp, *ent_q, *ent_pos;
+  const int *asm_row, *asm_col, *asm_src, *asm_rp, *asm_pos;
+  const int *u_off, *ug_rp, *ug_pos;
+  double *ge, *et, *cb;  // blocks: [X; E], [-E^T X^T], border updates
+  double* W;             // border, ld x ld column-major: its lower triangle becomes X = L^-1
+  double *xlo, *xup;     // row panels of X and X^T (k_border_pack)
+  uint8_t* dig;          // digits of the current panel's Y (bordered.cuh)
+  int* ey;               // row exponents of the digits
+  double* piv;           // the panel's pivot block: L^-1, 1/D, 1/sqrt(D)
+  double *u, *bt, *by;   // per solve: E b_F of the blocks, the border's right-hand side, X times it
+  double* y;             // per solve: X b_F of the blocks, in block order
+  int nfp, nbp;          // 64-row panels of the blocks of more than 32 rows: [X; E], [-E^T X^T]
+  const int *fp_blk, *fp_first, *bp_blk, *bp_first;  // their blocks, and each block's first panel
+  int rb, nrb;           // rows per panel, panels
+  int n_lo, n_up, nseg;  // tasks of the two products, most tasks per panel
+  double* part;          // sums of the panels with several tasks
+  int* rowcnt;
+  double *r2, *s2;       // CG residual and direction of every second iteration
+  double *rrp, *dlp;     // CG partial sums
+  unsigned long long* ctl;  // task counters of one launch
+};
+
 // Work lists of the blocked inversion of the large items' diagonal blocks,
 // per 32-row step.
 struct InverseWork {
@@ -287,6 +316,9 @@ class Engine {
   void alloc_and_upload();
   cudaStream_t begin_upload();
   void upload_all();
+  void upload_border();
+  void record_border_factor(cudaStream_t st);
+  void record_border_solve(cudaStream_t st, const double* b, double* x, int use_stop, bool cg);
   void wait_last_launch();
   static void copy_settings(const DevPlan& from, DevPlan& to);
   int64_t size_bytes_ = 0;
@@ -324,6 +356,8 @@ class Engine {
   std::vector<const int*> d_ea_sn_, d_ea_row0_;
   std::vector<int> n_ea_;
   SolveSched sched_{};
+  DevBorder bord_{};
+  std::vector<int> blk_class_;  // blocks by front size: launches of one shared-memory size each
   int64_t cnt_ints_ = 0;
   int grid_f_ = 1, grid_b_ = 1;
   int sms_ = 1, occ_f_ = 1, occ_b_ = 1, share_ = 1;

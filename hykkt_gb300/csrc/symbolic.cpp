@@ -3,6 +3,8 @@
 #include "symbolic.hpp"
 
 #include <algorithm>
+#include <climits>
+#include <cstdint>
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
@@ -114,6 +116,208 @@ ProductUnion product_union(const CsrPattern& base, const CsrPattern& B, const Tr
 }
 
 }  // namespace
+
+// ---------------------------------------------------------------------------
+// Bordered layout: where to cut, and its lists.
+// ---------------------------------------------------------------------------
+namespace {
+// The cut that keeps every subtree whose front (its columns and the border
+// rows its top column reaches) has at most `most` rows: block of each column
+// (-1: border), top column of each block.  Front sizes grow towards the root,
+// so the border is closed under parents.
+struct Cut {
+  std::vector<int> blk_of, top, ncols, nrows;
+  int nblk = 0, k = 0;
+};
+Cut cut_at(const Symbolic& S, int most) {
+  const int n = S.n_x;
+  Cut c;
+  c.blk_of.assign(n, -1);
+  std::vector<int> size(n, 1);
+  for (int j = 0; j < n; ++j)
+    if (S.parent[j] >= 0) size[S.parent[j]] += size[j];
+  for (int j = n - 1; j >= 0; --j) {
+    const int p = S.parent[j];
+    if (p >= 0 && c.blk_of[p] >= 0) {
+      c.blk_of[j] = c.blk_of[p];
+    } else if (size[j] + S.colcount[j] - 1 <= most) {
+      c.blk_of[j] = c.nblk++;
+      c.top.push_back(j);
+      c.ncols.push_back(size[j]);
+      c.nrows.push_back(S.colcount[j] - 1);
+    } else {
+      c.k++;
+    }
+  }
+  return c;
+}
+
+// Estimated microseconds of one factorization and kSolves triangular solve
+// pairs.  FP64 multiply-adds run at 6.3e5 per us on the whole GPU.
+constexpr double kFmaPerUs = 6.3e5, kSolves = 100;
+double border_cost(const Cut& c) {
+  const double k = c.k, panels = k / kBorderPanel;
+  double sweep = 0.0;  // the largest front's columns, one after the other
+  for (int b = 0; b < c.nblk; ++b) sweep = std::max(sweep, 0.5 * c.ncols[b] + 4e-3 * c.ncols[b] * c.nrows[b]);
+  return panels * (16.0 + 1.3 * k * k / kFmaPerUs) + sweep + kSolves * (1.2 * k * k / kFmaPerUs + (c.nblk ? 14.0 : 6.0));
+}
+double queue_cost(double stored, int levels, double flops) {
+  return 1.3 * 0.5 * flops / kFmaPerUs + 150.0 * levels + kSolves * (2.6 * stored / kFmaPerUs + 13.0 * levels);
+}
+}  // namespace
+
+// Cuts the factor for the bordered layout when that is estimated to be the
+// faster one.  Larger blocks leave a smaller border (its work grows as k^3 and
+// k^2), smaller ones a shorter sweep of the largest block; no blocks at all
+// (everything in the border) saves the block phases of every solve, which is
+// worth it for small systems.
+static bool choose_border(Symbolic& S, int levels, double flops) {
+  const int n = S.n_x;
+  Cut c;
+  double cost = 0.0;
+  for (int most : {kBlkRows, 176, 128, 96, 64, 32, 0}) {
+    Cut t = cut_at(S, most);
+    const double ct = border_cost(t);
+    if (most == kBlkRows || ct < cost) {
+      cost = ct;
+      c = std::move(t);
+    }
+  }
+  const int64_t k = c.k;
+  if (k == 0 || k > 65536 || cost > queue_cost((double)S.L_stored, levels, flops)) return false;
+  int64_t upd = 0;
+  for (int b = 0; b < c.nblk; ++b) upd += (int64_t)c.nrows[b] * (c.nrows[b] + 1) / 2;
+  if (upd >= INT32_MAX) return false;
+
+  Bordered& B = S.border;
+  B = Bordered();
+  B.k = (int)k;
+  B.nblk = c.nblk;
+  std::vector<int> order(c.nblk), pos(c.nblk);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int a, int b) { return c.ncols[a] + c.nrows[a] > c.ncols[b] + c.nrows[b]; });
+  B.blk_rp.assign(c.nblk + 1, 0);
+  B.blk_rrp.assign(c.nblk + 1, 0);
+  B.ge_off.assign(c.nblk + 1, 0);
+  B.et_off.assign(c.nblk + 1, 0);
+  B.c_off.assign(c.nblk + 1, 0);
+  B.u_off.assign(c.nblk + 1, 0);
+  for (int i = 0; i < c.nblk; ++i) {
+    const int b = order[i];
+    pos[b] = i;
+    const int64_t nt = c.ncols[b], R = c.nrows[b];
+    if (nt + R > 32) B.nbig = i + 1;
+    B.blk_rp[i + 1] = B.blk_rp[i] + (int)nt;
+    B.blk_rrp[i + 1] = B.blk_rrp[i] + (int)R;
+    B.ge_off[i + 1] = B.ge_off[i] + (nt + R + 63) / 64 * 64 * nt;
+    B.et_off[i + 1] = B.et_off[i] + (nt + 63) / 64 * 64 * (nt + R);
+    B.c_off[i + 1] = B.c_off[i] + R * (R + 1) / 2;
+    B.u_off[i + 1] = B.u_off[i] + (int)R;
+  }
+  B.blk_col.resize(n - k);
+  std::vector<int> bpos(n, -1);  // position of a border column
+  {
+    std::vector<int> nx(B.blk_rp.begin(), B.blk_rp.end() - 1);
+    for (int j = 0; j < n; ++j) {
+      if (c.blk_of[j] >= 0) {
+        B.blk_col[nx[pos[c.blk_of[j]]]++] = j;
+      } else {
+        bpos[j] = (int)B.bcol.size();
+        B.bcol.push_back(j);
+      }
+    }
+  }
+  // border rows, entries and update positions block by block
+  B.blk_row.reserve(B.blk_rrp[c.nblk]);
+  B.ent_rp.assign(c.nblk + 1, 0);
+  std::vector<int> local(n, -1), rows;
+  std::vector<std::vector<std::pair<int, int>>> into(B.k);  // per border column: (row, update position)
+  for (int i = 0; i < c.nblk; ++i) {
+    const int nt = B.blk_rp[i + 1] - B.blk_rp[i];
+    const int* cols = B.blk_col.data() + B.blk_rp[i];
+    rows.clear();
+    for (int t = 0; t < nt; ++t) {
+      local[cols[t]] = t;
+      for (int q = S.lp_cp[cols[t]]; q < S.lp_cp[cols[t] + 1]; ++q) {
+        const int r = S.lp_row[q];
+        if (bpos[r] >= 0 && local[r] < 0) {
+          local[r] = 0;
+          rows.push_back(r);
+        }
+      }
+    }
+    std::sort(rows.begin(), rows.end());
+    const int R = (int)rows.size();
+    if (R != B.blk_rrp[i + 1] - B.blk_rrp[i]) throw std::runtime_error("bordered layout: block rows differ from the column counts");
+    for (int a = 0; a < R; ++a) {
+      local[rows[a]] = nt + a;
+      B.blk_row.push_back(bpos[rows[a]]);
+      const int base = (int)B.c_off[i] + a * (a + 1) / 2;
+      for (int b = 0; b <= a; ++b) into[bpos[rows[b]]].push_back({bpos[rows[a]], base + b});
+    }
+    for (int t = 0; t < nt; ++t)
+      for (int q = S.lp_cp[cols[t]]; q < S.lp_cp[cols[t] + 1]; ++q) {
+        const int r = local[S.lp_row[q]];
+        B.ent_q.push_back(q);
+        B.ent_pos.push_back(r * (r + 1) / 2 + t);
+      }
+    B.ent_rp[i + 1] = (int)B.ent_q.size();
+    for (int r : rows) local[r] = -1;
+  }
+  // border entries, column by column: rows ascending, a row's block updates
+  // in block order (they were appended so), its original value first
+  B.asm_rp.assign(1, 0);
+  for (int j = 0; j < B.k; ++j) {
+    auto& v = into[j];
+    const int col = B.bcol[j], q0 = S.lp_cp[col], q1 = S.lp_cp[col + 1];
+    std::stable_sort(v.begin(), v.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+    size_t e = 0;
+    int q = q0;
+    while (e < v.size() || q < q1) {
+      const int rv = e < v.size() ? v[e].first : INT32_MAX, rq = q < q1 ? bpos[S.lp_row[q]] : INT32_MAX;
+      const int r = std::min(rv, rq);
+      B.asm_row.push_back(r);
+      B.asm_col.push_back(j);
+      B.asm_src.push_back(rq == r ? q++ : -1);
+      for (; e < v.size() && v[e].first == r; ++e) B.asm_pos.push_back(v[e].second);
+      B.asm_rp.push_back((int)B.asm_pos.size());
+    }
+    std::vector<std::pair<int, int>>().swap(v);
+  }
+  B.ug_rp.assign(B.k + 1, 0);
+  for (int r : B.blk_row) B.ug_rp[r + 1]++;
+  for (int j = 0; j < B.k; ++j) B.ug_rp[j + 1] += B.ug_rp[j];
+  B.ug_pos.resize(B.blk_row.size());
+  {
+    std::vector<int> nx(B.ug_rp.begin(), B.ug_rp.end() - 1);
+    for (size_t e = 0; e < B.blk_row.size(); ++e) B.ug_pos[nx[B.blk_row[e]]++] = (int)e;
+  }
+  B.on = true;
+  return true;
+}
+
+static void build_jc_permuted(Symbolic& S) {
+  const int n = S.n_x;
+  // ---- permuted Jc structures for the Schur CG -------------------------------
+  S.jcp_ci.resize(S.nnz_jc);
+  for (int p = 0; p < S.nnz_jc; ++p) S.jcp_ci[p] = S.rev_perm[S.Jc.ci[p]];
+  S.jctp_rp.assign(n + 1, 0);
+  for (int i = 0; i < n; ++i) {
+    int o = S.perm[i];
+    S.jctp_rp[i + 1] = S.jctp_rp[i] + (S.JcT.pat.rp[o + 1] - S.JcT.pat.rp[o]);
+  }
+  S.jctp_ci.resize(S.nnz_jc);
+  S.jctp_src.resize(S.nnz_jc);
+  for (int i = 0; i < n; ++i) {
+    int o = S.perm[i];
+    int d = S.jctp_rp[i];
+    for (int p = S.JcT.pat.rp[o]; p < S.JcT.pat.rp[o + 1]; ++p, ++d) {
+      S.jctp_ci[d] = S.JcT.pat.ci[p];
+      S.jctp_src[d] = S.JcT.src[p];
+    }
+  }
+}
 
 Symbolic build_symbolic(const CsrPattern& H, const CsrPattern& Ds, const CsrPattern& Jc,
                         const CsrPattern& Jd, const SymbolicOptions& opt, const int* user_perm) {
@@ -393,6 +597,35 @@ Symbolic build_symbolic(const CsrPattern& H, const CsrPattern& Ds, const CsrPatt
   for (int J = 0; J < nsn; ++J)
     for (int c = S.sn_first[J]; c < S.sn_first[J + 1]; ++c) S.sn_of[c] = J;
 
+  if (opt.bordered && n > 0) {
+    phase("border");
+    // estimated cost of the task-queue layout: levels of the supernodal tree
+    // and stored entries (front sizes from the amalgamation)
+    std::vector<int> lvl(nsn, 0);
+    int nlv = 0;
+    S.L_stored = 0;
+    double flops = 0;
+    for (int J = 0; J < nsn; ++J) {
+      const int last = S.sn_first[J + 1] - 1, nc = last + 1 - S.sn_first[J];
+      const double nr = nc - 1 + S.colcount[last];
+      S.L_stored += (int64_t)nr * nc;
+      flops += nr * nr * nc;
+      nlv = std::max(nlv, lvl[J] + 1);
+      if (S.parent[last] >= 0) {
+        int& p = lvl[S.sn_of[S.parent[last]]];
+        p = std::max(p, lvl[J] + 1);
+      }
+    }
+    if (choose_border(S, nlv, flops)) {
+      S.nlevels = S.nsq_levels = S.border.nblk ? 2 : 1;
+      S.nsq = S.border.nblk + 1;
+      S.L_stored = (int64_t)S.border.k * S.border.k + S.border.ge_off.back();
+      build_jc_permuted(S);
+      phase("");
+      return S;
+    }
+  }
+
   phase("rows");
   // ---- rows(J) = cols(J) U struct(L(:, last(J))) ------------------------------
   {
@@ -570,24 +803,7 @@ Symbolic build_symbolic(const CsrPattern& H, const CsrPattern& Ds, const CsrPatt
   build_solve_schedule(S, opt.chunk_fma, opt.unit_cols, opt.warp_subtree);
 
   phase("jc");
-  // ---- permuted Jc structures for the Schur CG -------------------------------
-  S.jcp_ci.resize(S.nnz_jc);
-  for (int p = 0; p < S.nnz_jc; ++p) S.jcp_ci[p] = S.rev_perm[Jc.ci[p]];
-  S.jctp_rp.assign(n + 1, 0);
-  for (int i = 0; i < n; ++i) {
-    int o = S.perm[i];
-    S.jctp_rp[i + 1] = S.jctp_rp[i] + (S.JcT.pat.rp[o + 1] - S.JcT.pat.rp[o]);
-  }
-  S.jctp_ci.resize(S.nnz_jc);
-  S.jctp_src.resize(S.nnz_jc);
-  for (int i = 0; i < n; ++i) {
-    int o = S.perm[i];
-    int d = S.jctp_rp[i];
-    for (int p = S.JcT.pat.rp[o]; p < S.JcT.pat.rp[o + 1]; ++p, ++d) {
-      S.jctp_ci[d] = S.JcT.pat.ci[p];
-      S.jctp_src[d] = S.JcT.src[p];
-    }
-  }
+  build_jc_permuted(S);
   phase("");
   return S;
 }

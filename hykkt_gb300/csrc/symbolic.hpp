@@ -50,6 +50,29 @@ struct SymbolicOptions {
   int chunk_fma = 4096;      // multiply-adds of one triangular-solve product task (sets rows per task)
   int unit_cols = 1024;      // columns of one unit of a staged item's panel product (64..kMaxUnitCols)
   int warp_subtree = 16;     // most items of one warp-subtree task (< 2: no subtree tasks; <= kMaxSubtree)
+  bool bordered = false;     // plans: the bordered layout where its estimated time is lower (choose_border)
+};
+
+// Bordered layout (bordered.cuh): the columns near the roots of the
+// elimination tree form one dense border (bcol, ascending), the subtrees below
+// them are the blocks.  A block's front holds its columns (blk_col, ascending)
+// and its border rows (blk_row, border positions, ascending).
+constexpr int kBlkRows = 232;      // most rows of a block front: its packed triangle fits one CTA's shared memory
+constexpr int kBorderPanel = 32;   // columns swept at a time in the border
+struct Bordered {
+  bool on = false;
+  int k = 0;          // border columns
+  std::vector<int> bcol;
+  int nblk = 0;       // blocks, by falling front size
+  int nbig = 0;       // blocks of more than 32 rows
+  std::vector<int> blk_rp, blk_col, blk_rrp, blk_row;
+  std::vector<int64_t> ge_off, et_off, c_off;  // per block: [X; E] and [-E^T X^T] in 64-row panels, border update (nblk + 1)
+  std::vector<int> ent_rp, ent_q, ent_pos;     // per block: lower entries and their packed front positions
+  // border entries with an original value (asm_src, -1: none) or block
+  // updates (positions in the update arena, blocks ascending)
+  std::vector<int> asm_row, asm_col, asm_src, asm_rp, asm_pos;
+  std::vector<int> u_off;                      // per block: first entry in the solve's update vector
+  std::vector<int> ug_rp, ug_pos;              // per border column: update entries
 };
 
 // Work item lists for one tree level of the factorization.
@@ -213,6 +236,10 @@ struct Symbolic {
   std::vector<int> bd_need;
   // task queues: kind, item, argument (chunk id, first column, first row or warp group)
   std::vector<int> tf_kind, tf_item, tf_arg, tb_kind, tb_item, tb_arg;
+
+  // set (on) for a plan that takes the bordered layout: the supernode rows,
+  // fronts and solve items above are then not built
+  Bordered border;
 
   // Jc with permuted column indices (Jc_p = Jc P^T, values in Jc order)
   std::vector<int> jcp_ci;
