@@ -29,58 +29,133 @@ void map_index(int n, const int* d_map, const double* d_old, double* d_new, cuda
   HYKKT_CUDA(cudaGetLastError());
 }
 
-// One warp per row of [A B^T; B 0]; the same operation order as the
-// product path (1/sqrt of the row max, v *= s_i*s_j).
-__global__ void k_ruizc_rowmax(int n, int m, const double* a_v, const int* a_i, const double* bt_v, const int* bt_i,
-                               const double* b_v, const int* b_i, double* scale) {
-  const int lane = threadIdx.x & 31;
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (row >= n + m) return;
-  double ml = 0.0, mu = 0.0;
-  if (row < n) {
-    for (int p = a_i[row] + lane; p < a_i[row + 1]; p += 32) { double e = fabs(a_v[p]); if (e > ml) ml = e; }
-    for (int p = bt_i[row] + lane; p < bt_i[row + 1]; p += 32) { double e = fabs(bt_v[p]); if (e > mu) mu = e; }
-  } else {
-    const int k = row - n;
-    for (int p = b_i[k] + lane; p < b_i[k + 1]; p += 32) { double e = fabs(b_v[p]); if (e > ml) ml = e; }
-  }
+// Ruiz sweeps on [A B^T; B 0], eight lanes per row (the rows of power-grid
+// blocks hold 2 to 16 entries: a warp each left most lanes idle); the same
+// operation order as the product path (1/sqrt of the row max, v *= s_i*s_j).
+// Bounded by latency and launches, not by the 10 MB that a 10,000-bus system
+// moves.
+constexpr int kRuizLanes = 8;
+
+struct RuizArrays {
+  int n, m;
+  double* a_v;
+  const int *a_i, *a_j;
+  double* bt_v;
+  const int *bt_i, *bt_j;
+  double* b_v;
+  const int *b_i, *b_j;
+  double *rhs1, *rhs2, *max_d;
+};
+
+// 1/sqrt of the row's largest magnitude, from the lanes' own maxima (a NaN
+// never compares greater, as in the reference's kernel)
+__device__ __forceinline__ double ruiz_row_scale(double ml, double mu, bool top) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    double a = __shfl_xor_sync(0xffffffffu, ml, o), b = __shfl_xor_sync(0xffffffffu, mu, o);
+  for (int o = kRuizLanes / 2; o > 0; o >>= 1) {
+    const double a = __shfl_xor_sync(0xffffffffu, ml, o), b = __shfl_xor_sync(0xffffffffu, mu, o);
     if (a > ml) ml = a;
     if (b > mu) mu = b;
   }
-  if (lane == 0) scale[row] = 1.0 / sqrt(row < n ? (ml > mu ? ml : mu) : ml);
+  return 1.0 / sqrt(top ? (ml > mu ? ml : mu) : ml);
 }
 
-__global__ void k_ruizc_scale(int n, int m, double* a_v, const int* a_i, const int* a_j, double* bt_v, const int* bt_i,
-                              const int* bt_j, double* b_v, const int* b_i, const int* b_j, const double* scale,
-                              double* rhs1, double* rhs2, double* max_d) {
-  const int lane = threadIdx.x & 31;
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (row >= n + m) return;
-  const double si = scale[row];
-  if (row < n) {
-    for (int p = a_i[row] + lane; p < a_i[row + 1]; p += 32) a_v[p] = __dmul_rn(a_v[p], __dmul_rn(si, scale[a_j[p]]));
-    for (int p = bt_i[row] + lane; p < bt_i[row + 1]; p += 32)
-      bt_v[p] = __dmul_rn(bt_v[p], __dmul_rn(si, scale[n + bt_j[p]]));
-    if (lane == 0) {
-      rhs1[row] = __dmul_rn(rhs1[row], si);
-      max_d[row] = __dmul_rn(max_d[row], si);
+__global__ void k_ruizc_rowmax(RuizArrays r, double* scale) {
+  const int lane = threadIdx.x & (kRuizLanes - 1);
+  const int row = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kRuizLanes);
+  const bool in = row < r.n + r.m, top = row < r.n;
+  double ml = 0.0, mu = 0.0;
+  if (in) {
+    const double* v = top ? r.a_v : r.b_v;
+    const int* rp = top ? r.a_i + row : r.b_i + (row - r.n);
+    for (int p = rp[0] + lane; p < rp[1]; p += kRuizLanes) { const double e = fabs(v[p]); if (e > ml) ml = e; }
+    if (top)
+      for (int p = r.bt_i[row] + lane; p < r.bt_i[row + 1]; p += kRuizLanes) { const double e = fabs(r.bt_v[p]); if (e > mu) mu = e; }
+  }
+  const double s = ruiz_row_scale(ml, mu, top);
+  if (in && lane == 0) scale[row] = s;
+}
+
+// One sweep's scaling.  first: max_d starts from it (reset_scaling,
+// RuizClass.cpp:95-98, sets 1).  next (optional): the row scales of the sweep
+// that follows, from the values just written, which saves that sweep's own
+// pass and launch.
+__global__ void k_ruizc_scale(RuizArrays r, const double* __restrict__ scale, double* next, int first) {
+  const int lane = threadIdx.x & (kRuizLanes - 1);
+  const int row = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kRuizLanes);
+  const bool in = row < r.n + r.m, top = row < r.n;
+  double ml = 0.0, mu = 0.0;
+  if (in) {
+    const double si = scale[row];
+    double* v = top ? r.a_v : r.b_v;
+    const int* ci = top ? r.a_j : r.b_j;
+    const int* rp = top ? r.a_i + row : r.b_i + (row - r.n);
+    for (int p = rp[0] + lane; p < rp[1]; p += kRuizLanes) {
+      const double x = __dmul_rn(v[p], __dmul_rn(si, scale[ci[p]])), e = fabs(x);
+      v[p] = x;
+      if (e > ml) ml = e;
     }
-  } else {
-    const int k = row - n;
-    for (int p = b_i[k] + lane; p < b_i[k + 1]; p += 32) b_v[p] = __dmul_rn(b_v[p], __dmul_rn(si, scale[b_j[p]]));
+    if (top)
+      for (int p = r.bt_i[row] + lane; p < r.bt_i[row + 1]; p += kRuizLanes) {
+        const double x = __dmul_rn(r.bt_v[p], __dmul_rn(si, scale[r.n + r.bt_j[p]])), e = fabs(x);
+        r.bt_v[p] = x;
+        if (e > mu) mu = e;
+      }
     if (lane == 0) {
-      rhs2[k] = __dmul_rn(rhs2[k], si);
-      max_d[row] = __dmul_rn(max_d[row], si);
+      double* rhs = top ? r.rhs1 + row : r.rhs2 + (row - r.n);
+      *rhs = __dmul_rn(*rhs, si);
+      r.max_d[row] = first ? si : __dmul_rn(r.max_d[row], si);
     }
   }
+  if (!next) return;
+  const double s = ruiz_row_scale(ml, mu, top);
+  if (in && lane == 0) next[row] = s;
 }
 
 __global__ void k_fill(int n, double v, double* x) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) x[i] = v;
+}
+
+// scale1 (optional): a second scale vector, for the fused sweeps
+static void ruiz_sweeps(int its, const RuizArrays& r, double* scale0, double* scale1, cudaStream_t st) {
+  const int tot = r.n + r.m;
+  if (its == 0) {
+    k_fill<<<(tot + 255) / 256, 256, 0, st>>>(tot, 1.0, r.max_d);
+  }
+  const int grid = (int)(((int64_t)tot * kRuizLanes + 255) / 256);
+  for (int s = 0; s < its; ++s) {
+    if (s == 0 || !scale1) k_ruizc_rowmax<<<grid, 256, 0, st>>>(r, scale0);
+    k_ruizc_scale<<<grid, 256, 0, st>>>(r, scale0, scale1 && s + 1 < its ? scale1 : nullptr, s == 0);
+    if (scale1) std::swap(scale0, scale1);
+  }
+  HYKKT_CUDA(cudaGetLastError());
+}
+
+// A pool of the library's own for the component's scratch, one per device:
+// with the default pool every call that is followed by a synchronisation gives
+// the memory back to the device and takes it again (300 us of a 340 us call on
+// the 10,000-bus system).  It keeps at most kRuizPoolKeep bytes between calls;
+// allocations are stream-ordered, so calls on several streams and threads each
+// have their own.
+constexpr uint64_t kRuizPoolKeep = 32ull << 20;
+static cudaMemPool_t ruiz_pool_on_current_device() {
+  static std::mutex mu;
+  static std::unordered_map<int, cudaMemPool_t> pools;
+  int dev = 0;
+  HYKKT_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = pools.find(dev);
+  if (it != pools.end()) return it->second;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  HYKKT_CUDA(cudaMemPoolCreate(&pool, &props));
+  uint64_t keep = kRuizPoolKeep;
+  HYKKT_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  pools[dev] = pool;
+  return pool;
 }
 
 void ruiz_scale(int its, int n, int m, double* a_v, const int* a_i, const int* a_j, double* bt_v, const int* bt_i,
@@ -90,14 +165,10 @@ void ruiz_scale(int its, int n, int m, double* a_v, const int* a_i, const int* a
   const int tot = n + m;
   if (tot <= 0) return;
   double* scale = nullptr;
-  HYKKT_CUDA(cudaMallocAsync(&scale, tot * sizeof(double), st));
-  k_fill<<<(tot + 255) / 256, 256, 0, st>>>(tot, 1.0, max_d);  // reset_scaling (RuizClass.cpp:95-98)
-  const int grid = (int)(((int64_t)tot * 32 + 255) / 256);
-  for (int s = 0; s < its; ++s) {
-    k_ruizc_rowmax<<<grid, 256, 0, st>>>(n, m, a_v, a_i, bt_v, bt_i, b_v, b_i, scale);
-    k_ruizc_scale<<<grid, 256, 0, st>>>(n, m, a_v, a_i, a_j, bt_v, bt_i, bt_j, b_v, b_i, b_j, scale, rhs1, rhs2, max_d);
-  }
-  HYKKT_CUDA(cudaGetLastError());
+  HYKKT_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scale), 2 * (size_t)tot * sizeof(double),
+                                     ruiz_pool_on_current_device(), st));
+  ruiz_sweeps(its, RuizArrays{n, m, a_v, a_i, a_j, bt_v, bt_i, bt_j, b_v, b_i, b_j, rhs1, rhs2, max_d}, scale,
+              scale + tot, st);
   HYKKT_CUDA(cudaFreeAsync(scale, st));
 }
 
@@ -154,13 +225,8 @@ void ruiz_scale_noalloc(int its, int n, int m, double* a_v, const int* a_i, cons
                                 " exceeds the fixed scratch of " + std::to_string(kRuizNoAllocMaxRows) + " rows");
   double* scale = ruiz_scratch_on_current_device();
   if (tot == 0) return;
-  k_fill<<<(int)((tot + 255) / 256), 256, 0, st>>>((int)tot, 1.0, max_d);  // reset_scaling (RuizClass.cpp:95-98)
-  const int grid = (int)((tot * 32 + 255) / 256);
-  for (int s = 0; s < its; ++s) {
-    k_ruizc_rowmax<<<grid, 256, 0, st>>>(n, m, a_v, a_i, bt_v, bt_i, b_v, b_i, scale);
-    k_ruizc_scale<<<grid, 256, 0, st>>>(n, m, a_v, a_i, a_j, bt_v, bt_i, bt_j, b_v, b_i, b_j, scale, rhs1, rhs2, max_d);
-  }
-  HYKKT_CUDA(cudaGetLastError());
+  ruiz_sweeps(its, RuizArrays{n, m, a_v, a_i, a_j, bt_v, bt_i, bt_j, b_v, b_i, b_j, rhs1, rhs2, max_d}, scale,
+              nullptr, st);
 }
 
 // FP64 throughput probe: 8 independent FMA chains per thread.
