@@ -152,10 +152,10 @@ constexpr int kTileCols = 32;                                     // columns of 
 constexpr int kAccs = 8;                                          // digit weights kept
 constexpr int kTmemCols = kAccs * kTileCols;
 constexpr int kBPlaneBytes = kTileCols * kBorderPanel * 2;
-// two CTAs per SM (their accumulators fill the 512 tensor-memory columns):
-// more than a third of the SM's shared memory keeps a third one out
-constexpr int kUpdateSmem = 78 * 1024;
-static_assert(kDigitBlockBytes + kDigits * kBPlaneBytes + 1024 <= kUpdateSmem, "update tiles must fit");
+// row digits and two buffers of column digits; two CTAs per SM (their sums
+// fill the 512 tensor-memory columns, their shared memory keeps a third out)
+constexpr int kUpdateSmem = kDigitBlockBytes + 2 * kDigits * kBPlaneBytes;
+static_assert(3 * kUpdateSmem > 227 * 1024, "a third CTA would wait for tensor memory");
 constexpr int kExpZero = -100000, kExpNan = 1000000;  // row exponents of rows that are zero / not finite
 constexpr unsigned kMbarLimit = 1u << 22;
 
@@ -204,31 +204,52 @@ __device__ __forceinline__ double pow2_or_nan(int e) {
 
 // L D L^T of a 32 x 32 diagonal block (lower triangle in A, row stride 33) by
 // 256 threads: M = L^-1 (unit lower), the reciprocals of D and of its roots.
-// Gauss elimination applied to [A I], two barriers per pivot.  It runs in the
-// update kernel's first tile (the one that completes the block), beside the
-// other tiles, so that the panel kernel starts with M ready.
+// Gauss elimination of [A I].  FP64 instructions are what it costs (a warp's
+// takes 64 clocks of its quarter of the SM), so the elements of a step are
+// packed onto the threads, and warp 0 runs ahead on the next pivot's column
+// (one multiply-add, reciprocal, multipliers) while the others finish the
+// step.  It runs in the update kernel's first CTA (the one that completes the
+// block), beside the others, so that the panel kernel starts with M ready.
 __device__ void pivot_block(DevPlan& d, const DevBorder& bd, int panel, double* A, double* M) {
   constexpr int n = kBorderPanel, ld = n + 1;
-  __shared__ double sinv[n];
-  const int tid = threadIdx.x;
+  __shared__ double sinv[n], mult[2][n];
+  const int tid = threadIdx.x, lane = tid & 31;
   for (int e = tid; e < n * n; e += 256) M[(e / n) * ld + e % n] = e / n == e % n ? 1.0 : 0.0;
   __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    if (tid == 0) {
-      const double p = A[k * ld + k];
+  // warp 0, lane i: pivot k's multipliers A(i,k) / A(k,k) from the column c
+  auto pivot = [&](int k, double c) {
+    const double p = __shfl_sync(0xffffffffu, c, k);
+    const double inv = 1.0 / p;
+    mult[k & 1][lane] = c * inv;
+    if (lane == 0) {
       const int col = panel * n + k;
       if (col < bd.k) note_pivot(d, bd.bcol[col], p);
-      sinv[k] = 1.0 / p;
+      sinv[k] = inv;
     }
-    __syncthreads();
-    const double inv = sinv[k];
-    // row i > k: columns j in (k, i] of A and j <= k of M; eight threads per row
-    const int i = tid >> 3, part = tid & 7;
-    if (i > k) {
-      const double l = A[i * ld + k] * inv;
-      for (int j = part; j <= i; j += 8) {
-        if (j > k) A[i * ld + j] = fma(-l, A[j * ld + k], A[i * ld + j]);
-        else M[i * ld + j] = fma(-l, M[k * ld + j], M[i * ld + j]);
+  };
+  if (tid < 32) pivot(0, A[lane * ld]);
+  __syncthreads();
+  for (int k = 0; k < n - 1; ++k) {
+    const double* l = mult[k & 1];
+    if (tid < 32) {
+      // column k + 1, then its pivot
+      double c = 0.0;
+      if (lane > k) {
+        c = fma(-l[lane], A[(k + 1) * ld + k], A[lane * ld + k + 1]);
+        A[lane * ld + k + 1] = c;
+      }
+      pivot(k + 1, c);
+    } else {
+      // rows i > k, i + 1 entries each without column k + 1: j <= k of M, j > k + 1 of A
+      const int first = k + 1, count = n * (n - 1) / 2 - first * (first - 1) / 2;
+      for (int e = tid - 32; e < count; e += 224) {
+        const int f = e + first * (first - 1) / 2;
+        int i = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)f)) * 0.5f);
+        if (i * (i - 1) / 2 > f) --i;
+        if ((i + 1) * i / 2 <= f) ++i;
+        const int t = f - i * (i - 1) / 2, j = t <= k ? t : t + 1;  // t < i
+        double* g = j <= k ? &M[i * ld + j] : &A[i * ld + j];
+        *g = fma(-l[i], j <= k ? M[k * ld + j] : A[j * ld + k], *g);
       }
     }
     __syncthreads();
@@ -345,122 +366,142 @@ __global__ void __launch_bounds__(128) k_border_panel(DevPlan d, DevBorder bd, i
   if (tid < 8) bd.ey[r0 + tid] = ex[tid];
 }
 
-// A -= Y Y^T on one 128 x 32 tile of the rows below the panel.  Bounded by the
-// epilogue's FP64 work (three operations an element; the 34 digit products
-// take a quarter of that on the tensor cores) and by the read and write of
-// A; two CTAs an SM overlap one's loads and products with the other's
-// epilogue.
+// A -= Y Y^T on kRun 128 x 32 tiles of a row block below the panel.  Bounded
+// by the epilogue's FP64 work (three operations an element) and by the read and
+// write of A.  A CTA keeps the row block's digits for its run of tiles and
+// fetches the next tile's 14 KB of column digits while it works on one; two
+// CTAs an SM overlap one's products with the other's epilogue.  The column
+// digits lie below one another in shared memory and the sums of a weight beside
+// one another in tensor memory, so that one instruction multiplies a row digit
+// with all column digits it is kept with (14 + 2 instructions instead of 68).
+template <int kRun>
 __global__ void __launch_bounds__(256, 2) k_border_update(DevPlan d, DevBorder bd, int p) {
   extern __shared__ __align__(1024) uint8_t usm[];
-  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ __align__(8) uint64_t bars[4];  // row digits, column digits (two buffers), products
   __shared__ uint32_t tmem_at;
-  __shared__ int ecol[kTileCols];
-  const int pn = p + 1;  // the next panel: its diagonal tile comes first, then its pivot block
-  const int t_0 = 2 * (pn / 4) * (pn / 4 + 1), t_next = t_0 + pn;  // tiles of the row blocks above: none
+  static_assert(kRun == 1 || kRun == 2 || kRun == 4, "runs end with the row block");
+  const int pn = p + 1;  // the next panel: the run with its diagonal tile comes first, then its pivot block
+  constexpr int kPer = 4 / kRun;  // runs per 128 columns
+  const int rb0 = pn / 4, t_0 = kPer * (rb0 * (rb0 + 1) / 2), t_next = t_0 + pn / kRun;  // row blocks above: none
   int t = t_0 + (int)blockIdx.x;
   t = t == t_0 ? t_next : t == t_next ? t_0 : t;
-  int rb = (int)((sqrtf(1.0f + 2.0f * (float)t) - 1.0f) * 0.5f);
-  while (2 * rb * (rb + 1) > t) --rb;
-  while (2 * (rb + 1) * (rb + 2) <= t) ++rb;
-  const int cb = t - 2 * rb * (rb + 1);
-  if (cb == p) return;  // the panel itself
+  int rb = (int)((sqrtf(1.0f + 8.0f / kPer * (float)t) - 1.0f) * 0.5f);
+  while (kPer * (rb * (rb + 1) / 2) > t) --rb;
+  while (kPer * ((rb + 1) * (rb + 2) / 2) <= t) ++rb;
+  const int cb0 = (t - kPer * (rb * (rb + 1) / 2)) * kRun;
+  // the run's tiles: inside the border, without the panel itself
+  const int cb1 = min(cb0 + kRun, bd.npan);
+  const int skip = p >= cb0 && p < cb1 ? p : -1;
+  const int ntile = cb1 - cb0 - (skip >= 0);
+  if (ntile <= 0) return;
+  auto tile_col = [&](int s) { return cb0 + s + (skip >= 0 && cb0 + s >= skip); };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sA = smem_addr(usm), sB = sA + kDigitBlockBytes;
-  const uint32_t bar_load = smem_addr(&bars[0]), bar_mma = smem_addr(&bars[1]);
+  const uint32_t bar_a = smem_addr(&bars[0]), bar_b = smem_addr(&bars[1]), bar_mma = smem_addr(&bars[3]);
+  auto load_b = [&](int s) {  // one thread
+    const int cb = tile_col(s);
+    const uint32_t bar = bar_b + 8 * (s & 1), dst = sB + (s & 1) * (kDigits * kBPlaneBytes);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kDigits * kBPlaneBytes) : "memory");
+    const uint8_t* gb = bd.dig + (int64_t)(cb >> 2) * kDigitBlockBytes + (cb & 3) * kBPlaneBytes;
+#pragma unroll
+    for (int q = 0; q < kDigits; ++q)
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       dst + q * kBPlaneBytes),
+                   "l"(gb + q * kPlaneBytes), "r"(kBPlaneBytes), "r"(bar) : "memory");
+  };
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_at)),
                  "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 32) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_load));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_mma));
+    for (int i = 0; i < 4; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a + 8 * i));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_load),
-                 "r"(kDigitBlockBytes + kDigits * kBPlaneBytes) : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_a), "r"(kDigitBlockBytes) : "memory");
     const uint8_t* ga = bd.dig + (int64_t)rb * kDigitBlockBytes;
-    const uint8_t* gb = bd.dig + (int64_t)(cb >> 2) * kDigitBlockBytes + (cb & 3) * kBPlaneBytes;
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sA),
-                 "l"(ga), "r"(kDigitBlockBytes), "r"(bar_load) : "memory");
-#pragma unroll
-    for (int q = 0; q < kDigits; ++q)
-      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                       sB + q * kBPlaneBytes),
-                   "l"(gb + q * kPlaneBytes), "r"(kBPlaneBytes), "r"(bar_load) : "memory");
+                 "l"(ga), "r"(kDigitBlockBytes), "r"(bar_a) : "memory");
+    load_b(0);
   }
-  if (tid >= 64 && tid < 64 + kTileCols) ecol[tid - 64] = bd.ey[cb * kTileCols + tid - 64];
-  // this thread's sixteen elements of A, on their way while the digits load
   const int quad = warp & 3, half = warp >> 2;
   const int row = rb * kRowBlock + quad * 32 + lane;
-  double* g = bd.W + (int64_t)(cb * kTileCols + half * 16) * bd.ld + row;
-  double a[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) a[j] = g[(int64_t)j * bd.ld];
   const int er = row < pn * kBorderPanel ? kExpZero : bd.ey[row] - 38;  // rows up to the panel are done
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_at;
-  if (tid == 0) {
-    bool ok = mbar_wait(bar_load, 0, d.sc);
-    if (!ok) ok = mbar_wait(bar_load, 0, d.sc);  // the copies in flight: once more, with a limit
-    if (d.dbg_unsatisfiable) mbar_wait_hook(bar_load, 1, d);
-    // D f32, A and B bf16, K-major both, M 128, N 32
-    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileCols / 8) << 17) | ((uint32_t)(kRowBlock / 16) << 24);
+  for (int s = 0; s < ntile; ++s) {
+    const int c0 = tile_col(s) * kTileCols + half * 16;
+    if (tid == 0) {
+      if (s + 1 < ntile) load_b(s + 1);
+      if (s == 0 && !mbar_wait(bar_a, 0, d.sc)) mbar_wait(bar_a, 0, d.sc);  // the copies in flight: once more, with a limit
+      if (!mbar_wait(bar_b + 8 * (s & 1), (s >> 1) & 1, d.sc)) mbar_wait(bar_b + 8 * (s & 1), (s >> 1) & 1, d.sc);
+      if (s == 0 && d.dbg_unsatisfiable) mbar_wait_hook(bar_a, 1, d);
+      // D f32, A and B bf16, K-major both, M 128, N 32 per column digit
+      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kRowBlock / 16) << 24);
+      auto mma = [&](int i, int j, int nj, int kk, uint32_t acc) {
+        const uint64_t da = operand_desc(sA + i * kPlaneBytes + kk * 256);
+        const uint64_t db = operand_desc(sB + (s & 1) * (kDigits * kBPlaneBytes) + j * kBPlaneBytes + kk * 256);
+        asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(
+                         tmem + (uint32_t)((i + j) * kTileCols)),
+                     "l"(da), "l"(db), "r"(idesc | ((uint32_t)(nj * kTileCols / 8) << 17)), "r"(acc) : "memory");
+      };
 #pragma unroll 1
-    for (int kk = 0; kk < 2; ++kk)
+      for (int kk = 0; kk < 2; ++kk) {
+        mma(0, 0, kDigits, kk, kk > 0);
+        mma(1, kDigits - 1, 1, kk, kk > 0);  // the last weight's first product
+        mma(1, 0, kDigits - 1, kk, 1);
 #pragma unroll 1
-      for (int i = 0; i < kDigits; ++i)
-#pragma unroll 1
-        for (int j = 0; j < kDigits && i + j < kAccs; ++j) {
-          const uint64_t da = operand_desc(sA + i * kPlaneBytes + kk * 256);
-          const uint64_t db = operand_desc(sB + j * kBPlaneBytes + kk * 256);
-          // first product of this weight: (0, w), or (1, 6) for weight 7
-          const uint32_t acc = kk > 0 || i > (i + j < kDigits ? 0 : i + j - (kDigits - 1));
-          asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(
-                           tmem + (uint32_t)((i + j) * kTileCols)),
-                       "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
-        }
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_mma) : "memory");
-    if (!mbar_wait(bar_mma, 0, d.sc)) mbar_wait(bar_mma, 0, d.sc);
-  }
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  // Per element the eight exact sums a_w of weight 2^(er + ec - 14 - 8 w) form
-  // hi 2^32 + lo with integers; as doubles through the bits of 1.5 * 2^52 + i,
-  // t = hi + lo 2^-32 is rounded once, and once more when it is subtracted.
-  const double kBiasHi = 6755399441055744.0 + 1572864.0;  // 1.5 * 2^52 and lo's bias 1.5 * 2^52 * 2^-32
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint32_t r[kAccs][8];
-#pragma unroll
-    for (int w = 0; w < kAccs; ++w) {
-      const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(w * kTileCols + half * 16 + h * 8);
-      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                   : "=r"(r[w][0]), "=r"(r[w][1]), "=r"(r[w][2]), "=r"(r[w][3]), "=r"(r[w][4]), "=r"(r[w][5]),
-                     "=r"(r[w][6]), "=r"(r[w][7])
-                   : "r"(ta));
+        for (int i = 2; i < kDigits; ++i) mma(i, 0, kAccs - i, kk, 1);
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_mma) : "memory");
     }
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    // this thread's sixteen elements of A, on their way meanwhile
+    double* g = bd.W + (int64_t)c0 * bd.ld + row;
+    double a[16];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      int s[kAccs];
+    for (int j = 0; j < 16; ++j) a[j] = g[(int64_t)j * bd.ld];
+    const int4* ecol = reinterpret_cast<const int4*>(bd.ey + c0);
+    if (!mbar_wait(bar_mma, s & 1, d.sc)) mbar_wait(bar_mma, s & 1, d.sc);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // Per element the eight exact sums a_w of weight 2^(er + ec - 14 - 8 w) form
+    // hi 2^32 + lo with integers; as doubles through the bits of 1.5 * 2^52 + i,
+    // t = hi + lo 2^-32 is rounded once, and once more when it is subtracted.
+    const double kBiasHi = 6755399441055744.0 + 1572864.0;  // 1.5 * 2^52 and lo's bias 1.5 * 2^52 * 2^-32
 #pragma unroll
-      for (int w = 0; w < kAccs; ++w)  // exact: |sum| <= 7 * 2^19 < 2^22
-        s[w] = __float_as_int(__uint_as_float(r[w][j]) + 12582912.0f) - 0x4B400000;
-      const long long hi = (long long)(s[0] * 256 + s[1]) * 65536 + (s[2] * 256 + s[3]);
-      const long long lo = (long long)(s[4] * 256 + s[5]) * 65536 + (s[6] * 256 + s[7]);
-      const double dh = __longlong_as_double(0x4338000000000000ll + hi) - kBiasHi;
-      const double t2 = fma(__longlong_as_double(0x4338000000000000ll + lo), 0x1p-32, dh);
-      const double sc = pow2_or_nan(er + ecol[half * 16 + h * 8 + j]);
-      a[h * 8 + j] = fma(-sc, t2, a[h * 8 + j]);
+    for (int h = 0; h < 2; ++h) {
+      uint32_t r[kAccs][8];
+#pragma unroll
+      for (int w = 0; w < kAccs; ++w) {
+        const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(w * kTileCols + half * 16 + h * 8);
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[w][0]), "=r"(r[w][1]), "=r"(r[w][2]), "=r"(r[w][3]), "=r"(r[w][4]), "=r"(r[w][5]),
+                       "=r"(r[w][6]), "=r"(r[w][7])
+                     : "r"(ta));
+      }
+      const int4 e0 = ecol[2 * h], e1 = ecol[2 * h + 1];
+      const int ec[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        int v[kAccs];
+#pragma unroll
+        for (int w = 0; w < kAccs; ++w)  // exact: |sum| <= 7 * 2^19 < 2^22
+          v[w] = __float_as_int(__uint_as_float(r[w][j]) + 12582912.0f) - 0x4B400000;
+        const long long hi = (long long)(v[0] * 256 + v[1]) * 65536 + (v[2] * 256 + v[3]);
+        const long long lo = (long long)(v[4] * 256 + v[5]) * 65536 + (v[6] * 256 + v[7]);
+        const double dh = __longlong_as_double(0x4338000000000000ll + hi) - kBiasHi;
+        const double t2 = fma(__longlong_as_double(0x4338000000000000ll + lo), 0x1p-32, dh);
+        a[h * 8 + j] = fma(-pow2_or_nan(er + ec[j]), t2, a[h * 8 + j]);
+      }
     }
-  }
 #pragma unroll
-  for (int j = 0; j < 16; ++j) g[(int64_t)j * bd.ld] = a[j];
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+    for (int j = 0; j < 16; ++j) g[(int64_t)j * bd.ld] = a[j];
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();  // the sums are read: the next tile's products may replace them
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
   if (blockIdx.x == 0 && pn < bd.npan) {

@@ -540,7 +540,9 @@ void Engine::upload_all() {
   HYKKT_CUDA(cudaFuncSetAttribute(k_block_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, block_smem(kBlkRows)));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
-  HYKKT_CUDA(cudaFuncSetAttribute(k_border_update, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_update<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_update<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_update<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
   if (!S.border.on) raise_front_small_smem(max_small_smem_);
 
   // pinned staging for host inputs / outputs (kept while device storage is released)
@@ -747,18 +749,23 @@ void Engine::record_border_factor(cudaStream_t st) {
   HYKKT_CUDA(cudaMemsetAsync(b.W, 0, (size_t)b.ld * b.ld * sizeof(double), st));
   LAUNCH(k_border_assemble, std::max(1, std::min(cdiv(b.nasm, kBlock), 152 * 16)), kBlock, 0, st, d, b);
   LAUNCH(k_border_pivot0, 1, 256, 0, st, d, b);
+  // tiles of a row block per CTA: runs of four where the panel's update still
+  // makes four waves of CTAs, single tiles for a small border
   const int nrb = cdiv(b.k, kRowBlock);
-  const int tiles = 2 * (nrb - 1) * nrb + std::min(4 * nrb, b.npan);
   for (int p = 0; p < b.npan; ++p) {
     LAUNCH(k_border_panel, b.ld / 8, 128, 0, st, d, b, p);
+    if (p + 1 == b.npan) break;
     const int rb = (p + 1) / 4;  // row blocks below the panel
-    if (p + 1 < b.npan) LAUNCH(k_border_update, tiles - 2 * rb * (rb + 1), 256, kUpdateSmem, st, d, b, p);
+    const int tri = nrb * (nrb + 1) / 2 - rb * (rb + 1) / 2;
+    if (tri >= 8 * sms_) LAUNCH(k_border_update<4>, tri, 256, kUpdateSmem, st, d, b, p);
+    else if (2 * tri >= 4 * sms_) LAUNCH(k_border_update<2>, 2 * tri, 256, kUpdateSmem, st, d, b, p);
+    else LAUNCH(k_border_update<1>, 4 * tri, 256, kUpdateSmem, st, d, b, p);
   }
   const int nt = cdiv(b.k, 64);
   LAUNCH(k_border_pack, nt * (nt + 1) / 2, 256, 0, st, b);
   if (prof_) {
     const double k = b.k;
-    prof_work("k_border_update", 2.0 / 3.0 * k * k * k, 16.0 / 3.0 * k * (k + 1) * b.npan);
+    prof_work("k_border_update<4>", 2.0 / 3.0 * k * k * k, 16.0 / 3.0 * k * (k + 1) * b.npan);
   }
 }
 
