@@ -920,6 +920,63 @@ __device__ __forceinline__ bool border_wait(const count_t* p, count_t need, cons
   return !*(volatile const count_t*)done;  // set before the count that a stopped CG publishes
 }
 
+// red[8] = the CTA's sum of v over every kStep-th lane (thread 0 reads it)
+template <int kStep>
+__device__ __forceinline__ void cta_sum(double v, double* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o >= kStep; o >>= 1) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  if (warp == 0) {
+    double t = lane < 8 ? red[lane] : 0.0;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t = dadd(t, __shfl_xor_sync(0xffffffffu, t, o));
+    if (lane == 0) red[8] = t;
+  }
+}
+
+// One thread, after the iteration's sums r.r and w.r: the recurrence for the
+// next iteration or the end of the loop, published through `ready`.  Every
+// iteration waits for this, and a division is 20 dependent FP64 instructions,
+// so the recurrence's divisions by the previous iteration's gamma and alpha
+// are products with reciprocals that were formed beside one another then, and
+// what only the end needs is computed there.
+__device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, double wr, int it, count_t* ready, count_t* done) {
+  DevScalars* S = d.sc;
+  double inv_gam, inv_alpha, stop2;
+  if (it == 0) {
+    const double thr = S->rtol_cur > 0.0 ? S->rtol_cur * sqrt(S->gam0) : d.cg_tol;
+    inv_gam = 1.0 / S->gam;
+    inv_alpha = 1.0 / S->alpha;
+    stop2 = thr * thr;
+    bd.scal[2] = stop2;
+  } else {
+    inv_gam = __ldcg(&bd.scal[0]);
+    inv_alpha = __ldcg(&bd.scal[1]);
+    stop2 = __ldcg(&bd.scal[2]);
+  }
+  const int stop = rr < stop2 || rr == 0.0 ? 1 : it + 1 >= d.cg_itmax ? 2 : 0;
+  if (!stop) {
+    const double beta = rr * inv_gam, den = fma(-(beta * rr), inv_alpha, wr), inv = 1.0 / rr;
+    *(volatile double*)&S->alpha = rr / den;
+    *(volatile double*)&S->beta = beta;
+    bd.scal[0] = inv;
+    bd.scal[1] = den * inv;
+  } else {
+    S->gam1 = rr;
+    S->delta = wr;
+    S->cg_err = sqrt(rr);
+    S->it = it + 1;
+    S->it_total += it + 1;
+    S->cond_calls = it + 1;
+    if (stop == 2) S->stop_main += 1;
+    S->stop = stop;
+    *(volatile count_t*)done = 1;
+  }
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(ready), "l"((count_t)(it + 1)) : "memory");
+}
+
 template <bool kCg>
 __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd, BorderTasks tk, const double* b, double* x, int use_stop) {
   extern __shared__ double sm[];
@@ -1004,8 +1061,8 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
         rout[k] = rn;
         part[0] = rn * rn;
       }
-      block_reduce_sum<1>(part, red);
-      if (threadIdx.x == 0) bd.rrp[c] = part[0];
+      cta_sum<1>(part[0], red);
+      if (threadIdx.x == 0) bd.rrp[c] = red[8];
     } else if (ph <= 1) {
       // bt = b_S - sum u (in phase 0 there are no blocks)
       const int j = (ph ? task : task - tk.n_fwd - tk.n_upd) * kRowTask + (threadIdx.x >> 2), sub = threadIdx.x & 3;
@@ -1045,8 +1102,8 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
         d.cg_w[k] = acc;
         part[0] = acc * r;
       }
-      block_reduce_sum<1>(part, red);
-      if (threadIdx.x == 0) bd.dlp[task] = part[0];
+      cta_sum<4>(part[0], red);
+      if (threadIdx.x == 0) bd.dlp[task] = red[8];
       scalars = true;
     }
     // done: the CTA's writes, then the count
@@ -1063,37 +1120,23 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     }
     __syncthreads();
     if (!last) continue;
-    // the last constraint task: both sums in task order, the recurrence and the
-    // stopping tests (k_spmv_jcp, k_cg_update)
-    double v[2] = {0.0, 0.0};
-    for (int i = threadIdx.x; i < tk.n_upd; i += 256) v[0] = dadd(v[0], __ldcg(&bd.rrp[i]));
-    for (int i = threadIdx.x; i < tk.n[5]; i += 256) v[1] = dadd(v[1], __ldcg(&bd.dlp[i]));
-    block_reduce_sum<2>(v, red);
-    if (threadIdx.x == 0) {
-      S->gam1 = v[0];
-      S->it += 1;
-      S->it_total += 1;
-      S->cg_err = sqrt(v[0]);
-      const double thr = S->rtol_cur > 0.0 ? S->rtol_cur * sqrt(S->gam0) : d.cg_tol;
-      int stop = 0;
-      if (S->cg_err < thr) stop = 1;
-      S->cond_calls += 1;
-      if (!stop && (S->it >= d.cg_itmax || S->cond_calls >= d.cg_itmax)) {
-        stop = 2;
-        S->stop_main += 1;
+    // the last constraint task: both sums in a fixed order, one warp each, the
+    // recurrence and the stopping tests (k_spmv_jcp, k_cg_update)
+    if (threadIdx.x < 64) {
+      const double* src = threadIdx.x < 32 ? bd.rrp : bd.dlp;
+      const int lane = threadIdx.x & 31, n = threadIdx.x < 32 ? tk.n_upd : tk.n[5];
+      double v = 0.0;
+      for (int i = lane; i < n; i += 128) {
+        double t[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) t[j] = i + 32 * j < n ? __ldcg(&src[i + 32 * j]) : 0.0;
+        v = dadd(v, dadd(dadd(t[0], t[1]), dadd(t[2], t[3])));
       }
-      S->delta = v[1];
-      if (!stop) {
-        const double gam = v[0], beta = gam / S->gam;
-        S->beta = beta;
-        S->gam = gam;
-        S->alpha = gam / (v[1] - beta * gam / S->alpha);
-      } else {
-        S->stop = stop;
-        *(volatile count_t*)done = 1;
-      }
-      asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(ready), "l"((count_t)(it + 1)) : "memory");
+      v = warp_sum(v);
+      if (lane == 0) red[threadIdx.x >> 5] = v;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) cg_scalars(d, bd, red[0], red[1], it, ready, done);
   }
 }
 

@@ -613,6 +613,7 @@ void Engine::upload_border() {
   b.s2 = dev_alloc<double>(A, B, S_.m_c);
   b.rrp = dev_alloc<double>(A, B, nm);
   b.dlp = dev_alloc<double>(A, B, cdiv(S_.m_c, kRowTask));
+  b.scal = dev_alloc<double>(A, B, 3);
   b.ctl = dev_alloc<unsigned long long>(A, B, kCtlWords);
   // blocks by front size, so that small fronts share an SM
   blk_class_.assign(1, 0);

@@ -195,6 +195,7 @@ struct DevBorder {
   int* rowcnt;
   double *r2, *s2;       // CG residual and direction of every second iteration
   double *rrp, *dlp;     // CG partial sums
+  double* scal;          // CG: 1/gamma, 1/alpha, the squared residual that stops
   unsigned long long* ctl;  // task counters of one launch
 };
 
