@@ -122,6 +122,15 @@ __global__ void k_border_assemble(DevPlan d, DevBorder bd) {
   for (int j = bd.k + tid; j < bd.npan * kBorderPanel; j += stride) bd.W[(int64_t)j * bd.ld + j] = 1.0;  // padding
 }
 
+// Schur plans (no blocks): the rows of Jc_p below the border's panels.  The
+// sweep turns [Hgamma Jc^T; Jc 0] into -S = -Jc Hgamma^-1 Jc^T below them.
+__global__ void k_border_constraints(DevPlan d, DevBorder bd) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= bd.mc) return;
+  double* W = bd.W + bd.npan * kBorderPanel + i;
+  for (int p = d.jc_rp[i]; p < d.jc_rp[i + 1]; ++p) W[(int64_t)d.jcp_ci[p] * bd.ld] = d.jc_s[p];
+}
+
 // ---------------------------------------------------------------------------
 // Border: Cholesky and the inverse of the factor in one sweep, 32 columns at
 // a time, in place: after panel p the rows up to it hold X = L^-1, the rows
@@ -388,9 +397,11 @@ __global__ void __launch_bounds__(256, 2) k_border_update(DevPlan d, DevBorder b
   int rb = (int)((sqrtf(1.0f + 8.0f / kPer * (float)t) - 1.0f) * 0.5f);
   while (kPer * (rb * (rb + 1) / 2) > t) --rb;
   while (kPer * ((rb + 1) * (rb + 2) / 2) <= t) ++rb;
-  const int cb0 = (t - kPer * (rb * (rb + 1) / 2)) * kRun;
-  // the run's tiles: inside the border, without the panel itself
-  const int cb1 = min(cb0 + kRun, bd.npan);
+  int cb0 = (t - kPer * (rb * (rb + 1) / 2)) * kRun;
+  // the run's tiles: without the panel itself; constraint rows (Schur plans)
+  // have no columns of X
+  const int cb1 = min(cb0 + kRun, bd.ncb);
+  if (rb * kRowBlock >= bd.npan * kBorderPanel) cb0 = max(cb0, pn);
   const int skip = p >= cb0 && p < cb1 ? p : -1;
   const int ntile = cb1 - cb0 - (skip >= 0);
   if (ntile <= 0) return;
@@ -936,13 +947,32 @@ __device__ __forceinline__ void cta_sum(double v, double* red) {
   }
 }
 
+// red[0], red[1] = the sums of the first n0 parts of r.r and n1 parts of w.r in
+// a fixed order, one warp each
+__device__ __forceinline__ void sum_parts(const DevBorder& bd, int n0, int n1, double* red) {
+  if (threadIdx.x < 64) {
+    const double* src = threadIdx.x < 32 ? bd.rrp : bd.dlp;
+    const int lane = threadIdx.x & 31, n = threadIdx.x < 32 ? n0 : n1;
+    double v = 0.0;
+    for (int i = lane; i < n; i += 128) {
+      double t[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) t[j] = i + 32 * j < n ? __ldcg(&src[i + 32 * j]) : 0.0;
+      v = dadd(v, dadd(dadd(t[0], t[1]), dadd(t[2], t[3])));
+    }
+    v = warp_sum(v);
+    if (lane == 0) red[threadIdx.x >> 5] = v;
+  }
+  __syncthreads();
+}
+
 // One thread, after the iteration's sums r.r and w.r: the recurrence for the
 // next iteration or the end of the loop, published through `ready`.  Every
 // iteration waits for this, and a division is 20 dependent FP64 instructions,
 // so the recurrence's divisions by the previous iteration's gamma and alpha
 // are products with reciprocals that were formed beside one another then, and
 // what only the end needs is computed there.
-__device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, double wr, int it, count_t* ready, count_t* done) {
+__device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, double wr, int it, int round, count_t* ready, count_t* done) {
   DevScalars* S = d.sc;
   double inv_gam, inv_alpha, stop2;
   if (it == 0) {
@@ -974,7 +1004,7 @@ __device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, dou
     S->stop = stop;
     *(volatile count_t*)done = 1;
   }
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(ready), "l"((count_t)(it + 1)) : "memory");
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(ready), "l"((count_t)round) : "memory");
 }
 
 template <bool kCg>
@@ -1122,21 +1152,180 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     if (!last) continue;
     // the last constraint task: both sums in a fixed order, one warp each, the
     // recurrence and the stopping tests (k_spmv_jcp, k_cg_update)
-    if (threadIdx.x < 64) {
-      const double* src = threadIdx.x < 32 ? bd.rrp : bd.dlp;
-      const int lane = threadIdx.x & 31, n = threadIdx.x < 32 ? tk.n_upd : tk.n[5];
-      double v = 0.0;
-      for (int i = lane; i < n; i += 128) {
-        double t[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) t[j] = i + 32 * j < n ? __ldcg(&src[i + 32 * j]) : 0.0;
-        v = dadd(v, dadd(dadd(t[0], t[1]), dadd(t[2], t[3])));
-      }
-      v = warp_sum(v);
-      if (lane == 0) red[threadIdx.x >> 5] = v;
+    sum_parts(bd, tk.n_upd, tk.n[5], red);
+    if (threadIdx.x == 0) cg_scalars(d, bd, red[0], red[1], it, it + 1, ready, done);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Schur plans: a small system's S = Jc Hgamma^-1 Jc^T itself, so that a CG
+// iteration is one product and one exchange of scalars instead of four
+// dependent phases.  (S comes out of the border's sweep as V^T V with
+// V = L^-1 Jc^T, which keeps the accuracy of the two triangular products.)
+// ---------------------------------------------------------------------------
+__host__ __device__ inline int64_t schur_panel(int64_t b, int rows, int mc) { return b * rows * mc; }
+
+// S in row panels of bd.srb rows, column after column, from the lower triangle
+// of -S; one CTA per 64 x 64 tile.
+__global__ void __launch_bounds__(256) k_schur_pack(DevBorder bd) {
+  __shared__ double tile[64][65];
+  int ti = (int)((sqrtf(1.0f + 8.0f * (float)blockIdx.x) - 1.0f) * 0.5f);
+  while (ti * (ti + 1) / 2 > (int)blockIdx.x) --ti;
+  while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.x) ++ti;
+  const int tj = blockIdx.x - ti * (ti + 1) / 2;
+  const int i0 = ti * 64, j0 = tj * 64, at = bd.npan * kBorderPanel, mc = bd.mc, rows = bd.srb;
+  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
+    const int i = e & 63, j = e >> 6;
+    if (i0 + i < mc && i0 + i >= j0 + j) {
+      const double v = -bd.W[(int64_t)(at + j0 + j) * bd.ld + at + i0 + i];
+      tile[j][i] = v;
+      if (ti == tj) tile[i][j] = v;
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
+    const int i = i0 + e % 64, j = j0 + e / 64;
+    if (i >= mc || j >= mc) continue;
+    bd.S[schur_panel(i / rows, rows, mc) + (int64_t)j * rows + i % rows] = tile[j - j0][i - i0];
+  }
+  if (ti == tj) return;
+  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
+    const int j = j0 + e % 64, i = i0 + e / 64;
+    if (i >= mc || j >= mc) continue;
+    bd.S[schur_panel(j / rows, rows, mc) + (int64_t)i * rows + j % rows] = tile[j - j0][i - i0];
+  }
+}
+
+// The whole CG run: round 0 takes r = b - S x0, round 1 w = S r, the others one
+// iteration each.  A task owns RB rows: it forms the updated residual of all
+// rows for its product (two multiply-adds each, cheaper than a phase of its
+// own), updates its own rows of the vectors, and leaves its part of w.r and
+// r.r.  Vectors that other tasks read are double-buffered.
+template <int RB>
+__global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, int tasks) {
+  extern __shared__ double sm[];
+  __shared__ double red[2];
+  __shared__ double sc2[2];
+  __shared__ int s_it, s_t, go, last;
+  __shared__ __align__(8) uint64_t bars[kStages];
+  DevScalars* S = d.sc;
+  if (*(volatile const int*)&S->stop) return;
+  Ring ring{smem_addr(bars), 0, 0};
+  count_t *head = bd.ctl, *ready = bd.ctl + kCtlReady, *done = bd.ctl + kCtlDone, *cnt = bd.ctl + kCtlCount;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ring.bar + 8 * i));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    s_it = 0;
+  }
+  const int mc = bd.mc;
+  count_t base = 0;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const count_t next = atomicAdd(head, count_t(1));
+      for (; next - base >= (count_t)tasks; base += tasks) ++s_it;
+      s_t = (int)(next - base);
     }
     __syncthreads();
-    if (threadIdx.x == 0) cg_scalars(d, bd, red[0], red[1], it, ready, done);
+    const int q = s_it, task = s_t, row = task * RB + threadIdx.x;
+    const bool own = threadIdx.x < RB && row < mc;
+    const Panel p{bd.S + schur_panel(task, RB, mc), RB * mc};
+    panel_start(ring, p, sm);
+    double* const rin = q & 1 ? bd.r2 : d.cg_r;
+    double* const rout = q & 1 ? d.cg_r : bd.r2;
+    double* const sin = q & 1 ? bd.s2 : d.cg_s;
+    double* const sout = q & 1 ? d.cg_s : bd.s2;
+    double* const win = q & 1 ? bd.w2 : d.cg_w;
+    double* const wout = q & 1 ? d.cg_w : bd.w2;
+    if (threadIdx.x == 0) {
+      const bool ok = border_wait(ready, (count_t)q, done, d);
+      go = ok;
+      if (!ok && (*(volatile int*)&S->solve_flags & 1)) {
+        *(volatile int*)&S->stop = 3;
+        *(volatile count_t*)done = 1;
+      }
+      sc2[0] = *(volatile double*)&S->alpha;
+      sc2[1] = *(volatile double*)&S->beta;
+    }
+    __syncthreads();
+    if (!go) {
+      panel_drain(ring, S);
+      return;
+    }
+    const double alpha = sc2[0], beta = sc2[1];
+    double* v = sm + kRed;
+    for (int h = threadIdx.x; h < mc; h += 4 * 256) {
+      double r[4], w[4], s[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int k = h + j * 256;
+        const bool in = k < mc;
+        r[j] = in ? (q ? __ldcg(&rin[k]) : __ldcg(&d.cg_x[k])) : 0.0;
+        w[j] = in && q > 1 ? __ldcg(&win[k]) : 0.0;
+        s[j] = in && q > 1 ? __ldcg(&sin[k]) : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (h + j * 256 < mc) v[h + j * 256] = q > 1 ? fma(-alpha, fma(beta, s[j], w[j]), r[j]) : r[j];
+    }
+    const double r0 = own ? __ldcg(&rin[row]) : 0.0, p0 = own ? __ldcg(&d.cg_p[row]) : 0.0, x0 = own ? __ldcg(&d.cg_x[row]) : 0.0;
+    double sv = 0.0;
+    if (own && q > 1) sv = fma(beta, __ldcg(&sin[row]), __ldcg(&win[row]));
+    __syncthreads();
+    const double t = panel_product<RB>(ring, p, sm, S);
+    double rr = 0.0, wr = 0.0;
+    if (own) {
+      double rn = r0;
+      if (q == 0) {
+        rn = dsub(r0, t);
+      } else {
+        wout[row] = t;
+        if (q > 1) {
+          rn = v[row];
+          const double pn = fma(beta, p0, r0);
+          d.cg_p[row] = pn;
+          d.cg_x[row] = fma(alpha, pn, x0);
+          sout[row] = sv;
+        }
+      }
+      rout[row] = rn;
+      rr = rn * rn;
+      wr = t * rn;
+    }
+    if (threadIdx.x < 32) {
+#pragma unroll
+      for (int o = RB / 2; o > 0; o >>= 1) {
+        rr = dadd(rr, __shfl_xor_sync(0xffffffffu, rr, o));
+        wr = dadd(wr, __shfl_xor_sync(0xffffffffu, wr, o));
+      }
+      if (threadIdx.x == 0) {
+        bd.rrp[task] = rr;
+        bd.dlp[task] = wr;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      count_t old;
+      asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], 1;" : "=l"(old) : "l"(cnt) : "memory");
+      last = old == (count_t)(q + 1) * tasks - 1;
+    }
+    __syncthreads();
+    if (!last) continue;
+    sum_parts(bd, tasks, tasks, red);
+    if (threadIdx.x == 0) {
+      if (q > 1) {
+        cg_scalars(d, bd, red[0], red[1], q - 2, q + 1, ready, done);
+      } else {
+        if (q == 0) {
+          S->gam = S->gam0 = red[0];
+        } else {
+          S->delta = red[1];
+          S->alpha = S->gam / red[1];
+          S->beta = 0.0;
+        }
+        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(ready), "l"((count_t)(q + 1)) : "memory");
+      }
+    }
   }
 }
 

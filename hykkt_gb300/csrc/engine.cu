@@ -538,6 +538,8 @@ void Engine::upload_all() {
 
   HYKKT_CUDA(cudaFuncSetAttribute(k_piece_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_block_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, block_smem(kBlkRows)));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_schur_cg<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_schur_cg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_update<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
@@ -561,8 +563,10 @@ void Engine::upload_border() {
   int64_t& B = dev_bytes_;
   DevBorder b{};
   b.k = S.k;
-  b.ld = cdiv(S.k, kRowBlock) * kRowBlock;
   b.npan = cdiv(S.k, kBorderPanel);
+  b.mc = S.schur ? S_.m_c : 0;
+  b.ncb = b.npan + cdiv(b.mc, kTileCols);
+  b.ld = cdiv(b.ncb * kBorderPanel, kRowBlock) * kRowBlock;
   b.nblk = S.nblk;
   b.nbig = S.nbig;
   b.nasm = (int)S.asm_row.size();
@@ -611,8 +615,13 @@ void Engine::upload_border() {
   const int nm = cdiv(S_.m_c, kCgRows);
   b.r2 = dev_alloc<double>(A, B, S_.m_c);
   b.s2 = dev_alloc<double>(A, B, S_.m_c);
-  b.rrp = dev_alloc<double>(A, B, nm);
-  b.dlp = dev_alloc<double>(A, B, cdiv(S_.m_c, kRowTask));
+  // Schur plans: four rows a task up to 640 constraints, else eight (a task
+  // forms the whole residual, which fewer rows repeat more often)
+  b.srb = S_.m_c <= 640 ? 4 : 8;
+  b.w2 = dev_alloc<double>(A, B, b.mc);
+  b.S = dev_alloc<double>(A, B, (int64_t)cdiv(b.mc, b.srb) * b.srb * b.mc);
+  b.rrp = dev_alloc<double>(A, B, std::max(nm, cdiv(b.mc, b.srb)));
+  b.dlp = dev_alloc<double>(A, B, std::max(cdiv(S_.m_c, kRowTask), cdiv(b.mc, b.srb)));
   b.scal = dev_alloc<double>(A, B, 3);
   b.ctl = dev_alloc<unsigned long long>(A, B, kCtlWords);
   // blocks by front size, so that small fronts share an SM
@@ -749,13 +758,14 @@ void Engine::record_border_factor(cudaStream_t st) {
   }
   HYKKT_CUDA(cudaMemsetAsync(b.W, 0, (size_t)b.ld * b.ld * sizeof(double), st));
   LAUNCH(k_border_assemble, std::max(1, std::min(cdiv(b.nasm, kBlock), 152 * 16)), kBlock, 0, st, d, b);
+  if (b.mc) LAUNCH(k_border_constraints, cdiv(b.mc, 128), 128, 0, st, d, b);
   LAUNCH(k_border_pivot0, 1, 256, 0, st, d, b);
   // tiles of a row block per CTA: runs of four where the panel's update still
   // makes four waves of CTAs, single tiles for a small border
-  const int nrb = cdiv(b.k, kRowBlock);
+  const int nrb = b.ld / kRowBlock;
   for (int p = 0; p < b.npan; ++p) {
     LAUNCH(k_border_panel, b.ld / 8, 128, 0, st, d, b, p);
-    if (p + 1 == b.npan) break;
+    if (p + 1 == b.npan && !b.mc) break;
     const int rb = (p + 1) / 4;  // row blocks below the panel
     const int tri = nrb * (nrb + 1) / 2 - rb * (rb + 1) / 2;
     if (tri >= 8 * sms_) LAUNCH(k_border_update<4>, tri, 256, kUpdateSmem, st, d, b, p);
@@ -764,14 +774,31 @@ void Engine::record_border_factor(cudaStream_t st) {
   }
   const int nt = cdiv(b.k, 64);
   LAUNCH(k_border_pack, nt * (nt + 1) / 2, 256, 0, st, b);
+  if (b.mc) LAUNCH(k_schur_pack, cdiv(b.mc, 64) * (cdiv(b.mc, 64) + 1) / 2, 256, 0, st, b);
   if (prof_) {
     const double k = b.k;
     prof_work("k_border_update<4>", 2.0 / 3.0 * k * k * k, 16.0 / 3.0 * k * (k + 1) * b.npan);
   }
 }
 
+// The whole CG run of a Schur plan, from the vectors that k_cg_setup leaves.
+void Engine::record_schur_cg(cudaStream_t st) {
+  const DevBorder& b = bord_;
+  const int tasks = cdiv(b.mc, b.srb), grid = std::min(2 * tasks, std::max(16, sms_ * 3 / share_));
+  HYKKT_CUDA(cudaMemsetAsync(b.ctl, 0, kCtlWords * sizeof(unsigned long long), st));
+  if (b.srb == 4) {
+    LAUNCH(k_schur_cg<4>, grid, 256, kSolveSmem, st, dp, b, tasks);
+  } else {
+    LAUNCH(k_schur_cg<8>, grid, 256, kSolveSmem, st, dp, b, tasks);
+  }
+}
+
 // x = Hgamma^-1 b, or (cg) the whole CG loop from its start vectors.
 void Engine::record_border_solve(cudaStream_t st, const double* rhs, double* x, int use_stop, bool cg) {
+  if (cg && bord_.mc) {
+    record_schur_cg(st);
+    return;
+  }
   const DevPlan& d = dp;
   const DevBorder& b = bord_;
   BorderTasks t{};
@@ -927,6 +954,7 @@ void Engine::record_cg_pre(cudaStream_t st, int zero_x0) {
   record_trisolve(st, d.rxp, d.hrxp, 0);
   LAUNCH(k_spmv_jcp, gm, kBlock, 0, st, d, d.hrxp, d.schur, d.ry_s, 0, 0);
   LAUNCH(k_cg_setup, gm, kBlock, 0, st, d, zero_x0);
+  if (S_.border.on && bord_.mc) return;  // the CG launch takes r, gam, w and alpha itself
   // r = b - S x0, gam = r.r
   LAUNCH(k_spmv_jctp, gn, kBlock, 0, st, d, d.cg_x, d.cg_yv, (const double*)nullptr, 0);
   record_trisolve(st, d.cg_yv, d.cg_z, 0);

@@ -171,7 +171,8 @@ struct SolveSched {
 
 // Device view of the bordered layout (Bordered in symbolic.hpp, bordered.cuh).
 struct DevBorder {
-  int k, ld, npan;  // ld: k rounded up to 128, npan: 32-column panels
+  int k, ld, npan;  // npan: 32-column panels; ld: rows (with the constraints of a Schur plan) rounded up to 128
+  int mc, ncb;      // constraint rows below the panels (Schur plans, else 0), 32-column blocks in all
   int nblk, nbig, nasm;
   const int* bcol;
   const int *blk_rp, *blk_col, *blk_rrp, *blk_row;
@@ -193,7 +194,9 @@ struct DevBorder {
   int n_lo, n_up, nseg;  // tasks of the two products, most tasks per panel
   double* part;          // sums of the panels with several tasks
   int* rowcnt;
-  double *r2, *s2;       // CG residual and direction of every second iteration
+  double *r2, *s2, *w2;  // CG residual, direction and product of every second iteration
+  double* S;             // Schur plans: S in panels of srb rows
+  int srb;
   double *rrp, *dlp;     // CG partial sums
   double* scal;          // CG: 1/gamma, 1/alpha, the squared residual that stops
   unsigned long long* ctl;  // task counters of one launch
@@ -319,6 +322,7 @@ class Engine {
   void upload_all();
   void upload_border();
   void record_border_factor(cudaStream_t st);
+  void record_schur_cg(cudaStream_t st);
   void record_border_solve(cudaStream_t st, const double* b, double* x, int use_stop, bool cg);
   void wait_last_launch();
   static void copy_settings(const DevPlan& from, DevPlan& to);

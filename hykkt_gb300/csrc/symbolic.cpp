@@ -152,14 +152,25 @@ Cut cut_at(const Symbolic& S, int most) {
   return c;
 }
 
-// Estimated microseconds of one factorization and kSolves triangular solve
-// pairs.  FP64 multiply-adds run at 6.3e5 per us on the whole GPU.
+// Estimated microseconds of one factorization and kSolves CG iterations, from
+// measurements on GB300: 30 us for a panel's launches and pivot block, FP64
+// multiply-adds at 6.3e5 per us on the whole GPU (the update's epilogue takes
+// three per element), 22 us for an iteration's phases without blocks, 30 us
+// and 0.06 us per row of the largest block with them, 9 us with S formed.
 constexpr double kFmaPerUs = 6.3e5, kSolves = 100;
 double border_cost(const Cut& c) {
   const double k = c.k, panels = k / kBorderPanel;
-  double sweep = 0.0;  // the largest front's columns, one after the other
-  for (int b = 0; b < c.nblk; ++b) sweep = std::max(sweep, 0.5 * c.ncols[b] + 4e-3 * c.ncols[b] * c.nrows[b]);
-  return panels * (16.0 + 1.3 * k * k / kFmaPerUs) + sweep + kSolves * (1.2 * k * k / kFmaPerUs + (c.nblk ? 14.0 : 6.0));
+  double sweep = 0.0, most = 0.0;  // the largest front's columns, one after the other; its rows
+  for (int b = 0; b < c.nblk; ++b) {
+    sweep = std::max(sweep, 0.5 * c.ncols[b] + 4e-3 * c.ncols[b] * c.nrows[b]);
+    most = std::max(most, (double)c.ncols[b] + c.nrows[b]);
+  }
+  return panels * (30.0 + 1.3 * k * k / kFmaPerUs) + sweep +
+         kSolves * (1.6 * k * k / kFmaPerUs + (c.nblk ? 30.0 + 0.06 * most : 22.0));
+}
+double schur_cost(double n, double mc) {
+  const double K = n + mc;
+  return n / kBorderPanel * (30.0 + 1.6 * K * K / kFmaPerUs) + kSolves * (9.0 + 1.5 * mc * mc / kFmaPerUs);
 }
 double queue_cost(double stored, int levels, double flops) {
   return 1.3 * 0.5 * flops / kFmaPerUs + 150.0 * levels + kSolves * (2.6 * stored / kFmaPerUs + 13.0 * levels);
@@ -182,6 +193,12 @@ static bool choose_border(Symbolic& S, int levels, double flops) {
       cost = ct;
       c = std::move(t);
     }
+  }
+  // forming S saves three of a CG iteration's four phases
+  const bool schur = S.m_c > 0 && S.m_c <= kSchurRows && schur_cost(n, S.m_c) < cost;
+  if (schur) {
+    c = cut_at(S, 0);
+    cost = schur_cost(n, S.m_c);
   }
   const int64_t k = c.k;
   if (k == 0 || k > 65536 || cost > queue_cost((double)S.L_stored, levels, flops)) return false;
@@ -293,6 +310,7 @@ static bool choose_border(Symbolic& S, int levels, double flops) {
     std::vector<int> nx(B.ug_rp.begin(), B.ug_rp.end() - 1);
     for (size_t e = 0; e < B.blk_row.size(); ++e) B.ug_pos[nx[B.blk_row[e]]++] = (int)e;
   }
+  B.schur = schur;
   B.on = true;
   return true;
 }

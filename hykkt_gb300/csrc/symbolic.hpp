@@ -58,9 +58,11 @@ struct SymbolicOptions {
 // them are the blocks.  A block's front holds its columns (blk_col, ascending)
 // and its border rows (blk_row, border positions, ascending).
 constexpr int kBlkRows = 232;      // most rows of a block front: its packed triangle fits one CTA's shared memory
+constexpr int kSchurRows = 2048;   // most constraints of a Schur plan (its CG task's vector)
 constexpr int kBorderPanel = 32;   // columns swept at a time in the border
 struct Bordered {
   bool on = false;
+  bool schur = false; // no blocks, and the Schur complement of the constraints is formed (k_schur_cg)
   int k = 0;          // border columns
   std::vector<int> bcol;
   int nblk = 0;       // blocks, by falling front size

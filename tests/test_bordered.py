@@ -165,3 +165,27 @@ def test_bordered_matches_task_queues(n_bus, monkeypatch):
         assert all(np.array_equal(a, b) for a, b in zip(sols[-1], p.solution()))
     for a, b in zip(*sols):
         assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(a)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_bus", [6, 16, 320, 321, 460])
+@pytest.mark.parametrize("start", [False, True])
+def test_schur_plan_matches_task_queues(n_bus, start, monkeypatch):
+    """Small systems form S itself (four rows a task up to 640 constraints,
+    eight above): the same solution as the task queues, from a zero and from a
+    given start vector, as many CG iterations up to a few of rounding."""
+    s = H.small_grid_system(n_bus=n_bus, seed=6)
+    y0 = np.random.default_rng(1).uniform(-1, 1, s.m_c) if start else None
+    sols, its = [], []
+    for v in ("0", "1"):
+        monkeypatch.setenv("HYKKT_BORDERED", v)
+        p = hk.Plan(s)
+        p.set_accuracy(2000, 1e-11, 0, 1e-10)
+        assert p.solve(s, y0=y0) == hk.OK
+        its.append(p.info()["cg_iterations"])
+        p.set_accuracy(2000, 1e-12, 4, 1e-13)
+        p.solve(s, y0=y0)
+        sols.append(p.solution())
+    assert abs(its[0] - its[1]) <= 2
+    for a, b in zip(*sols):
+        assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(a)
