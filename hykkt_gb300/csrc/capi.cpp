@@ -1266,7 +1266,6 @@ extern "C" int hykkt_ruiz_scale_noalloc_max_rows(void) { return ruiz_noalloc_max
 struct hykkt_chol_s {
   std::unique_ptr<Engine> eng;
   int n = 0, nnz = 0;
-  std::vector<int> entry_to_lp;  // input entry -> permuted lower slot (-1: upper, ignored)
   cudaStream_t stream = nullptr;
   ~hykkt_chol_s() {
     eng.reset();
@@ -1308,7 +1307,9 @@ extern "C" int hykkt_chol_create(hykkt_chol_t* c, int n, int nnz, const int* row
     auto h = std::make_unique<hykkt_chol_s>();
     h->n = n;
     h->nnz = nnz;
-    h->entry_to_lp.assign(nnz, -1);
+    // permuted lower slot -> input entry (upper entries are ignored, of
+    // entries given twice the last counts)
+    std::vector<int> src(S.lp_row.size(), -1);
     for (int i = 0; i < n; ++i)
       for (int p = rowptr[i]; p < rowptr[i + 1]; ++p) {
         const int j = colidx[p];
@@ -1319,9 +1320,10 @@ extern "C" int hykkt_chol_create(hykkt_chol_t* c, int n, int nnz, const int* row
         const int* end = S.lp_row.data() + S.lp_cp[b + 1];
         const int* it = std::lower_bound(beg, end, a);
         if (it == end || *it != a) throw std::runtime_error("chol: entry not in pattern");
-        h->entry_to_lp[p] = (int)(it - S.lp_row.data());
+        src[it - S.lp_row.data()] = p;
       }
     h->eng = std::make_unique<Engine>(std::move(S), 0.0, opt);
+    h->eng->set_entry_map(src, nnz);
     HYKKT_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     *c = h.release();
     return HYKKT_OK;
@@ -1330,11 +1332,7 @@ extern "C" int hykkt_chol_create(hykkt_chol_t* c, int n, int nnz, const int* row
 
 extern "C" int hykkt_chol_factor(hykkt_chol_t c, const double* vals) {
   return guarded([&]() {
-    const Symbolic& S = c->eng->sym();
-    std::vector<double> lp(S.lp_cp[S.n_x], 0.0);
-    for (int p = 0; p < c->nnz; ++p)
-      if (c->entry_to_lp[p] >= 0) lp[c->entry_to_lp[p]] = vals[p];
-    return c->eng->factor_values(lp.data(), c->stream);
+    return c->eng->factor_values(vals, c->stream);
   });
 }
 

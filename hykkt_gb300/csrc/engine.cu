@@ -219,6 +219,8 @@ Engine::~Engine() {
   if (cap_stream_) cudaStreamDestroy(cap_stream_);
   if (last_launch_) cudaEventDestroy(last_launch_);
   free_storage(allocs_);
+  if (entry_src_) cudaFree(entry_src_);
+  if (entry_vals_) cudaFree(entry_vals_);
   if (pin_in_) cudaFreeHost(pin_in_);
   if (pin_out_) cudaFreeHost(pin_out_);
   if (pin_sc_) cudaFreeHost(pin_sc_);
@@ -1472,10 +1474,47 @@ int Engine::trisolve(const double* b, double* x, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // Cholesky component: the plan of a single SPD matrix (no Jc/Jd blocks).
 // ---------------------------------------------------------------------------
-int Engine::factor_values(const double* lower_vals_host, cudaStream_t st) {
+// The values come as the caller's array; a gather on the device puts them into
+// the permuted lower order.  Where the GPU reaches pageable host memory itself
+// (Grace: over the chip-to-chip link) a kernel reads the array in place:
+// 27 MB of a dense 2,600-column matrix took 8 ms through a host gather and a
+// staged copy.
+__global__ void k_read_host(const double* __restrict__ src, double* __restrict__ dst, int64_t n) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + 3 * stride < n; i += 4 * stride) {
+    double t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) t[j] = src[i + j * stride];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) dst[i + j * stride] = t[j];
+  }
+  for (; i < n; i += stride) dst[i] = src[i];
+}
+__global__ void k_gather_lower(DevPlan d, const int* __restrict__ src, const double* __restrict__ vals) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < d.nnz_lo; q += gridDim.x * blockDim.x)
+    d.lp_v[q] = src[q] >= 0 ? vals[src[q]] : 0.0;
+}
+
+// Entry of the caller's array behind each permuted lower entry (-1: none, 0.0).
+void Engine::set_entry_map(const std::vector<int>& src, int64_t nnz) {
+  HYKKT_CUDA(cudaMalloc(&entry_src_, std::max<size_t>(src.size(), 1) * sizeof(int)));
+  HYKKT_CUDA(cudaMemcpy(entry_src_, src.data(), src.size() * sizeof(int), cudaMemcpyHostToDevice));
+  HYKKT_CUDA(cudaMalloc(&entry_vals_, std::max<int64_t>(nnz, 1) * sizeof(double)));
+  entry_n_ = nnz;
+  int dev = 0;
+  HYKKT_CUDA(cudaGetDevice(&dev));
+  HYKKT_CUDA(cudaDeviceGetAttribute(&reads_host_, cudaDevAttrPageableMemoryAccess, dev));
+}
+
+int Engine::factor_values(const double* vals_host, cudaStream_t st) {
   reload_device();
-  const int nlo = S_.lp_cp[S_.n_x];
-  HYKKT_CUDA(cudaMemcpyAsync(dp.lp_v, lower_vals_host, (size_t)nlo * sizeof(double), cudaMemcpyHostToDevice, st));
+  if (entry_n_ > 0) {
+    if (reads_host_) k_read_host<<<std::min(cdiv(entry_n_, 1024), 152 * 8), 256, 0, st>>>(vals_host, entry_vals_, entry_n_);
+    else HYKKT_CUDA(cudaMemcpyAsync(entry_vals_, vals_host, (size_t)entry_n_ * sizeof(double), cudaMemcpyHostToDevice, st));
+  }
+  k_gather_lower<<<std::max(1, std::min(cdiv(dp.nnz_lo, 256), 152 * 16)), 256, 0, st>>>(dp, entry_src_, entry_vals_);
+  HYKKT_CUDA(cudaGetLastError());
   DevScalars init{};
   init.pivot_col = INT_MAX;
   HYKKT_CUDA(cudaMemcpyAsync(dp.sc, &init, sizeof(DevScalars), cudaMemcpyHostToDevice, st));

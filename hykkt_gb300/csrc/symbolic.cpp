@@ -172,8 +172,12 @@ double schur_cost(double n, double mc) {
   const double K = n + mc;
   return n / kBorderPanel * (30.0 + 1.6 * K * K / kFmaPerUs) + kSolves * (9.0 + 1.5 * mc * mc / kFmaPerUs);
 }
-double queue_cost(double stored, int levels, double flops) {
-  return 1.3 * 0.5 * flops / kFmaPerUs + 150.0 * levels + kSolves * (2.6 * stored / kFmaPerUs + 13.0 * levels);
+// the task queues: FP64-bound updates, 150 us for the three kernels of each 32
+// columns along the tree (chain: the widest supernode of each level), 13 us a
+// level and solve pair
+double queue_cost(double stored, int levels, double flops, double chain) {
+  return 1.3 * 0.5 * flops / kFmaPerUs + 150.0 * (levels + chain / kBorderPanel) +
+         kSolves * (2.6 * stored / kFmaPerUs + 13.0 * levels);
 }
 }  // namespace
 
@@ -182,7 +186,7 @@ double queue_cost(double stored, int levels, double flops) {
 // k^2), smaller ones a shorter sweep of the largest block; no blocks at all
 // (everything in the border) saves the block phases of every solve, which is
 // worth it for small systems.
-static bool choose_border(Symbolic& S, int levels, double flops) {
+static bool choose_border(Symbolic& S, int levels, double flops, double chain) {
   const int n = S.n_x;
   Cut c;
   double cost = 0.0;
@@ -201,7 +205,7 @@ static bool choose_border(Symbolic& S, int levels, double flops) {
     cost = schur_cost(n, S.m_c);
   }
   const int64_t k = c.k;
-  if (k == 0 || k > 65536 || cost > queue_cost((double)S.L_stored, levels, flops)) return false;
+  if (k == 0 || k > 65536 || cost > queue_cost((double)S.L_stored, levels, flops, chain)) return false;
   int64_t upd = 0;
   for (int b = 0; b < c.nblk; ++b) upd += (int64_t)c.nrows[b] * (c.nrows[b] + 1) / 2;
   if (upd >= INT32_MAX) return false;
@@ -622,9 +626,12 @@ Symbolic build_symbolic(const CsrPattern& H, const CsrPattern& Ds, const CsrPatt
     std::vector<int> lvl(nsn, 0);
     int nlv = 0;
     S.L_stored = 0;
-    double flops = 0;
+    double flops = 0, chain = 0;
+    std::vector<int> widest(1, 0);
     for (int J = 0; J < nsn; ++J) {
       const int last = S.sn_first[J + 1] - 1, nc = last + 1 - S.sn_first[J];
+      if (lvl[J] >= (int)widest.size()) widest.resize(lvl[J] + 1, 0);
+      widest[lvl[J]] = std::max(widest[lvl[J]], nc);
       const double nr = nc - 1 + S.colcount[last];
       S.L_stored += (int64_t)nr * nc;
       flops += nr * nr * nc;
@@ -634,7 +641,8 @@ Symbolic build_symbolic(const CsrPattern& H, const CsrPattern& Ds, const CsrPatt
         p = std::max(p, lvl[J] + 1);
       }
     }
-    if (choose_border(S, nlv, flops)) {
+    for (int w : widest) chain += w;
+    if (choose_border(S, nlv, flops, chain)) {
       S.nlevels = S.nsq_levels = S.border.nblk ? 2 : 1;
       S.nsq = S.border.nblk + 1;
       S.L_stored = (int64_t)S.border.k * S.border.k + S.border.ge_off.back();
