@@ -100,9 +100,9 @@ __global__ void __launch_bounds__(256) k_block_sweep(DevPlan d, DevBorder bd, in
     GE[e] = a;
   }
   for (int e = tid; e < (nt + 63) / 64 * 64 * N; e += blockDim.x) {
-    const int t = e / (64 * N) * 64 + e % 64, i = e / 64 % N;  // entry i: border rows, then own
+    const int t = e / (64 * N) * 64 + e % 64, i = e / 64 % N;  // entry i: border rows, then own from the last on
     double a = 0.0;
-    if (t < nt) a = i < R ? A[packed_lower(nt + i, t)] : i - R >= t ? A[packed_lower(i - R, t)] : 0.0;
+    if (t < nt) a = i < R ? A[packed_lower(nt + i, t)] : N - 1 - i >= t ? A[packed_lower(N - 1 - i, t)] : 0.0;
     ET[e] = a;
   }
   double* C = bd.cb + bd.c_off[blk];  // the border update, packed lower R x R
@@ -583,16 +583,7 @@ __global__ void __launch_bounds__(256) k_border_pack(DevBorder bd) {
 constexpr int kCgRows = 256;  // rows of a vector task
 constexpr int kRowTask = 64;  // columns or constraints of a sparse task, four threads each
 
-struct BorderRhs {
-  const double* b;  // right-hand side, or null: Jc_p^T r of the CG's updated residual
-  const double *r, *w, *s;
-  double alpha, beta;
-};
-
-// r - alpha (w + beta s): the residual after this iteration's update
-__device__ __forceinline__ double cg_updated(const BorderRhs& q, int k) {
-  return fma(-q.alpha, fma(q.beta, __ldcg(&q.s[k]), __ldcg(&q.w[k])), __ldcg(&q.r[k]));
-}
+typedef unsigned long long count_t;  // tasks of all iterations of a CG run
 
 // Part of one row of a sparse product: L threads share a row (its entries
 // interleaved), each one's first eight indices and values are loaded ahead of
@@ -631,21 +622,74 @@ __device__ __forceinline__ double row_dot(SparseRow& r, const int* __restrict__ 
   }
   return acc;
 }
-// the L threads' parts (neighbouring lanes), L a power of two up to 4
-__device__ __forceinline__ double join_row(double s, int L) {
-  if (L > 1) s = dadd(s, __shfl_xor_sync(0xffffffffu, s, 1));
-  if (L > 2) s = dadd(s, __shfl_xor_sync(0xffffffffu, s, 2));
-  return s;
+// the four threads' parts (neighbouring lanes)
+__device__ __forceinline__ double join_row(double s) {
+  s = dadd(s, __shfl_xor_sync(0xffffffffu, s, 1));
+  return dadd(s, __shfl_xor_sync(0xffffffffu, s, 2));
 }
 
-// right-hand side of a permuted column in the CG: the column's row of Jc_p^T
-__device__ __forceinline__ void load_rhs_row(const DevPlan& d, SparseRow& r, int col, int L, int sub) {
-  const int* src = d.jctp_src;
-  load_row(r, d.jctp_rp[col], d.jctp_rp[col + 1], L, sub, d.jctp_ci, d.jc_s, [src](int p) { return src[p]; });
+// CG right-hand side Jc_p^T (r - alpha (w + beta s)): the three products come
+// from a phase of their own, beside the iteration's scalars, column after
+// column of the border and the blocks, so that a column's row of Jc_p^T is read
+// once and the scalars are followed by two multiply-adds.  (Each task that
+// needs a column formed its entry from the updated residual itself: a block of
+// 232 rows did so four times, 10.5 us a task at 5,000 buses, now 4.4.  Eight
+// threads a column end its phase 1 us earlier at 1,000 buses and 4 us later at
+// 10,000, where its tasks fill the GPU twice.)
+struct RhsParts {
+  double r, w, s;
+};
+__device__ __forceinline__ RhsParts load_parts(const DevBorder& bd, int j) {
+  return RhsParts{__ldcg(&bd.jt[j]), __ldcg(&bd.jt[bd.njt + j]), __ldcg(&bd.jt[2 * bd.njt + j])};
 }
-__device__ __forceinline__ double rhs_row_dot(const DevPlan& d, SparseRow& r, const BorderRhs& q) {
+__device__ __forceinline__ double rhs_value(const RhsParts& q, const double* sc) { return fma(-sc[0], fma(sc[1], q.s, q.w), q.r); }
+
+template <class Wait>
+__device__ __forceinline__ bool rhs_parts_task(const DevPlan& d, const DevBorder& bd, int task, const double* r, const double* s, Wait wait) {
+  const int j = task * kRowTask + (threadIdx.x >> 2), sub = threadIdx.x & 3;
+  const int col = j >= bd.njt ? 0 : j < bd.k ? bd.bcol[j] : bd.blk_col[j - bd.k];
   const int* src = d.jctp_src;
-  return row_dot(r, d.jctp_ci, d.jc_s, [src](int p) { return src[p]; }, [&](int k) { return cg_updated(q, k); });
+  auto vi = [src](int p) { return src[p]; };
+  SparseRow row;
+  row.p = row.e = 0;
+  row.L = 4;
+  if (j < bd.njt) load_row(row, d.jctp_rp[col], d.jctp_rp[col + 1], 4, sub, d.jctp_ci, d.jc_s, vi);
+  if (!wait()) return false;
+  RhsParts q{0.0, 0.0, 0.0};
+  for (;;) {
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+      if (row.p + h * 4 >= row.e) break;
+      double t[3][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool in = row.p + (h + i) * 4 < row.e;
+        const int c = row.c[h + i];
+        t[0][i] = in ? __ldcg(&r[c]) : 0.0;
+        t[1][i] = in ? __ldcg(&d.cg_w[c]) : 0.0;
+        t[2][i] = in ? __ldcg(&s[c]) : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (row.p + (h + i) * 4 < row.e) {
+          q.r = fma(row.a[h + i], t[0][i], q.r);
+          q.w = fma(row.a[h + i], t[1][i], q.w);
+          q.s = fma(row.a[h + i], t[2][i], q.s);
+        }
+    }
+    const int p = row.p + 32;
+    if (p >= row.e) break;
+    load_row(row, p, row.e, 4, 0, d.jctp_ci, d.jc_s, vi);
+  }
+  q.r = join_row(q.r);
+  q.w = join_row(q.w);
+  q.s = join_row(q.s);
+  if (j < bd.njt && sub == 0) {
+    bd.jt[j] = q.r;
+    bd.jt[bd.njt + j] = q.w;
+    bd.jt[2 * bd.njt + j] = q.s;
+  }
+  return true;
 }
 
 // every fourth of the blocks' contributions to border column j
@@ -664,61 +708,72 @@ __device__ __forceinline__ double border_updates(const DevBorder& bd, int j, int
 
 // Products of a dense row panel, column after column of its RB rows, with a
 // vector in shared memory: 256 / RB threads a row over interleaved columns.
-// The panel streams through kStages shared-memory chunks by bulk copies, the
-// first of them issued before the task waits for its vector.
+// The panel streams through kStages shared-memory chunks by bulk copies that
+// thread 0 issues, the first of them before the task waits for its vector.  A
+// warp that has read a chunk says so on the chunk's second mbarrier, so that
+// warps run apart (a CTA barrier per chunk was a third of their stalls).
 constexpr int kGemvSeg = 2048, kChunk = 2048, kStages = 3;  // most columns of a panel, entries of a chunk
 constexpr int kRed = 256;                                   // doubles before the vector
 constexpr int kSolveSmem = (kRed + kGemvSeg + kStages * kChunk) * 8;
 
-// state of the CTA's chunk ring: chunks issued and consumed since the launch
-struct Ring {
-  uint32_t bar;  // kStages mbarriers
-  unsigned put, got;
-};
-
-__device__ __forceinline__ void ring_put(Ring& g, double* chunks, const double* src, int n) {
-  const int st = g.put % kStages;
-  ++g.put;
-  if (threadIdx.x == 0) {
-    const uint32_t bar = g.bar + 8 * st;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n * 8) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(chunks + st * kChunk)),
-                 "l"(src), "r"(n * 8), "r"(bar) : "memory");
-  }
-}
-
-// every thread waits for the oldest chunk (bounded)
-__device__ __forceinline__ int ring_get(Ring& g, DevScalars* sc) {
-  const int st = g.got % kStages;
-  mbar_wait(g.bar + 8 * st, (g.got / kStages) & 1, sc);
-  ++g.got;
-  return st;
-}
-
 struct Panel {
   const double* M;
   int n;  // entries: columns * RB
+  __device__ __forceinline__ int chunks() const { return (n + kChunk - 1) / kChunk; }
 };
-__device__ __forceinline__ void panel_start(Ring& g, const Panel& p, double* sm) {
-  double* ch = sm + kRed + kGemvSeg;
-  for (int c = 0; c < kStages && c * kChunk < p.n; ++c) ring_put(g, ch, p.M + c * kChunk, min(kChunk, p.n - c * kChunk));
+
+// The CTA's chunk ring: barriers [chunk full, chunk read], chunks issued
+// (thread 0) and consumed since the launch.
+struct Ring {
+  uint32_t bar, buf;  // shared-memory addresses: 2 * kStages barriers, the chunks
+  unsigned put, got;
+};
+__device__ __forceinline__ Ring ring_init(uint64_t* bars, double* sm) {
+  Ring g{smem_addr(bars), smem_addr(sm + kRed + kGemvSeg), 0, 0};
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(g.bar + 8 * i));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(g.bar + 8 * (kStages + i)));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  return g;
 }
-// the copies in flight of a task that gives up
+// thread 0: chunk c of the panel into the next buffer, once all warps have read it
+__device__ __forceinline__ void ring_put(Ring& g, const Panel& p, int c, DevScalars* sc) {
+  const int st = g.put % kStages, n = min(kChunk, p.n - c * kChunk) * 8;
+  const uint32_t bar = g.bar + 8 * st;
+  mbar_wait(g.bar + 8 * (kStages + st), ((g.put / kStages) & 1) ^ 1, sc);
+  ++g.put;
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   g.buf + st * (kChunk * 8)),
+               "l"(p.M + c * kChunk), "r"(n), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void panel_start(Ring& g, const Panel& p, DevScalars* sc) {
+  if (threadIdx.x == 0)
+    for (int c = 0; c < kStages && c * kChunk < p.n; ++c) ring_put(g, p, c, sc);
+}
+// a task that gives up: thread 0 stays until the copies in flight have landed
 __device__ __forceinline__ void panel_drain(Ring& g, DevScalars* sc) {
-  while (g.got < g.put) ring_get(g, sc);
+  if (threadIdx.x == 0)
+    for (; g.got < g.put; ++g.got) mbar_wait(g.bar + 8 * (g.got % kStages), (g.got / kStages) & 1, sc);
 }
-// the product of row threadIdx.x in threads below RB; v = sm + kRed is complete
-template <int RB>
-__device__ __forceinline__ double panel_product(Ring& g, const Panel& p, double* sm, DevScalars* sc) {
+
+// The product of row threadIdx.x in threads below RB with the vector v in
+// shared memory.  refill(c): thread 0 issues what follows, chunk c's buffer (a
+// chunk ago) is free or about to be.
+template <int RB, class Refill>
+__device__ __forceinline__ double panel_product(Ring& g, const Panel& p, const double* v, double* sm, DevScalars* sc, Refill refill) {
   constexpr int P = 256 / RB, kCols = kChunk / RB;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const double* v = sm + kRed + threadIdx.x / RB;
-  double* ch = sm + kRed + kGemvSeg;
+  v += threadIdx.x / RB;
   double a[2] = {0.0, 0.0};
   int left = p.n / RB - threadIdx.x / RB;
   for (int c = 0; c * kChunk < p.n; ++c, v += kCols, left -= kCols) {
-    const double* m = ch + ring_get(g, sc) * kChunk + threadIdx.x;
+    const int st = g.got % kStages;
+    mbar_wait(g.bar + 8 * st, (g.got / kStages) & 1, sc);
+    ++g.got;
+    const double* m = sm + kRed + kGemvSeg + st * kChunk + threadIdx.x;
     if (left > 7 * P) {
 #pragma unroll
       for (int q = 0; q < 8; ++q) a[q & 1] = fma(m[q * 256], v[q * P], a[q & 1]);
@@ -727,90 +782,185 @@ __device__ __forceinline__ double panel_product(Ring& g, const Panel& p, double*
       for (int q = 0; q < 8; ++q)
         if (q * P < left) a[q & 1] = fma(m[q * 256], v[q * P], a[q & 1]);
     }
-    __syncthreads();
-    const int nx = (c + kStages) * kChunk;
-    if (nx < p.n) ring_put(g, ch, p.M + nx, min(kChunk, p.n - nx));
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(g.bar + 8 * (kStages + st)) : "memory");
+    if (threadIdx.x == 0 && c > 0) refill(c - 1);
   }
-  double s = dadd(a[0], a[1]);
-  constexpr int kParts = RB < 32 ? 8 : P;  // partial sums per row left after the shuffles
-#pragma unroll
-  for (int o = RB; o < 32; o <<= 1) s = dadd(s, __shfl_xor_sync(0xffffffffu, s, o));
-  if (RB >= 32) sm[threadIdx.x] = s;
-  else if (lane < RB) sm[warp * RB + lane] = s;
+  // the P parts of a row: through shared memory to as many threads of the
+  // first warps as leave eight parts each (FP64 adds by full warps cost the
+  // product's time)
+  sm[threadIdx.x] = dadd(a[0], a[1]);
   __syncthreads();
+  constexpr int kParts = P < 8 ? P : 8, kT = 256 / kParts;  // parts per thread, threads
   double t = 0.0;
-  if (threadIdx.x < RB) {
+  if (threadIdx.x < kT) {
     double w[kParts];
 #pragma unroll
-    for (int q = 0; q < kParts; ++q) w[q] = sm[q * RB + threadIdx.x];
+    for (int q = 0; q < kParts; ++q) w[q] = sm[q * kT + threadIdx.x];
 #pragma unroll
     for (int o = 1; o < kParts; o <<= 1)
 #pragma unroll
       for (int q = 0; q < kParts; q += 2 * o) w[q] = dadd(w[q], w[q + o]);
     t = w[0];
+#pragma unroll
+    for (int o = RB; o < kT; o <<= 1) t = dadd(t, __shfl_xor_sync(0xffffffffu, t, o));
+  }
+  return t;
+}
+template <int RB>
+__device__ __forceinline__ double panel_product(Ring& g, const Panel& p, double* sm, DevScalars* sc) {
+  return panel_product<RB>(g, p, sm + kRed, sm, sc, [&](int c) {
+    if (c + kStages < p.chunks()) ring_put(g, p, c + kStages, sc);
+  });
+}
+
+// by = X bt (up 0) or x_S = X^T by (up 1): a task is a panel's part in one
+// segment of kGemvSeg columns (X counts segments from the left, X^T from the
+// right).  A longer panel's tasks store their sums, the last one adds them in
+// segment order.  Bounded by FP64 issue (one multiply-add per entry, 2 per
+// clock and SM), by HBM where the panels exceed the L2.  Four rows a panel keep
+// a small border's tasks short, eight halve the vector reads of a large one.
+struct GemvTask {
+  int b, sg;      // panel, segment
+  int v0;         // first column of the segment (its vector starts there)
+  int j0, n;      // the task's columns
+  Panel p;
+};
+template <int RB>
+__device__ __forceinline__ GemvTask gemv_task(const DevBorder& bd, int task, bool up) {
+  // by segment, in a segment the panels that reach it, longest first
+  GemvTask t;
+  t.sg = 0;
+  t.b = task;
+  for (int c = bd.nrb; t.b >= c; c = bd.nrb - t.sg * (kGemvSeg / RB)) {
+    t.b -= c;
+    ++t.sg;
+  }
+  if (up) {
+    const int end = bd.nrb * RB - t.sg * kGemvSeg;
+    t.v0 = max(0, end - kGemvSeg);
+    t.j0 = max(t.b * RB, t.v0);
+    t.n = min(bd.k, end) - t.j0;
+    t.p = Panel{bd.xup + panel_up(t.b, bd.nrb, RB) + (int64_t)(t.j0 - t.b * RB) * RB, t.n * RB};
+  } else {
+    t.b = bd.nrb - 1 - t.b;
+    t.v0 = t.j0 = t.sg * kGemvSeg;
+    t.n = min(kGemvSeg, min(bd.k, (t.b + 1) * RB) - t.j0);
+    t.p = Panel{bd.xlo + panel_lo(t.b, RB) + (int64_t)t.j0 * RB, t.n * RB};
   }
   return t;
 }
 
-// by = X bt (up 0) or x_S = X^T by (up 1) for up to kGemvSeg columns of a
-// panel.  A longer panel's tasks store their sums, the last one adds them in
-// column order.  Bounded by FP64 issue (one multiply-add per entry, 2 per clock
-// and SM), by HBM where the panels exceed the L2.  Four rows a panel keep a
-// small border's tasks short, eight halve the vector reads of a large one.
-template <int RB, class Wait>
-__device__ __forceinline__ bool border_gemv(const DevPlan& d, const DevBorder& bd, Ring& g, int task, bool up, double* x, double* sm, Wait wait) {
-  __shared__ bool fin;
-  // tasks by column segment, in a segment the panels that reach it, longest first
-  int sg = 0, b = task;
-  for (int c = bd.nrb; b >= c; c = bd.nrb - (sg * kGemvSeg) / RB) {
-    b -= c;
-    ++sg;
-  }
-  if (!up) b = bd.nrb - 1 - b;
-  const int len = up ? bd.k - b * RB : min(bd.k, (b + 1) * RB);
-  const int j0 = sg * kGemvSeg, n = min(kGemvSeg, len - j0), segs = (len + kGemvSeg - 1) / kGemvSeg;
-  const Panel p{(up ? bd.xup + panel_up(b, bd.nrb, RB) : bd.xlo + panel_lo(b, RB)) + (int64_t)j0 * RB, n * RB};
-  panel_start(g, p, sm);
-  if (!wait()) {
-    panel_drain(g, d.sc);
-    return false;
-  }
-  const double* src = (up ? bd.by + b * RB : bd.bt) + j0;
-  double* v = sm + kRed;
+// the segment's vector into shared memory
+__device__ __forceinline__ void gemv_vector(const DevBorder& bd, const GemvTask& t, bool up, double* v) {
+  const double* src = (up ? bd.by : bd.bt) + t.v0;
+  const int n = min(kGemvSeg, bd.k - t.v0);
 #pragma unroll
   for (int h = 0; h < kGemvSeg / 256; h += 4) {
-    double t[4];
+    double r[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) t[q] = threadIdx.x + (h + q) * 256 < n ? __ldcg(&src[threadIdx.x + (h + q) * 256]) : 0.0;
+    for (int q = 0; q < 4; ++q) r[q] = threadIdx.x + (h + q) * 256 < n ? __ldcg(&src[threadIdx.x + (h + q) * 256]) : 0.0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v[threadIdx.x + (h + q) * 256] = t[q];
+    for (int q = 0; q < 4; ++q) v[threadIdx.x + (h + q) * 256] = r[q];
     if ((h + 4) * 256 >= n) break;
   }
-  __syncthreads();
-  double t = panel_product<RB>(g, p, sm, d.sc);
-  const int row = b * RB + threadIdx.x;
+}
+
+// warp 0: the task's sums (rows in lanes below RB) to the result, by way of the
+// panel's slots where it has several tasks
+template <int RB>
+__device__ __forceinline__ void gemv_store(const DevBorder& bd, const GemvTask& t, bool up, double s, double* x) {
+  const int len = up ? bd.nrb * RB - t.b * RB : min(bd.k, (t.b + 1) * RB);
+  const int segs = (len + kGemvSeg - 1) / kGemvSeg, lane = threadIdx.x, row = t.b * RB + lane;
   if (segs > 1) {
-    double* slot = bd.part + (int64_t)b * bd.nseg * RB;
-    if (threadIdx.x < RB) __stcg(&slot[sg * RB + threadIdx.x], t);
+    double* slot = bd.part + (int64_t)t.b * bd.nseg * RB;
+    if (lane < RB) __stcg(&slot[t.sg * RB + lane], s);
+    __syncwarp();
+    int fin = 0;
+    if (lane == 0) {
+      __threadfence();
+      fin = atomicAdd(&bd.rowcnt[t.b], 1) == segs - 1;
+      __threadfence();
+    }
+    if (!__shfl_sync(0xffffffffu, fin, 0)) return;
+    if (lane < RB) {
+      s = __ldcg(&slot[lane]);
+      for (int q = 1; q < segs; ++q) s = dadd(s, __ldcg(&slot[q * RB + lane]));
+    }
+    if (lane == 0) bd.rowcnt[t.b] = 0;  // for the next product
+  }
+  if (lane < RB && row < bd.k) {
+    if (up) x[bd.bcol[row]] = s;
+    else bd.by[row] = s;
+  }
+}
+
+// A run of product tasks by one CTA from its claimed task `cur` on.  While many
+// tasks of the phase are left (two per CTA of the grid, so that none is held
+// back at the phase's end) thread 0 claims the next one at the start of the
+// current one, its first chunks follow the current one's through the ring, and
+// a vector segment stays for the tasks of the segment: between tasks there is
+// no round trip.  Returns the number of tasks done; a claimed task that is not
+// of this phase stays in `pre` (thread 0).
+template <int RB, class Wait>
+__device__ __forceinline__ int gemv_run(const DevPlan& d, const DevBorder& bd, Ring& g, int cur, int ntask, bool up, double* x,
+                                        double* sm, count_t* head, count_t first, int* s_next, count_t& pre, bool& has_pre, int slot, Wait wait) {
+  double* v = sm + kRed;
+  GemvTask t = gemv_task<RB>(bd, cur, up);
+  int started = 0, have = -1, ndone = 0;  // started: thread 0, the task's chunks already issued
+  bool waited = false;
+  for (;;) {
+    const int chunks = t.p.chunks();
+    if (threadIdx.x == 0)
+      for (; started < kStages && started < chunks; ++started) ring_put(g, t.p, started, d.sc);
+    if (!waited && !wait()) {
+      panel_drain(g, d.sc);
+      return -1;
+    }
+    waited = true;
+    if (t.sg != have) {
+      gemv_vector(bd, t, up, v);
+      have = t.sg;
+    }
+    const bool ahead = cur + 2 * (int)gridDim.x < ntask;
+    count_t claim = 0;
+    if (ahead && threadIdx.x == 0) claim = atomicAdd(head, count_t(1));
     __syncthreads();
+    trace_mark(d, slot + cur, 1);  // timeline: the run's tasks from tk.off[ph] on
+    trace_mark(d, slot + cur, 3);
+    int next = -2;  // thread 0: not looked at yet
+    Panel np{nullptr, 0};
+    auto look = [&]() {
+      next = ahead && claim - first < (count_t)ntask ? (int)(claim - first) : -1;
+      if (next >= 0) np = gemv_task<RB>(bd, next, up).p;
+      started = 0;
+    };
+    const double s = panel_product<RB>(g, t.p, v + (t.j0 - t.v0), sm, d.sc, [&](int c) {
+      if (c + kStages < chunks) {
+        ring_put(g, t.p, c + kStages, d.sc);
+      } else {
+        if (next == -2) look();
+        if (chunks >= kStages && started * kChunk < np.n) ring_put(g, np, started++, d.sc);
+      }
+    });
+    if (threadIdx.x < 32) gemv_store<RB>(bd, t, up, s, x);
+    ++ndone;
+    trace_mark(d, slot + cur, 2);
+    if (!ahead) return ndone;
     if (threadIdx.x == 0) {
-      __threadfence();
-      fin = atomicAdd(&bd.rowcnt[b], 1) == segs - 1;
-      __threadfence();
+      if (next == -2) look();
+      if (next < 0) {
+        pre = claim;
+        has_pre = true;
+      }
+      *s_next = next;
     }
     __syncthreads();
-    if (!fin) return true;
-    if (threadIdx.x < RB) {
-      t = __ldcg(&slot[threadIdx.x]);
-      for (int q = 1; q < segs; ++q) t = dadd(t, __ldcg(&slot[q * RB + threadIdx.x]));
-    }
-    if (threadIdx.x == 0) bd.rowcnt[b] = 0;  // for the next product
+    cur = *s_next;
+    if (cur < 0) return ndone;
+    t = gemv_task<RB>(bd, cur, up);
   }
-  if (threadIdx.x < RB && row < bd.k) {
-    if (up) x[bd.bcol[row]] = t;
-    else bd.by[row] = t;
-  }
-  return true;
 }
 
 // Dot product of row `lane` of a warp's block panel (64 rows a column).
@@ -829,9 +979,11 @@ __device__ __forceinline__ double warp_rows(const double* __restrict__ M, int K,
 
 // y_F = X b_F, u = E b_F: 64 rows of a block of more than 32 rows per CTA, or
 // eight smaller blocks, one per warp.  (A block's rows on several CTAs: one
-// SM's FP64 rate would make a whole large block 20-40 us.)
-template <bool kCg, class Wait>
-__device__ __forceinline__ bool block_fwd(const DevPlan& d, const DevBorder& bd, const BorderRhs& q, Ring& g, int task, double* sm, Wait wait) {
+// SM's FP64 rate would make a whole large block 20-40 us.)  X is lower
+// triangular: a chunk of its rows ends at its diagonal.
+template <bool kCg, class Wait, class WaitScalars>
+__device__ __forceinline__ bool block_fwd(const DevBorder& bd, const double* b, const double* sc, Ring& g, int task, double* sm, DevScalars* S, Wait wait,
+                                          WaitScalars wait_scalars) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool big = task < bd.nfp;
   const int blk = big ? bd.fp_blk[task] : bd.nbig + (task - bd.nfp) * 8 + warp;
@@ -839,36 +991,31 @@ __device__ __forceinline__ bool block_fwd(const DevPlan& d, const DevBorder& bd,
   const int c0 = have ? bd.blk_rp[blk] : 0, nt = have ? bd.blk_rp[blk + 1] - c0 : 0;
   const int N = have ? nt + bd.blk_rrp[blk + 1] - bd.blk_rrp[blk] : 0;
   const int r0 = big ? 64 * (task - bd.fp_first[blk]) : 0;
-  // right-hand side: L threads per column (a warp's block: one)
-  const int L = !big || nt > 128 ? 1 : nt > 64 ? 2 : 4;
-  const int i = big ? (int)threadIdx.x / L : lane, sub = big ? threadIdx.x % L : 0;
+  const int i = big ? (int)threadIdx.x : lane;
   const int col = i < nt ? bd.blk_col[c0 + i] : 0;
-  const Panel p{bd.ge + (have ? bd.ge_off[blk] + (int64_t)r0 * nt : 0), 64 * nt};
-  SparseRow row;
-  row.p = row.e = 0;
-  row.L = 1;
-  if (kCg && i < nt) load_rhs_row(d, row, col, L, sub);
-  if (big) panel_start(g, p, sm);
+  const Panel p{bd.ge + (have ? bd.ge_off[blk] + (int64_t)r0 * nt : 0), 64 * (r0 + 64 <= nt ? r0 + 64 : nt)};
+  if (big) panel_start(g, p, S);
   else prefetch_bytes(p.M, (int64_t)64 * nt * 8, lane, 32);
-  if (!wait()) {
-    panel_drain(g, d.sc);
+  double w = 0.0;
+  if (!wait_scalars() || !wait()) {
+    panel_drain(g, S);
     return false;
   }
-  const double w = kCg ? join_row(rhs_row_dot(d, row, q), L) : i < nt ? q.b[col] : 0.0;
+  if (i < nt) w = kCg ? rhs_value(load_parts(bd, bd.k + c0 + i), sc) : b[col];
   double* v = big ? sm + kRed : sm + warp * 32;
-  if (i < nt && sub == 0) v[i] = w;
+  if (i < nt) v[i] = w;
   if (big) __syncthreads();
   else __syncwarp();
-  const double t = big ? panel_product<64>(g, p, sm, d.sc) : warp_rows(p.M + lane, nt, v);
-  const int r = big ? (int)threadIdx.x : lane;
-  if ((!big || r < 64) && r0 + r < N) {
-    if (r0 + r < nt) bd.y[c0 + r0 + r] = t;
-    else bd.u[bd.u_off[blk] + r0 + r - nt] = t;
+  const double t = big ? panel_product<64>(g, p, sm, S) : warp_rows(p.M + lane, nt, v);
+  if ((!big || i < 64) && r0 + i < N) {
+    if (r0 + i < nt) bd.y[c0 + r0 + i] = t;
+    else bd.u[bd.u_off[blk] + r0 + i - nt] = t;
   }
   return true;
 }
 
-// x_F = X^T y_F - E^T x_S: the same for 64 columns of a block
+// x_F = X^T y_F - E^T x_S: the same for 64 columns of a block, whose own rows
+// come last and from the last one on, so that a chunk ends at its diagonal
 template <class Wait>
 __device__ __forceinline__ bool block_bwd(const DevPlan& d, const DevBorder& bd, Ring& g, int task, double* x, double* sm, Wait wait) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -880,8 +1027,8 @@ __device__ __forceinline__ bool block_bwd(const DevPlan& d, const DevBorder& bd,
   const int t0 = big ? 64 * (task - bd.bp_first[blk]) : 0;
   const int i = big ? (int)threadIdx.x : lane;
   const int brow = i < R ? bd.bcol[bd.blk_row[b0 + i]] : 0;
-  const Panel p{bd.et + (have ? bd.et_off[blk] + (int64_t)t0 * N : 0), 64 * N};
-  if (big) panel_start(g, p, sm);
+  const Panel p{bd.et + (have ? bd.et_off[blk] + (int64_t)t0 * N : 0), 64 * (N - t0)};
+  if (big) panel_start(g, p, d.sc);
   else prefetch_bytes(p.M, (int64_t)64 * N * 8, lane, 32);
   const int r = t0 + (big ? (int)threadIdx.x & 63 : lane);
   const int col = r < nt ? bd.blk_col[c0 + r] : 0;
@@ -890,7 +1037,7 @@ __device__ __forceinline__ bool block_bwd(const DevPlan& d, const DevBorder& bd,
     return false;
   }
   double* v = big ? sm + kRed : sm + warp * 32;
-  if (i < N) v[i] = i < R ? __ldcg(&x[brow]) : __ldcg(&bd.y[c0 + i - R]);
+  if (i < N) v[i] = i < R ? __ldcg(&x[brow]) : __ldcg(&bd.y[c0 + N - 1 - i]);
   if (big) __syncthreads();
   else __syncwarp();
   const double t = big ? panel_product<64>(g, p, sm, d.sc) : warp_rows(p.M + lane, N, v);
@@ -898,16 +1045,19 @@ __device__ __forceinline__ bool block_bwd(const DevPlan& d, const DevBorder& bd,
   return true;
 }
 
-// Task table of one launch: phases in order, the phase each one waits for,
-// counters [head, ready, done, phase counts].
+// Task table of one launch: phases in order (0 products Jc^T of the CG's
+// vectors, 1 blocks forward and the CG's vector update, 2 border right-hand
+// side, 3 and 4 its products, 5 blocks back, 6 the product Jc x and the CG's
+// scalars), the phase each one waits for, counters [head, ready, done, phase
+// counts].
+constexpr int kPhases = 7;
 struct BorderTasks {
-  int n[6], off[7], dep[6];
-  int n_upd;  // CG: vector update tasks of phase 0
-  int n_fwd;  // block tasks of phase 0
+  int n[kPhases], off[kPhases + 1], dep[kPhases];
+  int n_upd;  // CG: vector update tasks of phase 1
+  int n_fwd;  // block tasks of phase 1
 };
 // each on a 128-byte line of its own: hundreds of CTAs poll them
-constexpr int kCtlReady = 16, kCtlDone = 32, kCtlCount = 48, kCtlStep = 16, kCtlWords = 48 + 6 * 16;
-typedef unsigned long long count_t;  // tasks of all iterations of a CG run
+constexpr int kCtlReady = 16, kCtlDone = 32, kCtlCount = 48, kCtlStep = 16, kCtlWords = 48 + kPhases * 16;
 __device__ __forceinline__ count_t load_acquire(const count_t* p) {
   count_t v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -949,9 +1099,9 @@ __device__ __forceinline__ void cta_sum(double v, double* red) {
 
 // red[0], red[1] = the sums of the first n0 parts of r.r and n1 parts of w.r in
 // a fixed order, one warp each
-__device__ __forceinline__ void sum_parts(const DevBorder& bd, int n0, int n1, double* red) {
+__device__ __forceinline__ void sum_parts(const double* rrp, const double* dlp, int n0, int n1, double* red) {
   if (threadIdx.x < 64) {
-    const double* src = threadIdx.x < 32 ? bd.rrp : bd.dlp;
+    const double* src = threadIdx.x < 32 ? rrp : dlp;
     const int lane = threadIdx.x & 31, n = threadIdx.x < 32 ? n0 : n1;
     double v = 0.0;
     for (int i = lane; i < n; i += 128) {
@@ -966,33 +1116,51 @@ __device__ __forceinline__ void sum_parts(const DevBorder& bd, int n0, int n1, d
   __syncthreads();
 }
 
-// One thread, after the iteration's sums r.r and w.r: the recurrence for the
-// next iteration or the end of the loop, published through `ready`.  Every
-// iteration waits for this, and a division is 20 dependent FP64 instructions,
-// so the recurrence's divisions by the previous iteration's gamma and alpha
-// are products with reciprocals that were formed beside one another then, and
-// what only the end needs is computed there.
+// The CG's recurrence after iteration `it` with the sums r.r and w.r.  Every
+// iteration waits for it, and a division is 20 dependent FP64 instructions, so
+// the divisions by the previous iteration's gamma and alpha are products with
+// reciprocals formed beside one another then.
+struct CgState {
+  double inv_gam, inv_alpha;
+};
+__device__ __forceinline__ double cg_stop2(const DevPlan& d) {  // threshold on r.r
+  const DevScalars* S = d.sc;
+  const double thr = S->rtol_cur > 0.0 ? S->rtol_cur * sqrt(S->gam0) : d.cg_tol;
+  return thr * thr;
+}
+// 0 go on, 1 converged, 2 iteration limit; sc = alpha, beta of the next iteration
+__device__ __forceinline__ int cg_step(const DevPlan& d, CgState& st, double stop2, double rr, double wr, int it, double* sc) {
+  if (rr < stop2 || rr == 0.0) return 1;
+  if (it + 1 >= d.cg_itmax) return 2;
+  const double beta = rr * st.inv_gam, den = fma(-(beta * rr), st.inv_alpha, wr), inv = 1.0 / rr;
+  sc[0] = rr / den;
+  sc[1] = beta;
+  st.inv_gam = inv;
+  st.inv_alpha = den * inv;
+  return 0;
+}
+// bd.scal: the threshold, then the state for the iterations of each parity
+__device__ __forceinline__ CgState cg_state(const DevPlan& d, const DevBorder& bd, int it) {
+  if (it == 0) return CgState{1.0 / d.sc->gam, 1.0 / d.sc->alpha};
+  return CgState{__ldcg(&bd.scal[1 + 2 * (it & 1)]), __ldcg(&bd.scal[2 + 2 * (it & 1)])};
+}
+// one thread: the step for good, its state, and its results (kShare: alpha and
+// beta for all CTAs; at the end what the loop leaves) through `ready`
+template <bool kShare>
 __device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, double wr, int it, int round, count_t* ready, count_t* done) {
   DevScalars* S = d.sc;
-  double inv_gam, inv_alpha, stop2;
-  if (it == 0) {
-    const double thr = S->rtol_cur > 0.0 ? S->rtol_cur * sqrt(S->gam0) : d.cg_tol;
-    inv_gam = 1.0 / S->gam;
-    inv_alpha = 1.0 / S->alpha;
-    stop2 = thr * thr;
-    bd.scal[2] = stop2;
-  } else {
-    inv_gam = __ldcg(&bd.scal[0]);
-    inv_alpha = __ldcg(&bd.scal[1]);
-    stop2 = __ldcg(&bd.scal[2]);
-  }
-  const int stop = rr < stop2 || rr == 0.0 ? 1 : it + 1 >= d.cg_itmax ? 2 : 0;
+  double sc[2];
+  CgState st = cg_state(d, bd, it);
+  const double stop2 = it ? __ldcg(&bd.scal[0]) : cg_stop2(d);
+  const int stop = cg_step(d, st, stop2, rr, wr, it, sc);
   if (!stop) {
-    const double beta = rr * inv_gam, den = fma(-(beta * rr), inv_alpha, wr), inv = 1.0 / rr;
-    *(volatile double*)&S->alpha = rr / den;
-    *(volatile double*)&S->beta = beta;
-    bd.scal[0] = inv;
-    bd.scal[1] = den * inv;
+    if (kShare) {
+      *(volatile double*)&S->alpha = sc[0];
+      *(volatile double*)&S->beta = sc[1];
+    }
+    if (it == 0) bd.scal[0] = stop2;
+    bd.scal[1 + 2 * ((it + 1) & 1)] = st.inv_gam;
+    bd.scal[2 + 2 * ((it + 1) & 1)] = st.inv_alpha;
   } else {
     S->gam1 = rr;
     S->delta = wr;
@@ -1011,27 +1179,36 @@ template <bool kCg>
 __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd, BorderTasks tk, const double* b, double* x, int use_stop) {
   extern __shared__ double sm[];
   __shared__ double red[2 * 32];
-  __shared__ int s_it, s_t, go, last;
-  __shared__ double sc2[2];
+  __shared__ int s_it, s_t, s_next, go[2], last;
+  // the CG's scalars as this CTA has them: alpha and beta of iteration sc_it,
+  // the recurrence's state for iteration st_it, the threshold
+  __shared__ double sc2[2], s_stop2;
+  __shared__ CgState st2;
+  __shared__ int sc_it, st_it;
   if ((kCg || use_stop) && *(volatile const int*)&d.sc->stop) return;
   count_t* head = bd.ctl;
   count_t* ready = bd.ctl + kCtlReady;
   count_t* done = bd.ctl + kCtlDone;
   count_t* cnt = bd.ctl + kCtlCount;
   DevScalars* S = d.sc;
-  const int T = tk.off[6];
-  __shared__ __align__(8) uint64_t bars[kStages];
-  Ring ring{smem_addr(bars), 0, 0};
+  const int T = tk.off[kPhases];
+  __shared__ __align__(8) uint64_t bars[2 * kStages];
+  Ring ring = ring_init(bars, sm);
+  // thread 0: the first task of iteration s_it, waits known to be over (8 per
+  // iteration), a task claimed ahead by a run of products
+  count_t base = 0, seen = 0, pre = 0;
+  bool has_pre = false;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kStages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ring.bar + 8 * i));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    s_it = sc_it = 0;
+    st_it = -1;
+    sc2[0] = S->alpha;
+    sc2[1] = S->beta;
   }
-  count_t base = 0, seen = 0;  // thread 0: the first task of iteration s_it; phases known to be done (6 per iteration)
-  if (threadIdx.x == 0) s_it = 0;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) {
-      const count_t next = atomicAdd(head, count_t(1));
+      const count_t next = has_pre ? pre : atomicAdd(head, count_t(1));
+      has_pre = false;
       for (; next - base >= (count_t)T; base += T) ++s_it;
       s_t = (int)(next - base);
     }
@@ -1047,74 +1224,84 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     double* rout = it & 1 ? d.cg_r : bd.r2;
     double* sin = it & 1 ? bd.s2 : d.cg_s;
     double* sout = it & 1 ? d.cg_s : bd.s2;
-    BorderRhs q{b, rin, d.cg_w, sin, 0.0, 0.0};
-    // the CTA waits for the previous iteration's scalars (kCg), or for a phase
-    auto wait_for = [&](const count_t* p, count_t need, bool scal) {
+    // the CTA waits for a count
+    auto wait_for = [&](const count_t* p, count_t need, int mark, int* g) {
       if (threadIdx.x == 0) {
-        const count_t mark = (count_t)it * 6 + (scal ? 0 : ph);
-        const bool ok = mark < seen || border_wait(p, need, done, d);
-        seen = mark + 1;
-        go = ok;
+        const count_t m = (count_t)it * 8 + mark;
+        const bool ok = (mark >= 0 && m < seen) || border_wait(p, need, done, d);
+        if (mark >= 0 && m >= seen) seen = m + 1;
+        *g = ok;
         if (!ok && kCg && (*(volatile int*)&S->solve_flags & 1)) {
           *(volatile int*)&S->stop = 3;
           *(volatile count_t*)done = 1;
         }
-        if (kCg && scal) {
-          sc2[0] = *(volatile double*)&S->alpha;
-          sc2[1] = *(volatile double*)&S->beta;
-        }
       }
       __syncthreads();
-      if (kCg && scal) {
-        q.alpha = sc2[0];
-        q.beta = sc2[1];
-      }
       trace_mark(d, t, 1);
-      return go != 0;
+      return *g != 0;
     };
-    auto wait_ready = [&]() { return wait_for(ready, (count_t)it, true); };
-    auto wait_phase = [&]() { return wait_for(&cnt[tk.dep[ph] * kCtlStep], (count_t)(it + 1) * tk.n[tk.dep[ph]], false); };
+    // the products Jc^T follow the previous iteration's constraint tasks
+    auto wait_phase = [&]() { return wait_for(&cnt[tk.dep[ph] * kCtlStep], (count_t)(ph ? it + 1 : it) * tk.n[tk.dep[ph]], ph, &go[0]); };
+    // the iteration's alpha and beta in sc2, which every CTA computes itself
+    // from the constraint tasks' sums (one CTA's step and a second wait for it
+    // took 7.5 us an iteration, this 4.5); false at the loop's end
+    auto wait_scalars = [&]() {
+      if (!kCg || sc_it == it) return true;
+      const bool late = st_it != it;  // no state of its own: the last constraint task's
+      if (late && !wait_for(ready, (count_t)it - 1, -1, &go[1])) return false;
+      if (late) __syncthreads();
+      if (!wait_for(&cnt[6 * kCtlStep], (count_t)it * tk.n[6], 0, &go[1])) return false;
+      sum_parts(bd.rrp + ((it - 1) & 1) * tk.n_upd, bd.dlp, tk.n_upd, tk.n[6], red);
+      if (threadIdx.x == 0) {
+        CgState st = late ? cg_state(d, bd, it - 1) : st2;
+        if (late) s_stop2 = it > 1 ? __ldcg(&bd.scal[0]) : cg_stop2(d);
+        go[1] = !cg_step(d, st, s_stop2, red[0], red[1], it - 1, sc2);
+        st2 = st;
+        st_it = it + 1;
+        sc_it = it;
+      }
+      __syncthreads();
+      return go[1] != 0;
+    };
     bool scalars = false;
-    if (ph == 0 && task < tk.n_fwd) {
-      if (!block_fwd<kCg>(d, bd, q, ring, task, sm, wait_ready)) return;
-    } else if (ph == 0 && task < tk.n_fwd + tk.n_upd) {
+    int ndone = 1;
+    if (ph == 0) {
+      if (!rhs_parts_task(d, bd, task, rin, sin, wait_phase)) return;
+    } else if (ph == 1 && task < tk.n_fwd) {
+      if (!block_fwd<kCg>(bd, b, sc2, ring, task, sm, S, wait_phase, wait_scalars)) return;
+    } else if (ph == 1 && task < tk.n_fwd + tk.n_upd) {
       // p = r + beta p; s = w + beta s; x += alpha p; r -= alpha s; r.r
-      if (!wait_ready()) return;
       const int c = task - tk.n_fwd, k = c * kCgRows + threadIdx.x;
+      if (!wait_scalars()) return;
       double part[1] = {0.0};
       if (k < d.m_c) {
         const double r = __ldcg(&rin[k]), s0 = __ldcg(&sin[k]), w = __ldcg(&d.cg_w[k]), p0 = __ldcg(&d.cg_p[k]), x0 = __ldcg(&d.cg_x[k]);
-        const double sv = fma(q.beta, s0, w), p = fma(q.beta, p0, r), rn = fma(-q.alpha, sv, r);
+        const double alpha = sc2[0], beta = sc2[1];
+        const double sv = fma(beta, s0, w), p = fma(beta, p0, r), rn = fma(-alpha, sv, r);
         d.cg_p[k] = p;
         sout[k] = sv;
-        d.cg_x[k] = fma(q.alpha, p, x0);
+        d.cg_x[k] = fma(alpha, p, x0);
         rout[k] = rn;
         part[0] = rn * rn;
       }
       cta_sum<1>(part[0], red);
-      if (threadIdx.x == 0) bd.rrp[c] = red[8];
-    } else if (ph <= 1) {
-      // bt = b_S - sum u (in phase 0 there are no blocks)
-      const int j = (ph ? task : task - tk.n_fwd - tk.n_upd) * kRowTask + (threadIdx.x >> 2), sub = threadIdx.x & 3;
+      if (threadIdx.x == 0) bd.rrp[(it & 1) * tk.n_upd + c] = red[8];
+    } else if (ph <= 2) {
+      // bt = b_S - sum u (in phase 1 there are no blocks)
+      const int j = (ph == 2 ? task : task - tk.n_fwd - tk.n_upd) * kRowTask + (threadIdx.x >> 2), sub = threadIdx.x & 3;
       const int col = j < bd.k ? bd.bcol[j] : 0;
-      SparseRow row;
-      row.p = row.e = 0;
-      row.L = 4;
-      if (kCg && j < bd.k) load_rhs_row(d, row, col, 4, sub);
-      if (!wait_ready()) return;
-      double v = kCg ? rhs_row_dot(d, row, q) : j < bd.k && sub == 0 ? b[col] : 0.0;
-      if (ph == 1) {
-        __syncthreads();  // go is read before it is written again
-        if (!wait_phase()) return;
-        if (j < bd.k) v = dsub(v, border_updates(bd, j, sub));
-      }
-      v = join_row(v, 4);
+      if (!wait_scalars() || !wait_phase()) return;
+      double v = 0.0;
+      if (j < bd.k && sub == 0) v = kCg ? rhs_value(load_parts(bd, j), sc2) : b[col];
+      if (ph == 2 && j < bd.k) v = dsub(v, border_updates(bd, j, sub));
+      v = join_row(v);
       if (j < bd.k && sub == 0) bd.bt[j] = v;
-    } else if (ph <= 3) {
-      if (!(bd.rb == 4 ? border_gemv<4>(d, bd, ring, task, ph == 3, x, sm, wait_phase)
-                       : border_gemv<8>(d, bd, ring, task, ph == 3, x, sm, wait_phase)))
-        return;
-    } else if (ph == 4) {
+    } else if (ph <= 4) {
+      const count_t first = base + tk.off[ph];  // thread 0's base
+      ndone = bd.rb == 4 ? gemv_run<4>(d, bd, ring, task, tk.n[ph], ph == 4, x, sm, head, first, &s_next, pre, has_pre, tk.off[ph], wait_phase)
+                         : gemv_run<8>(d, bd, ring, task, tk.n[ph], ph == 4, x, sm, head, first, &s_next, pre, has_pre, tk.off[ph], wait_phase);
+      if (ndone < 0) return;
+    } else if (ph == 5) {
       if (!block_bwd(d, bd, ring, task, x, sm, wait_phase)) return;
     } else {
       // w = Jc_p x, delta = w.r
@@ -1127,7 +1314,7 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
       if (!wait_phase()) return;
       double part[1] = {0.0};
       const double r = k < d.m_c ? __ldcg(&rout[k]) : 0.0;
-      const double acc = join_row(row_dot(row, d.jcp_ci, d.jc_s, vi, [&](int c) { return __ldcg(&x[c]); }), 4);
+      const double acc = join_row(row_dot(row, d.jcp_ci, d.jc_s, vi, [&](int c) { return __ldcg(&x[c]); }));
       if (k < d.m_c && sub == 0) {
         d.cg_w[k] = acc;
         part[0] = acc * r;
@@ -1138,22 +1325,22 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     }
     // done: the CTA's writes, then the count
     __syncthreads();
-    trace_mark(d, t, 2);
+    if (ph != 3 && ph != 4) trace_mark(d, t, 2);
     if (!scalars) {
-      if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&cnt[ph * kCtlStep]) : "memory");
+      if (threadIdx.x == 0)
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&cnt[ph * kCtlStep]), "l"((count_t)ndone) : "memory");
       continue;
     }
     if (threadIdx.x == 0) {
       count_t old;
       asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], 1;" : "=l"(old) : "l"(&cnt[ph * kCtlStep]) : "memory");
-      last = old == (count_t)(it + 1) * tk.n[5] - 1;
+      last = old == (count_t)(it + 1) * tk.n[6] - 1;
     }
     __syncthreads();
     if (!last) continue;
-    // the last constraint task: both sums in a fixed order, one warp each, the
-    // recurrence and the stopping tests (k_spmv_jcp, k_cg_update)
-    sum_parts(bd, tk.n_upd, tk.n[5], red);
-    if (threadIdx.x == 0) cg_scalars(d, bd, red[0], red[1], it, it + 1, ready, done);
+    // the last constraint task: the step for good (k_spmv_jcp, k_cg_update)
+    sum_parts(bd.rrp + (it & 1) * tk.n_upd, bd.dlp, tk.n_upd, tk.n[6], red);
+    if (threadIdx.x == 0) cg_scalars<false>(d, bd, red[0], red[1], it, it + 1, ready, done);
   }
 }
 
@@ -1207,16 +1394,12 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
   __shared__ double red[2];
   __shared__ double sc2[2];
   __shared__ int s_it, s_t, go, last;
-  __shared__ __align__(8) uint64_t bars[kStages];
+  __shared__ __align__(8) uint64_t bars[2 * kStages];
   DevScalars* S = d.sc;
   if (*(volatile const int*)&S->stop) return;
-  Ring ring{smem_addr(bars), 0, 0};
+  Ring ring = ring_init(bars, sm);
   count_t *head = bd.ctl, *ready = bd.ctl + kCtlReady, *done = bd.ctl + kCtlDone, *cnt = bd.ctl + kCtlCount;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kStages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ring.bar + 8 * i));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    s_it = 0;
-  }
+  if (threadIdx.x == 0) s_it = 0;
   const int mc = bd.mc;
   count_t base = 0;
   for (;;) {
@@ -1230,7 +1413,7 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     const int q = s_it, task = s_t, row = task * RB + threadIdx.x;
     const bool own = threadIdx.x < RB && row < mc;
     const Panel p{bd.S + schur_panel(task, RB, mc), RB * mc};
-    panel_start(ring, p, sm);
+    panel_start(ring, p, S);
     double* const rin = q & 1 ? bd.r2 : d.cg_r;
     double* const rout = q & 1 ? d.cg_r : bd.r2;
     double* const sin = q & 1 ? bd.s2 : d.cg_s;
@@ -1311,10 +1494,10 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     }
     __syncthreads();
     if (!last) continue;
-    sum_parts(bd, tasks, tasks, red);
+    sum_parts(bd.rrp, bd.dlp, tasks, tasks, red);
     if (threadIdx.x == 0) {
       if (q > 1) {
-        cg_scalars(d, bd, red[0], red[1], q - 2, q + 1, ready, done);
+        cg_scalars<true>(d, bd, red[0], red[1], q - 2, q + 1, ready, done);
       } else {
         if (q == 0) {
           S->gam = S->gam0 = red[0];

@@ -584,8 +584,9 @@ void Engine::upload_border() {
   b.et = dev_alloc<double>(A, B, S.et_off[S.nblk]);
   b.cb = dev_alloc<double>(A, B, S.c_off[S.nblk]);
   b.W = dev_alloc<double>(A, B, (int64_t)b.ld * b.ld);
-  // products of the solves: with four rows a panel a border of up to 1,536
-  // columns runs in one wave of short tasks; above, eight
+  // products of the solves: four rows a panel keep the tasks of a small border
+  // short, eight halve the vector reads of a large one (5,000 buses, 3,342
+  // columns: 147 ms a solve against 164 with four)
   b.rb = S.k <= 1536 ? 4 : 8;
   b.nrb = cdiv(S.k, b.rb);
   b.nseg = cdiv(S.k, kGemvSeg);
@@ -615,6 +616,8 @@ void Engine::upload_border() {
   b.bt = dev_alloc<double>(A, B, b.ld);
   b.by = dev_alloc<double>(A, B, b.ld);
   const int nm = cdiv(S_.m_c, kCgRows);
+  b.njt = (int)(S.bcol.size() + S.blk_col.size());
+  b.jt = dev_alloc<double>(A, B, 3 * (int64_t)b.njt);
   b.r2 = dev_alloc<double>(A, B, S_.m_c);
   b.s2 = dev_alloc<double>(A, B, S_.m_c);
   // Schur plans: four rows a task up to 640 constraints, else eight (a task
@@ -622,9 +625,9 @@ void Engine::upload_border() {
   b.srb = S_.m_c <= 640 ? 4 : 8;
   b.w2 = dev_alloc<double>(A, B, b.mc);
   b.S = dev_alloc<double>(A, B, (int64_t)cdiv(b.mc, b.srb) * b.srb * b.mc);
-  b.rrp = dev_alloc<double>(A, B, std::max(nm, cdiv(b.mc, b.srb)));
+  b.rrp = dev_alloc<double>(A, B, std::max(2 * nm, cdiv(b.mc, b.srb)));
   b.dlp = dev_alloc<double>(A, B, std::max(cdiv(S_.m_c, kRowTask), cdiv(b.mc, b.srb)));
-  b.scal = dev_alloc<double>(A, B, 3);
+  b.scal = dev_alloc<double>(A, B, 5);
   b.ctl = dev_alloc<unsigned long long>(A, B, kCtlWords);
   // blocks by front size, so that small fronts share an SM
   blk_class_.assign(1, 0);
@@ -807,21 +810,25 @@ void Engine::record_border_solve(cudaStream_t st, const double* rhs, double* x, 
   t.n_fwd = b.nfp + cdiv(b.nblk - b.nbig, 8);
   t.n_upd = cg ? cdiv(d.m_c, kCgRows) : 0;
   const int rhs_tasks = cdiv(b.k, kRowTask);
-  t.n[0] = t.n_fwd + t.n_upd + (t.n_fwd ? 0 : rhs_tasks);
-  t.n[1] = t.n_fwd ? rhs_tasks : 0;
-  t.n[2] = b.n_lo;
-  t.n[3] = b.n_up;
-  t.n[4] = b.nbp + cdiv(b.nblk - b.nbig, 8);
-  t.n[5] = cg ? cdiv(d.m_c, kRowTask) : 0;
-  for (int q = 0, last = 0; q < 6; ++q) {
+  t.n[0] = cg ? cdiv(b.njt, kRowTask) : 0;
+  t.n[1] = t.n_fwd + t.n_upd + (t.n_fwd ? 0 : rhs_tasks);
+  t.n[2] = t.n_fwd ? rhs_tasks : 0;
+  t.n[3] = b.n_lo;
+  t.n[4] = b.n_up;
+  t.n[5] = b.nbp + cdiv(b.nblk - b.nbig, 8);
+  t.n[6] = cg ? cdiv(d.m_c, kRowTask) : 0;
+  for (int q = 0, last = 6; q < kPhases; ++q) {  // phase 0: the previous iteration's last; without the CG, nobody's
     t.off[q + 1] = t.off[q] + t.n[q];
     t.dep[q] = last;
     if (t.n[q]) last = q;
   }
   HYKKT_CUDA(cudaMemsetAsync(b.ctl, 0, kCtlWords * sizeof(unsigned long long), st));
-  // three CTAs per SM; with CTAs for all tasks (and, in the loop, the next
-  // iteration's) each one waits for its phase with its data at hand
-  const int grid = std::min(cg ? 2 * t.off[6] : t.off[6], std::max(16, sms_ * 3 / share_));
+  // a CTA per task of the longest phase, up to three per SM.  (CTAs for all
+  // phases claim earlier, but then a phase's tasks gather on the SMs whose CTAs
+  // came first: 34.3 us an iteration at 1,000 buses, so 30.9; 5,000: the same.)
+  int most = 0;
+  for (int q = 0; q < kPhases; ++q) most = std::max(most, t.n[q]);
+  const int grid = std::min(most, std::max(16, sms_ * 3 / share_));
   if (cg) {
     LAUNCH(k_border_solve<true>, grid, 256, kSolveSmem, st, d, b, t, rhs, x, use_stop);
   } else {

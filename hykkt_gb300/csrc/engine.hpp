@@ -194,11 +194,13 @@ struct DevBorder {
   int n_lo, n_up, nseg;  // tasks of the two products, most tasks per panel
   double* part;          // sums of the panels with several tasks
   int* rowcnt;
+  int njt;     // columns: border, then blocks
+  double* jt;  // CG: Jc_p^T r, Jc_p^T w, Jc_p^T s in that order
   double *r2, *s2, *w2;  // CG residual, direction and product of every second iteration
   double* S;             // Schur plans: S in panels of srb rows
   int srb;
-  double *rrp, *dlp;     // CG partial sums
-  double* scal;          // CG: 1/gamma, 1/alpha, the squared residual that stops
+  double *rrp, *dlp;     // CG partial sums (r.r: of two iterations)
+  double* scal;          // CG: the squared residual that stops; 1/gamma, 1/alpha of two iterations
   unsigned long long* ctl;  // task counters of one launch
 };
 
