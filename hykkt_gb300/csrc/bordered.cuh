@@ -566,11 +566,12 @@ __global__ void __launch_bounds__(256) k_border_pack(DevBorder bd) {
 // ---------------------------------------------------------------------------
 // Solves and the CG loop: one launch each, its CTAs claiming tasks of dense
 // phases from a counter in phase order.
-//   0  blocks:  y_F = X b_F, u = E b_F;       CG: the vector update as well
-//   1  border right-hand side  bt = b_S - sum u   (in phase 0 without blocks)
-//   2  by = X bt               3  x_S = X^T by
-//   4  blocks:  x_F = X^T y_F - E^T x_S
-//   5  CG: w = Jc_p x and the recurrence's scalars
+//   0  CG: Jc^T r, Jc^T w, Jc^T s
+//   1  blocks:  y_F = X b_F, u = E b_F;       CG: the vector update as well
+//   2  border right-hand side  bt = b_S - sum u   (in phase 1 without blocks)
+//   3  by = X bt               4  x_S = X^T by
+//   5  blocks:  x_F = X^T y_F - E^T x_S
+//   6  CG: w = Jc_p x and the sums of the recurrence's scalars
 // A task waits (bounded) until the tasks of the phase it reads from are done;
 // they were claimed before it by CTAs that are running, so the scheme cannot
 // deadlock whatever the number of resident CTAs.  What a task reads that the
@@ -707,97 +708,101 @@ __device__ __forceinline__ double border_updates(const DevBorder& bd, int j, int
 }
 
 // Products of a dense row panel, column after column of its RB rows, with a
-// vector in shared memory: 256 / RB threads a row over interleaved columns.
-// The panel streams through kStages shared-memory chunks by bulk copies that
-// thread 0 issues, the first of them before the task waits for its vector.  A
-// warp that has read a chunk says so on the chunk's second mbarrier, so that
-// warps run apart (a CTA barrier per chunk was a third of their stalls).
-constexpr int kGemvSeg = 2048, kChunk = 2048, kStages = 3;  // most columns of a panel, entries of a chunk
-constexpr int kRed = 256;                                   // doubles before the vector
-constexpr int kSolveSmem = (kRed + kGemvSeg + kStages * kChunk) * 8;
-
-struct Panel {
-  const double* M;
-  int n;  // entries: columns * RB
-  __device__ __forceinline__ int chunks() const { return (n + kChunk - 1) / kChunk; }
-};
+// vector: 256 / RB threads a row over interleaved columns.  Panels stream
+// through kStages shared-memory chunks by bulk copies that thread 0 issues, the
+// first of them before the task waits for its vector.  A warp that has read a
+// chunk says so on the chunk's second mbarrier, so that warps run apart (a CTA
+// barrier per chunk was a third of their stalls).
+constexpr int kChunk = 2048, kStages = 3;   // entries of a chunk
+constexpr int kRed = 512, kMaxVec = 256;    // doubles: two sets of partial sums, a block's vector
+constexpr int kChunkVec = 512;              // a chunk's piece of the vector (four rows a panel)
+constexpr int kSolveSmem = (kRed + kMaxVec + kStages * (kChunk + kChunkVec)) * 8;
+constexpr int kSchurMax = 2048;             // rows of a Schur plan, its vector in shared memory
+constexpr int kSchurSmem = (kRed + kSchurMax + kStages * kChunk) * 8;
 
 // The CTA's chunk ring: barriers [chunk full, chunk read], chunks issued
-// (thread 0) and consumed since the launch.
+// (thread 0), vector pieces issued (thread 0) and chunks consumed since the
+// launch.
 struct Ring {
-  uint32_t bar, buf;  // shared-memory addresses: 2 * kStages barriers, the chunks
-  unsigned put, got;
+  uint32_t bar;
+  double* buf;
+  int stride;  // doubles from chunk to chunk
+  unsigned put, vec, got;
 };
-__device__ __forceinline__ Ring ring_init(uint64_t* bars, double* sm) {
-  Ring g{smem_addr(bars), smem_addr(sm + kRed + kGemvSeg), 0, 0};
+// arrivals: 1, or 2 where a chunk's piece of the vector comes with it
+__device__ __forceinline__ Ring ring_init(uint64_t* bars, double* buf, int stride, int arrivals) {
+  Ring g{smem_addr(bars), buf, stride, 0, 0, 0};
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(g.bar + 8 * i));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(g.bar + 8 * i), "r"(arrivals));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(g.bar + 8 * (kStages + i)));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   return g;
 }
-// thread 0: chunk c of the panel into the next buffer, once all warps have read it
-__device__ __forceinline__ void ring_put(Ring& g, const Panel& p, int c, DevScalars* sc) {
-  const int st = g.put % kStages, n = min(kChunk, p.n - c * kChunk) * 8;
-  const uint32_t bar = g.bar + 8 * st;
+__device__ __forceinline__ void ring_copy(uint32_t bar, const double* dst, const double* src, int bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)), "l"(src),
+               "r"(bytes), "r"(bar) : "memory");
+}
+// thread 0: n entries from M into the next buffer, once all warps have read it
+__device__ __forceinline__ void ring_put(Ring& g, const double* M, int n, DevScalars* sc) {
+  const int st = g.put % kStages;
   mbar_wait(g.bar + 8 * (kStages + st), ((g.put / kStages) & 1) ^ 1, sc);
   ++g.put;
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   g.buf + st * (kChunk * 8)),
-               "l"(p.M + c * kChunk), "r"(n), "r"(bar) : "memory");
+  ring_copy(g.bar + 8 * st, g.buf + st * g.stride, M, n * 8);
 }
-__device__ __forceinline__ void panel_start(Ring& g, const Panel& p, DevScalars* sc) {
-  if (threadIdx.x == 0)
-    for (int c = 0; c < kStages && c * kChunk < p.n; ++c) ring_put(g, p, c, sc);
+// thread 0: the vector's part of the next chunk, n entries from v (0: none)
+__device__ __forceinline__ void ring_vec(Ring& g, const double* v, int n) {
+  const int st = g.vec % kStages;
+  ++g.vec;
+  if (n) ring_copy(g.bar + 8 * st, g.buf + st * g.stride + kChunk, v, (n * 8 + 15) & ~15);
+  else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(g.bar + 8 * st) : "memory");
 }
 // a task that gives up: thread 0 stays until the copies in flight have landed
-__device__ __forceinline__ void panel_drain(Ring& g, DevScalars* sc) {
-  if (threadIdx.x == 0)
+__device__ __forceinline__ void ring_drain(Ring& g, DevScalars* sc, bool vec) {
+  if (threadIdx.x == 0) {
+    for (; vec && g.vec < g.put;) ring_vec(g, nullptr, 0);
     for (; g.got < g.put; ++g.got) mbar_wait(g.bar + 8 * (g.got % kStages), (g.got / kStages) & 1, sc);
+  }
 }
 
-// The product of row threadIdx.x in threads below RB with the vector v in
-// shared memory.  refill(c): thread 0 issues what follows, chunk c's buffer (a
-// chunk ago) is free or about to be.
-template <int RB, class Refill>
-__device__ __forceinline__ double panel_product(Ring& g, const Panel& p, const double* v, double* sm, DevScalars* sc, Refill refill) {
-  constexpr int P = 256 / RB, kCols = kChunk / RB;
-  v += threadIdx.x / RB;
-  double a[2] = {0.0, 0.0};
-  int left = p.n / RB - threadIdx.x / RB;
-  for (int c = 0; c * kChunk < p.n; ++c, v += kCols, left -= kCols) {
-    const int st = g.got % kStages;
-    mbar_wait(g.bar + 8 * st, (g.got / kStages) & 1, sc);
-    ++g.got;
-    const double* m = sm + kRed + kGemvSeg + st * kChunk + threadIdx.x;
-    if (left > 7 * P) {
+// One chunk: `left` columns from this thread's first one on, into two sums
+template <int RB>
+__device__ __forceinline__ void chunk_product(Ring& g, const double* v, int left, double (&a)[2], DevScalars* sc) {
+  constexpr int P = 256 / RB;
+  const int st = g.got % kStages;
+  mbar_wait(g.bar + 8 * st, (g.got / kStages) & 1, sc);
+  ++g.got;
+  const double* m = g.buf + st * g.stride + threadIdx.x;
+  if (!v) v = g.buf + st * g.stride + kChunk + threadIdx.x / RB;
+  if (left > 7 * P) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) a[q & 1] = fma(m[q * 256], v[q * P], a[q & 1]);
-    } else {
+    for (int q = 0; q < 8; ++q) a[q & 1] = fma(m[q * 256], v[q * P], a[q & 1]);
+  } else {
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (q * P < left) a[q & 1] = fma(m[q * 256], v[q * P], a[q & 1]);
-    }
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0)
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(g.bar + 8 * (kStages + st)) : "memory");
-    if (threadIdx.x == 0 && c > 0) refill(c - 1);
+    for (int q = 0; q < 8; ++q)
+      if (q * P < left) a[q & 1] = fma(m[q * 256], v[q * P], a[q & 1]);
   }
-  // the P parts of a row: through shared memory to as many threads of the
-  // first warps as leave eight parts each (FP64 adds by full warps cost the
-  // product's time)
-  sm[threadIdx.x] = dadd(a[0], a[1]);
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0)
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(g.bar + 8 * (kStages + st)) : "memory");
+}
+
+// The 256 / RB parts of each row: through shared memory to as many threads of
+// the first warps as leave eight parts each (FP64 adds by full warps cost the
+// product's time).  Row threadIdx.x in threads below RB.
+template <int RB>
+__device__ __forceinline__ double panel_sum(double part, double* red) {
+  constexpr int P = 256 / RB, kParts = P < 8 ? P : 8, kT = 256 / kParts;  // parts per thread, threads
+  red[threadIdx.x] = part;
   __syncthreads();
-  constexpr int kParts = P < 8 ? P : 8, kT = 256 / kParts;  // parts per thread, threads
   double t = 0.0;
   if (threadIdx.x < kT) {
     double w[kParts];
 #pragma unroll
-    for (int q = 0; q < kParts; ++q) w[q] = sm[q * kT + threadIdx.x];
+    for (int q = 0; q < kParts; ++q) w[q] = red[q * kT + threadIdx.x];
 #pragma unroll
     for (int o = 1; o < kParts; o <<= 1)
 #pragma unroll
@@ -808,159 +813,121 @@ __device__ __forceinline__ double panel_product(Ring& g, const Panel& p, const d
   }
   return t;
 }
-template <int RB>
-__device__ __forceinline__ double panel_product(Ring& g, const Panel& p, double* sm, DevScalars* sc) {
-  return panel_product<RB>(g, p, sm + kRed, sm, sc, [&](int c) {
-    if (c + kStages < p.chunks()) ring_put(g, p, c + kStages, sc);
-  });
-}
 
-// by = X bt (up 0) or x_S = X^T by (up 1): a task is a panel's part in one
-// segment of kGemvSeg columns (X counts segments from the left, X^T from the
-// right).  A longer panel's tasks store their sums, the last one adds them in
-// segment order.  Bounded by FP64 issue (one multiply-add per entry, 2 per
-// clock and SM), by HBM where the panels exceed the L2.  Four rows a panel keep
-// a small border's tasks short, eight halve the vector reads of a large one.
-struct GemvTask {
-  int b, sg;      // panel, segment
-  int v0;         // first column of the segment (its vector starts there)
-  int j0, n;      // the task's columns
-  Panel p;
+// One panel with a vector that is in shared memory
+struct Panel {
+  const double* M;
+  int n;  // entries: columns * RB
 };
-template <int RB>
-__device__ __forceinline__ GemvTask gemv_task(const DevBorder& bd, int task, bool up) {
-  // by segment, in a segment the panels that reach it, longest first
-  GemvTask t;
-  t.sg = 0;
-  t.b = task;
-  for (int c = bd.nrb; t.b >= c; c = bd.nrb - t.sg * (kGemvSeg / RB)) {
-    t.b -= c;
-    ++t.sg;
-  }
-  if (up) {
-    const int end = bd.nrb * RB - t.sg * kGemvSeg;
-    t.v0 = max(0, end - kGemvSeg);
-    t.j0 = max(t.b * RB, t.v0);
-    t.n = min(bd.k, end) - t.j0;
-    t.p = Panel{bd.xup + panel_up(t.b, bd.nrb, RB) + (int64_t)(t.j0 - t.b * RB) * RB, t.n * RB};
-  } else {
-    t.b = bd.nrb - 1 - t.b;
-    t.v0 = t.j0 = t.sg * kGemvSeg;
-    t.n = min(kGemvSeg, min(bd.k, (t.b + 1) * RB) - t.j0);
-    t.p = Panel{bd.xlo + panel_lo(t.b, RB) + (int64_t)t.j0 * RB, t.n * RB};
-  }
-  return t;
-}
-
-// the segment's vector into shared memory
-__device__ __forceinline__ void gemv_vector(const DevBorder& bd, const GemvTask& t, bool up, double* v) {
-  const double* src = (up ? bd.by : bd.bt) + t.v0;
-  const int n = min(kGemvSeg, bd.k - t.v0);
-#pragma unroll
-  for (int h = 0; h < kGemvSeg / 256; h += 4) {
-    double r[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) r[q] = threadIdx.x + (h + q) * 256 < n ? __ldcg(&src[threadIdx.x + (h + q) * 256]) : 0.0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[threadIdx.x + (h + q) * 256] = r[q];
-    if ((h + 4) * 256 >= n) break;
-  }
-}
-
-// warp 0: the task's sums (rows in lanes below RB) to the result, by way of the
-// panel's slots where it has several tasks
-template <int RB>
-__device__ __forceinline__ void gemv_store(const DevBorder& bd, const GemvTask& t, bool up, double s, double* x) {
-  const int len = up ? bd.nrb * RB - t.b * RB : min(bd.k, (t.b + 1) * RB);
-  const int segs = (len + kGemvSeg - 1) / kGemvSeg, lane = threadIdx.x, row = t.b * RB + lane;
-  if (segs > 1) {
-    double* slot = bd.part + (int64_t)t.b * bd.nseg * RB;
-    if (lane < RB) __stcg(&slot[t.sg * RB + lane], s);
-    __syncwarp();
-    int fin = 0;
-    if (lane == 0) {
-      __threadfence();
-      fin = atomicAdd(&bd.rowcnt[t.b], 1) == segs - 1;
-      __threadfence();
+__device__ __forceinline__ void panel_start(Ring& g, const Panel& p, DevScalars* sc, bool vec) {
+  if (threadIdx.x == 0)
+    for (int c = 0; c < kStages && c * kChunk < p.n; ++c) {
+      ring_put(g, p.M + c * kChunk, min(kChunk, p.n - c * kChunk), sc);
+      if (vec) ring_vec(g, nullptr, 0);
     }
-    if (!__shfl_sync(0xffffffffu, fin, 0)) return;
-    if (lane < RB) {
-      s = __ldcg(&slot[lane]);
-      for (int q = 1; q < segs; ++q) s = dadd(s, __ldcg(&slot[q * RB + lane]));
+}
+template <int RB>
+__device__ __forceinline__ double panel_product(Ring& g, const Panel& p, const double* v, double* red, DevScalars* sc, bool vec) {
+  constexpr int kCols = kChunk / RB;
+  v += threadIdx.x / RB;
+  double a[2] = {0.0, 0.0};
+  int left = p.n / RB - threadIdx.x / RB;
+  for (int c = 0; c * kChunk < p.n; ++c, v += kCols, left -= kCols) {
+    chunk_product<RB>(g, v, left, a, sc);
+    const int next = (c - 1 + kStages) * kChunk;  // into the buffer of the chunk before, which all warps have or are about to have read
+    if (threadIdx.x == 0 && c > 0 && next < p.n) {
+      ring_put(g, p.M + next, min(kChunk, p.n - next), sc);
+      if (vec) ring_vec(g, nullptr, 0);
     }
-    if (lane == 0) bd.rowcnt[t.b] = 0;  // for the next product
   }
-  if (lane < RB && row < bd.k) {
-    if (up) x[bd.bcol[row]] = s;
-    else bd.by[row] = s;
-  }
+  return panel_sum<RB>(dadd(a[0], a[1]), red);
 }
 
-// A run of product tasks by one CTA from its claimed task `cur` on.  While many
-// tasks of the phase are left (two per CTA of the grid, so that none is held
-// back at the phase's end) thread 0 claims the next one at the start of the
-// current one, its first chunks follow the current one's through the ring, and
-// a vector segment stays for the tasks of the segment: between tasks there is
-// no round trip.  Returns the number of tasks done; a claimed task that is not
-// of this phase stays in `pre` (thread 0).
+// by = X bt or x_S = X^T by (up): a task is every stride-th of the bins from
+// `bin` on, a bin a set of whole panels; the bins hold equal work (the longest
+// panel of one side with short ones), longest first.  A chunk of a panel and
+// its piece of the vector come together, and the chunks of all the task's
+// panels follow one another through the ring.  Bounded by the FP64 pipe (an
+// entry is one multiply-add, two a clock and SM), by HBM where the panels
+// exceed the L2.  Measured: 44 us a product at 10,000 buses (6,746 columns, 39
+// at the FP64 peak) and 14 at 5,000 (3,342; 9).  (Tasks of one panel's piece of
+// 2,048 columns, unequal and claimed one by one, left an SM without a task for
+// 0.2 of the phase and with one or two for 0.25: 59 and 17 us.  Claiming the
+// next task ahead, during the last chunks: the same at 5,000, 2 % slower at
+// 10,000.)
+struct BinCursor {
+  int bin, i, next;  // bin, position in its list, the panel that follows there (read ahead; -1: none)
+  int b, n, c;       // panel, its entries, chunk
+  __device__ __forceinline__ void open(const DevBorder& bd, int q, bool up, int RB) {
+    next = bd.bin_panel[++i];
+    b = up ? bd.nrb - 1 - q : q;
+    n = up ? (bd.k - b * RB) * RB : min(bd.k, (b + 1) * RB) * RB;
+    c = 0;
+  }
+  __device__ __forceinline__ void start(const DevBorder& bd, int first, bool up, int RB) {
+    bin = first;
+    i = bin * bd.binw;
+    open(bd, bd.bin_panel[i], up, RB);
+  }
+  __device__ __forceinline__ void next_panel(const DevBorder& bd, int stride, bool up, int RB) {
+    if (next >= 0) {
+      open(bd, next, up, RB);
+      return;
+    }
+    bin += stride;
+    if (bin < bd.nbin) start(bd, bin, up, RB);
+  }
+  __device__ __forceinline__ void next_chunk(const DevBorder& bd, int stride, bool up, int RB) {
+    if (++c * kChunk >= n) next_panel(bd, stride, up, RB);
+  }
+};
+
 template <int RB, class Wait>
-__device__ __forceinline__ int gemv_run(const DevPlan& d, const DevBorder& bd, Ring& g, int cur, int ntask, bool up, double* x,
-                                        double* sm, count_t* head, count_t first, int* s_next, count_t& pre, bool& has_pre, int slot, Wait wait) {
-  double* v = sm + kRed;
-  GemvTask t = gemv_task<RB>(bd, cur, up);
-  int started = 0, have = -1, ndone = 0;  // started: thread 0, the task's chunks already issued
-  bool waited = false;
-  for (;;) {
-    const int chunks = t.p.chunks();
-    if (threadIdx.x == 0)
-      for (; started < kStages && started < chunks; ++started) ring_put(g, t.p, started, d.sc);
-    if (!waited && !wait()) {
-      panel_drain(g, d.sc);
-      return -1;
-    }
-    waited = true;
-    if (t.sg != have) {
-      gemv_vector(bd, t, up, v);
-      have = t.sg;
-    }
-    const bool ahead = cur + 2 * (int)gridDim.x < ntask;
-    count_t claim = 0;
-    if (ahead && threadIdx.x == 0) claim = atomicAdd(head, count_t(1));
-    __syncthreads();
-    trace_mark(d, slot + cur, 1);  // timeline: the run's tasks from tk.off[ph] on
-    trace_mark(d, slot + cur, 3);
-    int next = -2;  // thread 0: not looked at yet
-    Panel np{nullptr, 0};
-    auto look = [&]() {
-      next = ahead && claim - first < (count_t)ntask ? (int)(claim - first) : -1;
-      if (next >= 0) np = gemv_task<RB>(bd, next, up).p;
-      started = 0;
-    };
-    const double s = panel_product<RB>(g, t.p, v + (t.j0 - t.v0), sm, d.sc, [&](int c) {
-      if (c + kStages < chunks) {
-        ring_put(g, t.p, c + kStages, d.sc);
-      } else {
-        if (next == -2) look();
-        if (chunks >= kStages && started * kChunk < np.n) ring_put(g, np, started++, d.sc);
-      }
-    });
-    if (threadIdx.x < 32) gemv_store<RB>(bd, t, up, s, x);
-    ++ndone;
-    trace_mark(d, slot + cur, 2);
-    if (!ahead) return ndone;
-    if (threadIdx.x == 0) {
-      if (next == -2) look();
-      if (next < 0) {
-        pre = claim;
-        has_pre = true;
-      }
-      *s_next = next;
-    }
-    __syncthreads();
-    cur = *s_next;
-    if (cur < 0) return ndone;
-    t = gemv_task<RB>(bd, cur, up);
+__device__ __forceinline__ bool bin_task(const DevBorder& bd, Ring& g, int bin, int stride, bool up, double* x, double* sm, DevScalars* sc, Wait wait) {
+  constexpr int kCols = kChunk / RB;
+  BinCursor cur, put, vec;  // consumed (all threads); issued, vector pieces issued (thread 0)
+  cur.start(bd, bin, up, RB);
+  put = vec = cur;
+  auto put_next = [&]() {
+    const double* M = up ? bd.xup + panel_up(put.b, bd.nrb, RB) : bd.xlo + panel_lo(put.b, RB);
+    ring_put(g, M + put.c * kChunk, min(kChunk, put.n - put.c * kChunk), sc);
+    put.next_chunk(bd, stride, up, RB);
+  };
+  auto vec_next = [&]() {
+    const int j = vec.c * kCols;
+    ring_vec(g, up ? bd.by + vec.b * RB + j : bd.bt + j, min(kCols, vec.n / RB - j));
+    vec.next_chunk(bd, stride, up, RB);
+  };
+  if (threadIdx.x == 0)
+    for (int s = 0; s < kStages && put.bin < bd.nbin; ++s) put_next();
+  if (!wait()) {
+    ring_drain(g, sc, true);
+    return false;
   }
+  if (threadIdx.x == 0) {
+    asm volatile("fence.proxy.async;" ::: "memory");  // the vector was written by other CTAs' stores
+    while (g.vec < g.put) vec_next();
+  }
+  double* red = sm;
+  while (cur.bin < bd.nbin) {
+    const int row = cur.b * RB + threadIdx.x;
+    const int at = threadIdx.x < RB && row < bd.k ? (up ? bd.bcol[row] : row) : -1;
+    double a[2] = {0.0, 0.0};
+    int left = cur.n / RB - threadIdx.x / RB;
+    for (int e = cur.n; e > 0; e -= kChunk, left -= kCols) {
+      chunk_product<RB>(g, nullptr, left, a, sc);
+      if (threadIdx.x == 0)  // one chunk late, as above
+        while (g.put + 1 < g.got + kStages && put.bin < bd.nbin) {
+          put_next();
+          vec_next();
+              }
+    }
+    const double s = panel_sum<RB>(dadd(a[0], a[1]), red);
+    if (at >= 0) (up ? x : bd.by)[at] = s;
+    red = sm + (red == sm ? 256 : 0);  // warps below may still read this one
+    cur.next_panel(bd, stride, up, RB);
+  }
+  return true;
 }
 
 // Dot product of row `lane` of a warp's block panel (64 rows a column).
@@ -994,11 +961,11 @@ __device__ __forceinline__ bool block_fwd(const DevBorder& bd, const double* b, 
   const int i = big ? (int)threadIdx.x : lane;
   const int col = i < nt ? bd.blk_col[c0 + i] : 0;
   const Panel p{bd.ge + (have ? bd.ge_off[blk] + (int64_t)r0 * nt : 0), 64 * (r0 + 64 <= nt ? r0 + 64 : nt)};
-  if (big) panel_start(g, p, S);
+  if (big) panel_start(g, p, S, true);
   else prefetch_bytes(p.M, (int64_t)64 * nt * 8, lane, 32);
   double w = 0.0;
   if (!wait_scalars() || !wait()) {
-    panel_drain(g, S);
+    if (big) ring_drain(g, S, true);
     return false;
   }
   if (i < nt) w = kCg ? rhs_value(load_parts(bd, bd.k + c0 + i), sc) : b[col];
@@ -1006,7 +973,7 @@ __device__ __forceinline__ bool block_fwd(const DevBorder& bd, const double* b, 
   if (i < nt) v[i] = w;
   if (big) __syncthreads();
   else __syncwarp();
-  const double t = big ? panel_product<64>(g, p, sm, S) : warp_rows(p.M + lane, nt, v);
+  const double t = big ? panel_product<64>(g, p, v, sm, S, true) : warp_rows(p.M + lane, nt, v);
   if ((!big || i < 64) && r0 + i < N) {
     if (r0 + i < nt) bd.y[c0 + r0 + i] = t;
     else bd.u[bd.u_off[blk] + r0 + i - nt] = t;
@@ -1028,19 +995,19 @@ __device__ __forceinline__ bool block_bwd(const DevPlan& d, const DevBorder& bd,
   const int i = big ? (int)threadIdx.x : lane;
   const int brow = i < R ? bd.bcol[bd.blk_row[b0 + i]] : 0;
   const Panel p{bd.et + (have ? bd.et_off[blk] + (int64_t)t0 * N : 0), 64 * (N - t0)};
-  if (big) panel_start(g, p, d.sc);
+  if (big) panel_start(g, p, d.sc, true);
   else prefetch_bytes(p.M, (int64_t)64 * N * 8, lane, 32);
   const int r = t0 + (big ? (int)threadIdx.x & 63 : lane);
   const int col = r < nt ? bd.blk_col[c0 + r] : 0;
   if (!wait()) {
-    panel_drain(g, d.sc);
+    if (big) ring_drain(g, d.sc, true);
     return false;
   }
   double* v = big ? sm + kRed : sm + warp * 32;
   if (i < N) v[i] = i < R ? __ldcg(&x[brow]) : __ldcg(&bd.y[c0 + N - 1 - i]);
   if (big) __syncthreads();
   else __syncwarp();
-  const double t = big ? panel_product<64>(g, p, sm, d.sc) : warp_rows(p.M + lane, N, v);
+  const double t = big ? panel_product<64>(g, p, v, sm, d.sc, true) : warp_rows(p.M + lane, N, v);
   if ((!big || threadIdx.x < 64) && r < nt) x[col] = t;
   return true;
 }
@@ -1179,7 +1146,7 @@ template <bool kCg>
 __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd, BorderTasks tk, const double* b, double* x, int use_stop) {
   extern __shared__ double sm[];
   __shared__ double red[2 * 32];
-  __shared__ int s_it, s_t, s_next, go[2], last;
+  __shared__ int s_it, s_t, go[2], last;
   // the CG's scalars as this CTA has them: alpha and beta of iteration sc_it,
   // the recurrence's state for iteration st_it, the threshold
   __shared__ double sc2[2], s_stop2;
@@ -1193,11 +1160,10 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
   DevScalars* S = d.sc;
   const int T = tk.off[kPhases];
   __shared__ __align__(8) uint64_t bars[2 * kStages];
-  Ring ring = ring_init(bars, sm);
+  Ring ring = ring_init(bars, sm + kRed + kMaxVec, kChunk + kChunkVec, 2);
   // thread 0: the first task of iteration s_it, waits known to be over (8 per
-  // iteration), a task claimed ahead by a run of products
-  count_t base = 0, seen = 0, pre = 0;
-  bool has_pre = false;
+  // iteration)
+  count_t base = 0, seen = 0;
   if (threadIdx.x == 0) {
     s_it = sc_it = 0;
     st_it = -1;
@@ -1207,8 +1173,7 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) {
-      const count_t next = has_pre ? pre : atomicAdd(head, count_t(1));
-      has_pre = false;
+      const count_t next = atomicAdd(head, count_t(1));
       for (; next - base >= (count_t)T; base += T) ++s_it;
       s_t = (int)(next - base);
     }
@@ -1264,7 +1229,6 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
       return go[1] != 0;
     };
     bool scalars = false;
-    int ndone = 1;
     if (ph == 0) {
       if (!rhs_parts_task(d, bd, task, rin, sin, wait_phase)) return;
     } else if (ph == 1 && task < tk.n_fwd) {
@@ -1297,10 +1261,9 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
       v = join_row(v);
       if (j < bd.k && sub == 0) bd.bt[j] = v;
     } else if (ph <= 4) {
-      const count_t first = base + tk.off[ph];  // thread 0's base
-      ndone = bd.rb == 4 ? gemv_run<4>(d, bd, ring, task, tk.n[ph], ph == 4, x, sm, head, first, &s_next, pre, has_pre, tk.off[ph], wait_phase)
-                         : gemv_run<8>(d, bd, ring, task, tk.n[ph], ph == 4, x, sm, head, first, &s_next, pre, has_pre, tk.off[ph], wait_phase);
-      if (ndone < 0) return;
+      if (!(bd.rb == 4 ? bin_task<4>(bd, ring, task, tk.n[ph], ph == 4, x, sm, S, wait_phase)
+                       : bin_task<8>(bd, ring, task, tk.n[ph], ph == 4, x, sm, S, wait_phase)))
+        return;
     } else if (ph == 5) {
       if (!block_bwd(d, bd, ring, task, x, sm, wait_phase)) return;
     } else {
@@ -1325,10 +1288,10 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     }
     // done: the CTA's writes, then the count
     __syncthreads();
-    if (ph != 3 && ph != 4) trace_mark(d, t, 2);
+    trace_mark(d, t, 2);
     if (!scalars) {
       if (threadIdx.x == 0)
-        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&cnt[ph * kCtlStep]), "l"((count_t)ndone) : "memory");
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&cnt[ph * kCtlStep]), "l"(count_t(1)) : "memory");
       continue;
     }
     if (threadIdx.x == 0) {
@@ -1397,7 +1360,7 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
   __shared__ __align__(8) uint64_t bars[2 * kStages];
   DevScalars* S = d.sc;
   if (*(volatile const int*)&S->stop) return;
-  Ring ring = ring_init(bars, sm);
+  Ring ring = ring_init(bars, sm + kRed + kSchurMax, kChunk, 1);
   count_t *head = bd.ctl, *ready = bd.ctl + kCtlReady, *done = bd.ctl + kCtlDone, *cnt = bd.ctl + kCtlCount;
   if (threadIdx.x == 0) s_it = 0;
   const int mc = bd.mc;
@@ -1413,7 +1376,7 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     const int q = s_it, task = s_t, row = task * RB + threadIdx.x;
     const bool own = threadIdx.x < RB && row < mc;
     const Panel p{bd.S + schur_panel(task, RB, mc), RB * mc};
-    panel_start(ring, p, S);
+    panel_start(ring, p, S, false);
     double* const rin = q & 1 ? bd.r2 : d.cg_r;
     double* const rout = q & 1 ? d.cg_r : bd.r2;
     double* const sin = q & 1 ? bd.s2 : d.cg_s;
@@ -1432,7 +1395,7 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     }
     __syncthreads();
     if (!go) {
-      panel_drain(ring, S);
+      ring_drain(ring, S, false);
       return;
     }
     const double alpha = sc2[0], beta = sc2[1];
@@ -1455,7 +1418,7 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     double sv = 0.0;
     if (own && q > 1) sv = fma(beta, __ldcg(&sin[row]), __ldcg(&win[row]));
     __syncthreads();
-    const double t = panel_product<RB>(ring, p, sm, S);
+    const double t = panel_product<RB>(ring, p, sm + kRed, sm, S, false);
     double rr = 0.0, wr = 0.0;
     if (own) {
       double rn = r0;

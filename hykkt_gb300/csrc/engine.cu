@@ -11,6 +11,7 @@
 #include <mutex>
 #include <climits>
 #include <numeric>
+#include <queue>
 #include <stdexcept>
 #include <vector>
 
@@ -540,8 +541,8 @@ void Engine::upload_all() {
 
   HYKKT_CUDA(cudaFuncSetAttribute(k_piece_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_block_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, block_smem(kBlkRows)));
-  HYKKT_CUDA(cudaFuncSetAttribute(k_schur_cg<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
-  HYKKT_CUDA(cudaFuncSetAttribute(k_schur_cg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_schur_cg<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSchurSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_schur_cg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSchurSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_update<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
@@ -563,6 +564,9 @@ void Engine::upload_border() {
   const Bordered& S = S_.border;
   auto& A = allocs_;
   int64_t& B = dev_bytes_;
+  int dev = 0;
+  HYKKT_CUDA(cudaGetDevice(&dev));
+  HYKKT_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
   DevBorder b{};
   b.k = S.k;
   b.npan = cdiv(S.k, kBorderPanel);
@@ -584,16 +588,38 @@ void Engine::upload_border() {
   b.et = dev_alloc<double>(A, B, S.et_off[S.nblk]);
   b.cb = dev_alloc<double>(A, B, S.c_off[S.nblk]);
   b.W = dev_alloc<double>(A, B, (int64_t)b.ld * b.ld);
-  // products of the solves: four rows a panel keep the tasks of a small border
-  // short, eight halve the vector reads of a large one (5,000 buses, 3,342
-  // columns: 147 ms a solve against 164 with four)
-  b.rb = S.k <= 1536 ? 4 : 8;
+  // products of the solves: whole panels in as many bins as three CTAs per SM
+  // take at once (fewer, of at least 4,096 entries, but one per SM where the
+  // border is small), longest panel to emptiest bin.  Eight rows a panel where
+  // the longest one is a bin's share, else four, which read the vector twice as
+  // often but fill the bins evenly.
+  const int64_t entries = (int64_t)S.k * S.k / 2;
+  b.nbin = (int)std::min<int64_t>(3 * sms_, std::max<int64_t>(sms_, entries / 4096));
+  b.rb = 8LL * S.k * 9 <= entries / b.nbin * 10 ? 8 : 4;
   b.nrb = cdiv(S.k, b.rb);
-  b.nseg = cdiv(S.k, kGemvSeg);
-  for (int q = 0; q < b.nseg; ++q) b.n_lo += b.nrb - q * kGemvSeg / b.rb;
-  b.n_up = b.n_lo;
-  b.part = dev_alloc<double>(A, B, (int64_t)b.nrb * b.nseg * b.rb);
-  b.rowcnt = dev_alloc<int>(A, B, b.nrb);
+  b.nbin = std::min(b.nbin, b.nrb);
+  std::vector<int> bin_panel;
+  {
+    std::vector<std::vector<int>> bins(b.nbin);
+    std::vector<int64_t> sum(b.nbin, 0);
+    typedef std::pair<int64_t, int> Fill;
+    std::priority_queue<Fill, std::vector<Fill>, std::greater<Fill>> fill;
+    for (int q = 0; q < b.nbin; ++q) fill.push(Fill(0, q));
+    for (int q = b.nrb - 1; q >= 0; --q) {
+      const int to = fill.top().second;
+      fill.pop();
+      bins[to].push_back(q);
+      sum[to] += (int64_t)(q + 1) * b.rb * b.rb + kChunk / 2;  // half a chunk's time for a panel's sums
+      fill.push(Fill(sum[to], to));
+    }
+    std::vector<int> order(b.nbin);
+    for (int q = 0; q < b.nbin; ++q) order[q] = q;
+    std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return sum[p] > sum[q]; });
+    for (const auto& v : bins) b.binw = std::max(b.binw, (int)v.size() + 1);
+    bin_panel.assign((size_t)b.nbin * b.binw, -1);
+    for (int q = 0; q < b.nbin; ++q) std::copy(bins[order[q]].begin(), bins[order[q]].end(), bin_panel.begin() + (size_t)q * b.binw);
+  }
+  b.bin_panel = dev_upload(A, B, bin_panel);
   b.xlo = dev_alloc<double>(A, B, panel_lo(b.nrb, b.rb));
   b.xup = dev_alloc<double>(A, B, panel_up(b.nrb, b.nrb, b.rb));
   b.dig = dev_alloc<uint8_t>(A, B, (int64_t)b.ld / kRowBlock * kDigitBlockBytes);
@@ -636,9 +662,6 @@ void Engine::upload_border() {
     while (i < S.nblk && S.blk_rp[i + 1] - S.blk_rp[i] + S.blk_rrp[i + 1] - S.blk_rrp[i] > most) ++i;
     blk_class_.push_back(i);
   }
-  int dev = 0;
-  HYKKT_CUDA(cudaGetDevice(&dev));
-  HYKKT_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
   bord_ = b;
 }
 
@@ -792,9 +815,9 @@ void Engine::record_schur_cg(cudaStream_t st) {
   const int tasks = cdiv(b.mc, b.srb), grid = std::min(2 * tasks, std::max(16, sms_ * 3 / share_));
   HYKKT_CUDA(cudaMemsetAsync(b.ctl, 0, kCtlWords * sizeof(unsigned long long), st));
   if (b.srb == 4) {
-    LAUNCH(k_schur_cg<4>, grid, 256, kSolveSmem, st, dp, b, tasks);
+    LAUNCH(k_schur_cg<4>, grid, 256, kSchurSmem, st, dp, b, tasks);
   } else {
-    LAUNCH(k_schur_cg<8>, grid, 256, kSolveSmem, st, dp, b, tasks);
+    LAUNCH(k_schur_cg<8>, grid, 256, kSchurSmem, st, dp, b, tasks);
   }
 }
 
@@ -813,8 +836,11 @@ void Engine::record_border_solve(cudaStream_t st, const double* rhs, double* x, 
   t.n[0] = cg ? cdiv(b.njt, kRowTask) : 0;
   t.n[1] = t.n_fwd + t.n_upd + (t.n_fwd ? 0 : rhs_tasks);
   t.n[2] = t.n_fwd ? rhs_tasks : 0;
-  t.n[3] = b.n_lo;
-  t.n[4] = b.n_up;
+  // as many product tasks as CTAs at most: with a share of the GPU a task is
+  // several bins (eight 5,000-bus plans: 925 ms, 940 with two tasks per CTA, 965
+  // with a task per bin)
+  const int cap = std::max(16, sms_ * 3 / share_);
+  t.n[3] = t.n[4] = std::min(b.nbin, cap);
   t.n[5] = b.nbp + cdiv(b.nblk - b.nbig, 8);
   t.n[6] = cg ? cdiv(d.m_c, kRowTask) : 0;
   for (int q = 0, last = 6; q < kPhases; ++q) {  // phase 0: the previous iteration's last; without the CG, nobody's
@@ -828,7 +854,7 @@ void Engine::record_border_solve(cudaStream_t st, const double* rhs, double* x, 
   // came first: 34.3 us an iteration at 1,000 buses, so 30.9; 5,000: the same.)
   int most = 0;
   for (int q = 0; q < kPhases; ++q) most = std::max(most, t.n[q]);
-  const int grid = std::min(most, std::max(16, sms_ * 3 / share_));
+  const int grid = std::min(most, cap);
   if (cg) {
     LAUNCH(k_border_solve<true>, grid, 256, kSolveSmem, st, d, b, t, rhs, x, use_stop);
   } else {
@@ -1449,7 +1475,7 @@ void Engine::trace_trisolve(cudaStream_t st, std::vector<unsigned long long>& ou
   throw std::invalid_argument("the solve timeline is in measurement builds only (HYKKT_MEASURE=1)");
 #else
   const int n_blk = bord_.nfp + bord_.nbp + 2 * cdiv(bord_.nblk - bord_.nbig, 8);
-  const int64_t n = S_.border.on ? 4LL * (n_blk + cdiv(bord_.k, kRowTask) + bord_.n_lo + bord_.n_up) : 4LL * (sched_.ntasks_f + sched_.ntasks_b);
+  const int64_t n = S_.border.on ? 4LL * (n_blk + cdiv(bord_.k, kRowTask) + 2 * bord_.nbin) : 4LL * (sched_.ntasks_f + sched_.ntasks_b);
   unsigned long long* buf = nullptr;
   HYKKT_CUDA(cudaMallocAsync(&buf, std::max<int64_t>(n, 1) * sizeof(unsigned long long), st));
   HYKKT_CUDA(cudaMemsetAsync(buf, 0, std::max<int64_t>(n, 1) * sizeof(unsigned long long), st));

@@ -191,9 +191,8 @@ struct DevBorder {
   int nfp, nbp;          // 64-row panels of the blocks of more than 32 rows: [X; E], [-E^T X^T]
   const int *fp_blk, *fp_first, *bp_blk, *bp_first;  // their blocks, and each block's first panel
   int rb, nrb;           // rows per panel, panels
-  int n_lo, n_up, nseg;  // tasks of the two products, most tasks per panel
-  double* part;          // sums of the panels with several tasks
-  int* rowcnt;
+  int nbin, binw;        // sets of panels of equal work, longest first; list length
+  const int* bin_panel;  // nbin lists of panels, ended by -1
   int njt;     // columns: border, then blocks
   double* jt;  // CG: Jc_p^T r, Jc_p^T w, Jc_p^T s in that order
   double *r2, *s2, *w2;  // CG residual, direction and product of every second iteration

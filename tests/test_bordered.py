@@ -189,3 +189,20 @@ def test_schur_plan_matches_task_queues(n_bus, start, monkeypatch):
     assert abs(its[0] - its[1]) <= 2
     for a, b in zip(*sols):
         assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(a)
+
+
+@pytest.mark.gpu
+def test_wide_border_on_shares_of_the_gpu():
+    """A border wide enough for product panels of eight rows: tasks of one bin
+    and of several, the same bits from each, refined to the residual target."""
+    s = H.small_grid_system(n_bus=10000, seed=4)
+    p = hk.Plan(s)
+    assert len(p.symbolic("bd_col")) > 6600
+    p.set_accuracy(3000, 1e-11, 4, 1e-11)
+    sols = []
+    for share in (1, 3, 40):
+        p.set_concurrency(share)
+        assert p.solve(s) == hk.OK
+        sols.append(p.solution())
+    for other in sols[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(sols[0], other))
