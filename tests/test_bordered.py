@@ -129,6 +129,24 @@ def test_cholesky_sizes(shape, scale):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [65, 257, 700])
+@pytest.mark.parametrize("scale", [2.0 ** 300, 2.0 ** 964])
+def test_cholesky_near_overflow(n, scale):
+    """The update's sums are rounded with integers, beyond 2^900 by FP64: a
+    power of two through the matrix changes no bit of the solution."""
+    rng = np.random.default_rng(12)
+    A = _spd(n, rng)
+    r, c = np.nonzero(np.tril(A))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.int32)
+    ch = hk.Chol(n, rp, c.astype(np.int32))
+    b = rng.standard_normal(n)
+    assert ch.factor(A[r, c]) == hk.OK
+    x = ch.solve(b)
+    assert ch.factor(A[r, c] * scale) == hk.OK
+    assert np.array_equal(ch.solve(b * 2.0 ** 20) * (scale / 2.0 ** 20), x)
+
+
+@pytest.mark.gpu
 def test_not_finite_and_not_spd_are_reported():
     rng = np.random.default_rng(5)
     for shape in (200, (30, 20, 300)):
