@@ -253,8 +253,23 @@ __device__ __forceinline__ double minus_sums(double a, const int (&v)[8], int e)
 // block), beside the others, so that the panel kernel starts with M ready.
 __device__ void pivot_block(DevPlan& d, const DevBorder& bd, int panel, double* A, double* M) {
   constexpr int n = kBorderPanel, ld = n + 1;
-  __shared__ double sinv[n], mult[2][n];
+  __shared__ double sinv[n], piv[n], mult[2][n];
   const int tid = threadIdx.x, lane = tid & 31;
+  // threads 32 on: up to three (row, t < row) each, t the column of M, or past
+  // the pivot's the column t + 1 of A
+  int ei[3], et[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int f = tid - 32 + 224 * q;
+    int i = 0;
+    if (f >= 0 && f < n * (n - 1) / 2) {
+      i = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)f)) * 0.5f);
+      if (i * (i - 1) / 2 > f) --i;
+      if ((i + 1) * i / 2 <= f) ++i;
+    }
+    ei[q] = i;
+    et[q] = f - i * (i - 1) / 2;
+  }
   for (int e = tid; e < n * n; e += 256) M[(e / n) * ld + e % n] = e / n == e % n ? 1.0 : 0.0;
   __syncthreads();
   // warp 0, lane i: pivot k's multipliers A(i,k) / A(k,k) from the column c
@@ -263,8 +278,7 @@ __device__ void pivot_block(DevPlan& d, const DevBorder& bd, int panel, double* 
     const double inv = 1.0 / p;
     mult[k & 1][lane] = c * inv;
     if (lane == 0) {
-      const int col = panel * n + k;
-      if (col < bd.k) note_pivot(d, bd.bcol[col], p);
+      piv[k] = p;
       sinv[k] = inv;
     }
   };
@@ -281,23 +295,22 @@ __device__ void pivot_block(DevPlan& d, const DevBorder& bd, int panel, double* 
       }
       pivot(k + 1, c);
     } else {
-      // rows i > k, i + 1 entries each without column k + 1: j <= k of M, j > k + 1 of A
-      const int first = k + 1, count = n * (n - 1) / 2 - first * (first - 1) / 2;
-      for (int e = tid - 32; e < count; e += 224) {
-        const int f = e + first * (first - 1) / 2;
-        int i = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)f)) * 0.5f);
-        if (i * (i - 1) / 2 > f) --i;
-        if ((i + 1) * i / 2 <= f) ++i;
-        const int t = f - i * (i - 1) / 2, j = t <= k ? t : t + 1;  // t < i
-        double* g = j <= k ? &M[i * ld + j] : &A[i * ld + j];
-        *g = fma(-l[i], j <= k ? M[k * ld + j] : A[j * ld + k], *g);
-      }
+      // rows i > k: j <= k of M, j > k + 1 of A (column k + 1 is warp 0's)
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (ei[q] > k) {
+          const int i = ei[q], j = et[q] <= k ? et[q] : et[q] + 1;
+          double* g = j <= k ? &M[i * ld + j] : &A[i * ld + j];
+          *g = fma(-l[i], j <= k ? M[k * ld + j] : A[j * ld + k], *g);
+        }
     }
     __syncthreads();
   }
   double* out = bd.piv;
   for (int e = tid; e < n * n; e += 256) out[e] = M[(e / n) * ld + e % n];
   if (tid < n) {
+    const int col = panel * n + tid;
+    if (col < bd.k) note_pivot(d, bd.bcol[col], piv[tid]);
     out[n * n + tid] = sinv[tid];
     out[n * n + n + tid] = sqrt(sinv[tid]);
   }
