@@ -29,6 +29,8 @@ namespace hykkt {
 // so that F ends as X, B as -E and the border part as the Schur update.  A block's columns are sparse (they come from a subtree), so only
 // the nonzeros of v and w are visited.  Bounded by the pivots' latency.
 // ---------------------------------------------------------------------------
+// block columns of a back task's panel, by the rows of a border panel
+__host__ __device__ constexpr int back_rows(int rb) { return rb == 8 ? 64 : 32; }
 __device__ __forceinline__ int packed_lower(int i, int j) { return i * (i + 1) / 2 + j; }
 
 __global__ void __launch_bounds__(256) k_block_sweep(DevPlan d, DevBorder bd, int blk0) {
@@ -88,7 +90,7 @@ __global__ void __launch_bounds__(256) k_block_sweep(DevPlan d, DevBorder bd, in
     if (tid == 0) A[packed_lower(p, p)] = rs;
     __syncthreads();
   }
-  // [X; E] in panels of 64 rows and [-E^T X^T] in panels of 64 block columns,
+  // [X; E] in panels of 64 rows and [-E^T X^T] in panels of back_rows block columns,
   // column after column of the panel, zeros past the last row
   double* GE = bd.ge + bd.ge_off[blk];
   double* ET = bd.et + bd.et_off[blk];
@@ -99,8 +101,9 @@ __global__ void __launch_bounds__(256) k_block_sweep(DevPlan d, DevBorder bd, in
     else if (i < N) a = -A[packed_lower(i, t)];
     GE[e] = a;
   }
-  for (int e = tid; e < (nt + 63) / 64 * 64 * N; e += blockDim.x) {
-    const int t = e / (64 * N) * 64 + e % 64, i = e / 64 % N;  // entry i: border rows, then own from the last on
+  const int br = back_rows(bd.rb);
+  for (int e = tid; e < (nt + br - 1) / br * br * N; e += blockDim.x) {
+    const int t = e / (br * N) * br + e % br, i = e / br % N;  // entry i: border rows, then own from the last on
     double a = 0.0;
     if (t < nt) a = i < R ? A[packed_lower(nt + i, t)] : N - 1 - i >= t ? A[packed_lower(N - 1 - i, t)] : 0.0;
     ET[e] = a;
@@ -966,13 +969,14 @@ __device__ __forceinline__ bool bin_task(const DevBorder& bd, Ring& g, int bin, 
   return true;
 }
 
-// Dot product of row `lane` of a warp's block panel (64 rows a column).
+// Dot product of row `lane` of a warp's block panel (kRows rows a column).
+template <int kRows>
 __device__ __forceinline__ double warp_rows(const double* __restrict__ M, int K, const double* v) {
   double a[2] = {0.0, 0.0};
   for (int t = 0; t < K; t += 8) {
     double m[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) m[j] = t + j < K ? M[(t + j) * 64] : 0.0;
+    for (int j = 0; j < 8; ++j) m[j] = t + j < K ? M[(t + j) * kRows] : 0.0;
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       if (t + j < K) a[j & 1] = fma(m[j], v[t + j], a[j & 1]);
@@ -1009,7 +1013,7 @@ __device__ __forceinline__ bool block_fwd(const DevBorder& bd, const double* b, 
   if (i < nt) v[i] = w;
   if (big) __syncthreads();
   else __syncwarp();
-  const double t = big ? panel_product<64>(g, p, v, sm, S, true) : warp_rows(p.M + lane, nt, v);
+  const double t = big ? panel_product<64>(g, p, v, sm, S, true) : warp_rows<64>(p.M + lane, nt, v);
   if ((!big || i < 64) && r0 + i < N) {
     if (r0 + i < nt) bd.y[c0 + r0 + i] = t;
     else bd.u[bd.u_off[blk] + r0 + i - nt] = t;
@@ -1017,9 +1021,12 @@ __device__ __forceinline__ bool block_fwd(const DevBorder& bd, const double* b, 
   return true;
 }
 
-// x_F = X^T y_F - E^T x_S: the same for 64 columns of a block, whose own rows
-// come last and from the last one on, so that a chunk ends at its diagonal
-template <class Wait>
+// x_F = X^T y_F - E^T x_S: the same for 32 columns of a block, whose own rows
+// come last and from the last one on, so that a chunk ends at its diagonal.
+// (64 columns in wide systems, where tasks of 32 are more than the GPU holds:
+// the phase takes 9 us with 32 and 11.5 with 64 at 5,000 buses, 17.5 and 16 at
+// 10,000.)
+template <int kBackRows, class Wait>
 __device__ __forceinline__ bool block_bwd(const DevPlan& d, const DevBorder& bd, Ring& g, int task, double* x, double* sm, Wait wait) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool big = task < bd.nbp;
@@ -1027,13 +1034,13 @@ __device__ __forceinline__ bool block_bwd(const DevPlan& d, const DevBorder& bd,
   const bool have = blk < bd.nblk;
   const int c0 = have ? bd.blk_rp[blk] : 0, nt = have ? bd.blk_rp[blk + 1] - c0 : 0;
   const int b0 = have ? bd.blk_rrp[blk] : 0, R = have ? bd.blk_rrp[blk + 1] - b0 : 0, N = nt + R;
-  const int t0 = big ? 64 * (task - bd.bp_first[blk]) : 0;
+  const int t0 = big ? kBackRows * (task - bd.bp_first[blk]) : 0;
   const int i = big ? (int)threadIdx.x : lane;
   const int brow = i < R ? bd.bcol[bd.blk_row[b0 + i]] : 0;
-  const Panel p{bd.et + (have ? bd.et_off[blk] + (int64_t)t0 * N : 0), 64 * (N - t0)};
+  const Panel p{bd.et + (have ? bd.et_off[blk] + (int64_t)t0 * N : 0), kBackRows * (N - t0)};
   if (big) panel_start(g, p, d.sc, true);
-  else prefetch_bytes(p.M, (int64_t)64 * N * 8, lane, 32);
-  const int r = t0 + (big ? (int)threadIdx.x & 63 : lane);
+  else prefetch_bytes(p.M, (int64_t)kBackRows * N * 8, lane, 32);
+  const int r = t0 + (big ? (int)threadIdx.x % kBackRows : lane);
   const int col = r < nt ? bd.blk_col[c0 + r] : 0;
   if (!wait()) {
     if (big) ring_drain(g, d.sc, true);
@@ -1043,8 +1050,8 @@ __device__ __forceinline__ bool block_bwd(const DevPlan& d, const DevBorder& bd,
   if (i < N) v[i] = i < R ? __ldcg(&x[brow]) : __ldcg(&bd.y[c0 + N - 1 - i]);
   if (big) __syncthreads();
   else __syncwarp();
-  const double t = big ? panel_product<64>(g, p, v, sm, d.sc, true) : warp_rows(p.M + lane, N, v);
-  if ((!big || threadIdx.x < 64) && r < nt) x[col] = t;
+  const double t = big ? panel_product<kBackRows>(g, p, v, sm, d.sc, true) : warp_rows<kBackRows>(p.M + lane, N, v);
+  if ((!big || threadIdx.x < kBackRows) && r < nt) x[col] = t;
   return true;
 }
 
@@ -1178,8 +1185,8 @@ __device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, dou
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(ready), "l"((count_t)round) : "memory");
 }
 
-template <bool kCg>
-__global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd, BorderTasks tk, const double* b, double* x, int use_stop) {
+template <bool kCg, int RB>
+__global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd, const __grid_constant__ BorderTasks tk, const double* b, double* x, int use_stop) {
   extern __shared__ double sm[];
   __shared__ double red[2 * 32];
   __shared__ int s_it, s_t, go[2], last;
@@ -1297,11 +1304,9 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
       v = join_row(v);
       if (j < bd.k && sub == 0) bd.bt[j] = v;
     } else if (ph <= 4) {
-      if (!(bd.rb == 4 ? bin_task<4>(bd, ring, task, tk.n[ph], ph == 4, x, sm, S, wait_phase)
-                       : bin_task<8>(bd, ring, task, tk.n[ph], ph == 4, x, sm, S, wait_phase)))
-        return;
+      if (!bin_task<RB>(bd, ring, task, tk.n[ph], ph == 4, x, sm, S, wait_phase)) return;
     } else if (ph == 5) {
-      if (!block_bwd(d, bd, ring, task, x, sm, wait_phase)) return;
+      if (!block_bwd<back_rows(RB)>(d, bd, ring, task, x, sm, wait_phase)) return;
     } else {
       // w = Jc_p x, delta = w.r
       const int k = task * kRowTask + (threadIdx.x >> 2), sub = threadIdx.x & 3;

@@ -543,8 +543,10 @@ void Engine::upload_all() {
   HYKKT_CUDA(cudaFuncSetAttribute(k_block_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, block_smem(kBlkRows)));
   HYKKT_CUDA(cudaFuncSetAttribute(k_schur_cg<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSchurSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_schur_cg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSchurSmem));
-  HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
-  HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<true, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
+  HYKKT_CUDA(cudaFuncSetAttribute(k_border_solve<false, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_update<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_update<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
   HYKKT_CUDA(cudaFuncSetAttribute(k_border_update<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
@@ -633,7 +635,7 @@ void Engine::upload_border() {
     fpf.push_back((int)fpb.size());
     bpf.push_back((int)bpb.size());
     fpb.insert(fpb.end(), cdiv(nt + R, 64), i);
-    bpb.insert(bpb.end(), cdiv(nt, 64), i);
+    bpb.insert(bpb.end(), cdiv(nt, back_rows(b.rb)), i);
   }
   b.nfp = (int)fpb.size();
   b.nbp = (int)bpb.size();
@@ -856,9 +858,11 @@ void Engine::record_border_solve(cudaStream_t st, const double* rhs, double* x, 
   for (int q = 0; q < kPhases; ++q) most = std::max(most, t.n[q]);
   const int grid = std::min(most, cap);
   if (cg) {
-    LAUNCH(k_border_solve<true>, grid, 256, kSolveSmem, st, d, b, t, rhs, x, use_stop);
+    const auto k_border_cg = b.rb == 4 ? k_border_solve<true, 4> : k_border_solve<true, 8>;
+    LAUNCH(k_border_cg, grid, 256, kSolveSmem, st, d, b, t, rhs, x, use_stop);
   } else {
-    LAUNCH(k_border_solve<false>, grid, 256, kSolveSmem, st, d, b, t, rhs, x, use_stop);
+    const auto k_border_once = b.rb == 4 ? k_border_solve<false, 4> : k_border_solve<false, 8>;
+    LAUNCH(k_border_once, grid, 256, kSolveSmem, st, d, b, t, rhs, x, use_stop);
   }
 }
 

@@ -188,7 +188,7 @@ struct DevBorder {
   double* piv;           // the panel's pivot block: L^-1, 1/D, 1/sqrt(D)
   double *u, *bt, *by;   // per solve: E b_F of the blocks, the border's right-hand side, X times it
   double* y;             // per solve: X b_F of the blocks, in block order
-  int nfp, nbp;          // 64-row panels of the blocks of more than 32 rows: [X; E], [-E^T X^T]
+  int nfp, nbp;          // panels of the blocks of more than 32 rows: [X; E], [-E^T X^T]
   const int *fp_blk, *fp_first, *bp_blk, *bp_first;  // their blocks, and each block's first panel
   int rb, nrb;           // rows per panel, panels
   int nbin, binw;        // sets of panels of equal work, longest first; list length
