@@ -1074,8 +1074,11 @@ __device__ __forceinline__ count_t load_acquire(const count_t* p) {
   return v;
 }
 
-// thread 0: waits until *p >= need; false when the CG has stopped or the wait
-// gave up (wait_ge in kernels.cuh: the same limit, flag and test hook)
+// thread 0: waits until *p >= need; false when the wait gave up (wait_ge in
+// kernels.cuh: the same limit, flag and test hook) or, while it was not
+// satisfied, the CG has stopped.  kLast: also when it was satisfied after the
+// stop, which costs a second round trip.
+template <bool kLast>
 __device__ __forceinline__ bool border_wait(const count_t* p, count_t need, const count_t* done, const DevPlan& d) {
   need += d.dbg_unsatisfiable;
   if (need > 0) {
@@ -1088,7 +1091,7 @@ __device__ __forceinline__ bool border_wait(const count_t* p, count_t need, cons
       }
     }
   }
-  return !*(volatile const count_t*)done;  // set before the count that a stopped CG publishes
+  return !kLast || !*(volatile const count_t*)done;  // set before the count that a stopped CG publishes
 }
 
 // red[8] = the CTA's sum of v over every kStep-th lane (thread 0 reads it)
@@ -1232,11 +1235,14 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     double* rout = it & 1 ? d.cg_r : bd.r2;
     double* sin = it & 1 ? bd.s2 : d.cg_s;
     double* sout = it & 1 ? d.cg_s : bd.s2;
-    // the CTA waits for a count
+    // the CTA waits for a count.  (After the CG's end only the products Jc^T of
+    // the next iteration, which nobody reads, find theirs complete: what follows
+    // them computes the stop itself, and what follows that waits in vain until
+    // it sees the end.  So a wait costs one round trip, not two.)
     auto wait_for = [&](const count_t* p, count_t need, int mark, int* g) {
       if (threadIdx.x == 0) {
         const count_t m = (count_t)it * 8 + mark;
-        const bool ok = (mark >= 0 && m < seen) || border_wait(p, need, done, d);
+        const bool ok = (mark >= 0 && m < seen) || border_wait<false>(p, need, done, d);
         if (mark >= 0 && m >= seen) seen = m + 1;
         *g = ok;
         if (!ok && kCg && (*(volatile int*)&S->solve_flags & 1)) {
@@ -1425,7 +1431,7 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     double* const win = q & 1 ? bd.w2 : d.cg_w;
     double* const wout = q & 1 ? d.cg_w : bd.w2;
     if (threadIdx.x == 0) {
-      const bool ok = border_wait(ready, (count_t)q, done, d);
+      const bool ok = border_wait<true>(ready, (count_t)q, done, d);
       go = ok;
       if (!ok && (*(volatile int*)&S->solve_flags & 1)) {
         *(volatile int*)&S->stop = 3;
