@@ -1157,9 +1157,8 @@ __device__ __forceinline__ CgState cg_state(const DevPlan& d, const DevBorder& b
   if (it == 0) return CgState{1.0 / d.sc->gam, 1.0 / d.sc->alpha};
   return CgState{__ldcg(&bd.scal[1 + 2 * (it & 1)]), __ldcg(&bd.scal[2 + 2 * (it & 1)])};
 }
-// one thread: the step for good, its state, and its results (kShare: alpha and
-// beta for all CTAs; at the end what the loop leaves) through `ready`
-template <bool kShare>
+// one thread: the step for good, its state, and at the end what the loop leaves,
+// through `ready`
 __device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, double wr, int it, int round, count_t* ready, count_t* done) {
   DevScalars* S = d.sc;
   double sc[2];
@@ -1167,10 +1166,6 @@ __device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, dou
   const double stop2 = it ? __ldcg(&bd.scal[0]) : cg_stop2(d);
   const int stop = cg_step(d, st, stop2, rr, wr, it, sc);
   if (!stop) {
-    if (kShare) {
-      *(volatile double*)&S->alpha = sc[0];
-      *(volatile double*)&S->beta = sc[1];
-    }
     if (it == 0) bd.scal[0] = stop2;
     bd.scal[1 + 2 * ((it + 1) & 1)] = st.inv_gam;
     bd.scal[2 + 2 * ((it + 1) & 1)] = st.inv_alpha;
@@ -1350,7 +1345,7 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     if (!last) continue;
     // the last constraint task: the step for good (k_spmv_jcp, k_cg_update)
     sum_parts(bd.rrp + (it & 1) * tk.n_upd, bd.dlp, tk.n_upd, tk.n[6], red);
-    if (threadIdx.x == 0) cg_scalars<false>(d, bd, red[0], red[1], it, it + 1, ready, done);
+    if (threadIdx.x == 0) cg_scalars(d, bd, red[0], red[1], it, it + 1, ready, done);
   }
 }
 
@@ -1402,14 +1397,15 @@ template <int RB>
 __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, int tasks) {
   extern __shared__ double sm[];
   __shared__ double red[2];
-  __shared__ double sc2[2];
-  __shared__ int s_it, s_t, go, last;
+  __shared__ double sc2[2], s_stop2;  // as in k_border_solve
+  __shared__ CgState st2;
+  __shared__ int s_it, s_t, st_it, go, last;
   __shared__ __align__(8) uint64_t bars[2 * kStages];
   DevScalars* S = d.sc;
   if (*(volatile const int*)&S->stop) return;
   Ring ring = ring_init(bars, sm + kRed + kSchurMax, kChunk, 1);
   count_t *head = bd.ctl, *ready = bd.ctl + kCtlReady, *done = bd.ctl + kCtlDone, *cnt = bd.ctl + kCtlCount;
-  if (threadIdx.x == 0) s_it = 0;
+  if (threadIdx.x == 0) s_it = st_it = 0;
   const int mc = bd.mc;
   count_t base = 0;
   for (;;) {
@@ -1430,18 +1426,40 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     double* const sout = q & 1 ? d.cg_s : bd.s2;
     double* const win = q & 1 ? bd.w2 : d.cg_w;
     double* const wout = q & 1 ? d.cg_w : bd.w2;
+    // rounds 1 and 2 follow the last task's scalars, the later ones the tasks of
+    // the round before: every CTA computes their scalars itself, with the last
+    // task's state from two rounds before where it has none of its own
     if (threadIdx.x == 0) {
-      const bool ok = border_wait<true>(ready, (count_t)q, done, d);
+      bool ok = true;
+      if (q < 3 || st_it < q) ok = border_wait<true>(ready, (count_t)(q < 3 ? q : q - 1), done, d);
+      if (ok && q >= 3 && st_it <= q) ok = border_wait<false>(cnt, (count_t)q * tasks, done, d);
       go = ok;
       if (!ok && (*(volatile int*)&S->solve_flags & 1)) {
         *(volatile int*)&S->stop = 3;
         *(volatile count_t*)done = 1;
       }
-      sc2[0] = *(volatile double*)&S->alpha;
-      sc2[1] = *(volatile double*)&S->beta;
+      if (q < 3) {
+        sc2[0] = *(volatile double*)&S->alpha;
+        sc2[1] = *(volatile double*)&S->beta;
+      }
     }
     __syncthreads();
-    if (!go) {
+    bool on = go != 0;
+    if (on && q >= 3 && st_it <= q) {  // not its second task of the round
+      const int old = ((q - 1) & 1) * tasks;
+      sum_parts(bd.rrp + old, bd.dlp + old, tasks, tasks, red);
+      if (threadIdx.x == 0) {
+        const bool late = st_it != q;
+        CgState st = late ? cg_state(d, bd, q - 3) : st2;
+        if (late) s_stop2 = q > 3 ? __ldcg(&bd.scal[0]) : cg_stop2(d);
+        go = !cg_step(d, st, s_stop2, red[0], red[1], q - 3, sc2);
+        st2 = st;
+        st_it = q + 1;
+      }
+      __syncthreads();
+      on = go != 0;
+    }
+    if (!on) {
       ring_drain(ring, S, false);
       return;
     }
@@ -1492,8 +1510,8 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
         wr = dadd(wr, __shfl_xor_sync(0xffffffffu, wr, o));
       }
       if (threadIdx.x == 0) {
-        bd.rrp[task] = rr;
-        bd.dlp[task] = wr;
+        bd.rrp[(q & 1) * tasks + task] = rr;
+        bd.dlp[(q & 1) * tasks + task] = wr;
       }
     }
     __syncthreads();
@@ -1504,10 +1522,10 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     }
     __syncthreads();
     if (!last) continue;
-    sum_parts(bd.rrp, bd.dlp, tasks, tasks, red);
+    sum_parts(bd.rrp + (q & 1) * tasks, bd.dlp + (q & 1) * tasks, tasks, tasks, red);
     if (threadIdx.x == 0) {
       if (q > 1) {
-        cg_scalars<true>(d, bd, red[0], red[1], q - 2, q + 1, ready, done);
+        cg_scalars(d, bd, red[0], red[1], q - 2, q + 1, ready, done);
       } else {
         if (q == 0) {
           S->gam = S->gam0 = red[0];
