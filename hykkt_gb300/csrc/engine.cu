@@ -736,6 +736,23 @@ int Engine::profile(cudaStream_t st, int upto, std::vector<KernelTime>& out) {
     if (it == out.end()) out.push_back({e.name, 1, ms, 0.0, 0.0});
     else { it->launches += 1; it->ms += ms; }
   }
+  if (S_.border.on && upto >= 3) {
+    // a solve reads every entry of the border's X twice and of the blocks once
+    // in each direction; a Schur plan's iteration reads S
+    HYKKT_CUDA(cudaMemcpy(pin_sc_, dp.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost));
+    const Bordered& S = S_.border;
+    double e = (double)S.k * (S.k + 1);
+    for (int i = 0; i < S.nblk; ++i) {
+      const double nt = S.blk_rp[i + 1] - S.blk_rp[i], R = S.blk_rrp[i + 1] - S.blk_rrp[i];
+      e += nt * (nt + 1) + 2.0 * R * nt;
+    }
+    const double its = pin_sc_->it_total, mc2 = (double)S_.m_c * S_.m_c;
+    for (auto& k : out) {
+      if (k.name == "k_border_once") prof_work("k_border_once", 2.0 * e * k.launches, 8.0 * e * k.launches);
+      if (k.name == "k_border_cg") prof_work("k_border_cg", 2.0 * e * its, 8.0 * e * its);
+      if (k.name.rfind("k_schur_cg", 0) == 0) prof_work(k.name.c_str(), 2.0 * mc2 * its, 8.0 * mc2 * its);
+    }
+  }
   for (auto& k : out) {
     auto w = prof_work_.find(k.name);
     if (w != prof_work_.end()) { k.flops = w->second.first; k.bytes = w->second.second; }

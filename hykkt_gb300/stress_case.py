@@ -70,8 +70,11 @@ STAGES = {
     "formation": ("k_prepare", "k_ruiz_rowmax", "k_ruiz_scale", "k_hgamma"),
     "factorization": ("k_front_small", "k_front_scatter", "k_front_extadd", "k_panel_potrf", "k_panel_trsm",
                       "k_panel_update", "k_piece_inverse", "k_trtri_init", "k_trtri_diag", "k_trtri_update",
-                      "k_xpanel_pack"),
-    "triangular_solves": ("k_trsv_fwd", "k_trsv_bwd"),
+                      "k_xpanel_pack", "k_block_sweep", "k_border_assemble", "k_border_constraints",
+                      "k_border_pivot0", "k_border_panel", "k_border_update<1>", "k_border_update<2>",
+                      "k_border_update<4>", "k_border_pack", "k_schur_pack"),
+    # task queues: a launch a direction; bordered layout: one for both
+    "triangular_solves": ("k_trsv_fwd", "k_trsv_bwd", "k_border_once"),
 }
 
 
@@ -100,7 +103,9 @@ def main() -> None:
     sz = plan.sizes()
     out.update(nnz_L=sz["nnz_L"], front_arena_doubles=sz["front_arena"], n_supernodes=sz["n_supernodes"])
     sq_c0, sq_c1 = plan.symbolic("sq_c0"), plan.symbolic("sq_c1")
-    out["widest_solve_item"] = int((sq_c1 - sq_c0).max())
+    if len(sq_c0):  # task queues
+        out["widest_solve_item"] = int((sq_c1 - sq_c0).max())
+    out["border_columns"] = len(plan.symbolic("bd_col"))
     out["widest_supernode"] = int(np.diff(plan.symbolic("sn_first")).max())
     # accuracy-mode solve through the graph
     plan.set_accuracy(a.cg_itmax, a.cg_rtol, a.refine_max, 1e-8)
@@ -131,7 +136,7 @@ def main() -> None:
         v["GB_s"] = v["algorithmic_bytes"] / (v["ms"] * 1e6) if v["ms"] > 0 else None
         v["TFLOP_s"] = v["flops"] / (v["ms"] * 1e9) if v["ms"] > 0 and v["flops"] > 0 else None
     tri = stages["triangular_solves"]
-    tri["pair_ms"] = tri["ms"] / max(1, tri["launches"] // 2)
+    tri["pair_ms"] = tri["ms"] / max(1, tri["launches"] // (1 if "k_border_once" in prof else 2))
     out["stages"] = stages
     out["profile"] = {"cg_iterations": a.profile_cg_its, "kernels": {k: list(v) for k, v in prof.items()}}
     print(json.dumps(out), flush=True)

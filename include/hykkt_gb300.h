@@ -148,7 +148,9 @@ int hykkt_plan_create(hykkt_plan_t* plan, int n_x, int m_c, int m_d,
  * solve stages.  With pieces, small subtrees of warp-sized items are not
  * grouped into one-CTA tasks (that grouping shortens a lone solve and costs
  * throughput when plans share the GPU).  0 = whole supernodes (the default
- * of hykkt_plan_create). */
+ * of hykkt_plan_create).  With 0, and from 512 on, a plan takes the bordered
+ * layout instead of supernode tasks where that is estimated to be faster
+ * (HYKKT_BORDERED=0 in the environment keeps the tasks). */
 int hykkt_plan_create_ex(hykkt_plan_t* plan, int n_x, int m_c, int m_d,
                          const int* h_rowptr, const int* h_colidx, int nnz_h,
                          const int* ds_rowptr, const int* ds_colidx, int nnz_ds,
