@@ -1183,6 +1183,14 @@ __device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, dou
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(ready), "l"((count_t)round) : "memory");
 }
 
+// Whether the CG has stopped, one answer for the whole CTA (thread 0's read).
+// A CTA that starts late reads the flag while another one of the same launch
+// sets it: warps that read it for themselves could leave one by one, and the
+// ones that stay would run on barriers and shared variables that nobody set.
+__device__ __forceinline__ bool stopped_before(const DevScalars* S) {
+  return __syncthreads_or(threadIdx.x == 0 && *(volatile const int*)&S->stop) != 0;
+}
+
 template <bool kCg, int RB>
 __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd, const __grid_constant__ BorderTasks tk, const double* b, double* x, int use_stop) {
   extern __shared__ double sm[];
@@ -1193,7 +1201,7 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
   __shared__ double sc2[2], s_stop2;
   __shared__ CgState st2;
   __shared__ int sc_it, st_it;
-  if ((kCg || use_stop) && *(volatile const int*)&d.sc->stop) return;
+  if ((kCg || use_stop) && stopped_before(d.sc)) return;
   count_t* head = bd.ctl;
   count_t* ready = bd.ctl + kCtlReady;
   count_t* done = bd.ctl + kCtlDone;
@@ -1402,7 +1410,7 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
   __shared__ int s_it, s_t, st_it, go, last;
   __shared__ __align__(8) uint64_t bars[2 * kStages];
   DevScalars* S = d.sc;
-  if (*(volatile const int*)&S->stop) return;
+  if (stopped_before(S)) return;
   Ring ring = ring_init(bars, sm + kRed + kSchurMax, kChunk, 1);
   count_t *head = bd.ctl, *ready = bd.ctl + kCtlReady, *done = bd.ctl + kCtlDone, *cnt = bd.ctl + kCtlCount;
   if (threadIdx.x == 0) s_it = st_it = 0;
