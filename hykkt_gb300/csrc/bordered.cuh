@@ -1238,6 +1238,13 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     double* rout = it & 1 ? d.cg_r : bd.r2;
     double* sin = it & 1 ? bd.s2 : d.cg_s;
     double* sout = it & 1 ? d.cg_s : bd.s2;
+    // a wait that ran out ends the CG for all CTAs
+    auto gave_up = [&]() {
+      if (kCg && (*(volatile int*)&S->solve_flags & 1)) {
+        *(volatile int*)&S->stop = 3;
+        *(volatile count_t*)done = 1;
+      }
+    };
     // the CTA waits for a count.  (After the CG's end only the products Jc^T of
     // the next iteration, which nobody reads, find theirs complete: what follows
     // them computes the stop itself, and what follows that waits in vain until
@@ -1245,13 +1252,9 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     auto wait_for = [&](const count_t* p, count_t need, int mark, int* g) {
       if (threadIdx.x == 0) {
         const count_t m = (count_t)it * 8 + mark;
-        const bool ok = (mark >= 0 && m < seen) || border_wait<false>(p, need, done, d);
-        if (mark >= 0 && m >= seen) seen = m + 1;
-        *g = ok;
-        if (!ok && kCg && (*(volatile int*)&S->solve_flags & 1)) {
-          *(volatile int*)&S->stop = 3;
-          *(volatile count_t*)done = 1;
-        }
+        *g = m < seen || border_wait<false>(p, need, done, d);
+        if (m >= seen) seen = m + 1;
+        if (!*g) gave_up();
       }
       __syncthreads();
       trace_mark(d, t, 1);
@@ -1261,14 +1264,20 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     auto wait_phase = [&]() { return wait_for(&cnt[tk.dep[ph] * kCtlStep], (count_t)(ph ? it + 1 : it) * tk.n[tk.dep[ph]], ph, &go[0]); };
     // the iteration's alpha and beta in sc2, which every CTA computes itself
     // from the constraint tasks' sums (one CTA's step and a second wait for it
-    // took 7.5 us an iteration, this 4.5); false at the loop's end
+    // took 7.5 us an iteration, this 4.5); false at the loop's end.  Another
+    // thread waits meanwhile for the scalars that the CTA of the last
+    // constraint task left two iterations ago, which is nearly always over:
+    // that CTA sums the parts after its task counts as done, and this
+    // iteration's tasks write the buffers it read.
     auto wait_scalars = [&]() {
       if (!kCg || sc_it == it) return true;
       const bool late = st_it != it;  // no state of its own: the last constraint task's
-      if (late && !wait_for(ready, (count_t)it - 1, -1, &go[1])) return false;
-      if (late) __syncthreads();
-      if (!wait_for(&cnt[6 * kCtlStep], (count_t)it * tk.n[6], 0, &go[1])) return false;
-      sum_parts(bd.rrp + ((it - 1) & 1) * tk.n_upd, bd.dlp, tk.n_upd, tk.n[6], red);
+      if (threadIdx.x == 32) {
+        go[0] = border_wait<false>(ready, (count_t)it - 1, done, d);
+        if (!go[0]) gave_up();
+      }
+      if (!wait_for(&cnt[6 * kCtlStep], (count_t)it * tk.n[6], 0, &go[1]) || !go[0]) return false;
+      sum_parts(bd.rrp + ((it - 1) & 1) * tk.n_upd, bd.dlp + ((it - 1) & 1) * tk.n[6], tk.n_upd, tk.n[6], red);
       if (threadIdx.x == 0) {
         CgState st = late ? cg_state(d, bd, it - 1) : st2;
         if (late) s_stop2 = it > 1 ? __ldcg(&bd.scal[0]) : cg_stop2(d);
@@ -1333,7 +1342,7 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
         part[0] = acc * r;
       }
       cta_sum<4>(part[0], red);
-      if (threadIdx.x == 0) bd.dlp[task] = red[8];
+      if (threadIdx.x == 0) bd.dlp[(it & 1) * tk.n[6] + task] = red[8];
       scalars = true;
     }
     // done: the CTA's writes, then the count
@@ -1351,9 +1360,13 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     }
     __syncthreads();
     if (!last) continue;
-    // the last constraint task: the step for good (k_spmv_jcp, k_cg_update)
-    sum_parts(bd.rrp + (it & 1) * tk.n_upd, bd.dlp, tk.n_upd, tk.n[6], red);
-    if (threadIdx.x == 0) cg_scalars(d, bd, red[0], red[1], it, it + 1, ready, done);
+    // the last constraint task: the step for good (k_spmv_jcp, k_cg_update),
+    // after the previous iteration's, whose state it starts from
+    sum_parts(bd.rrp + (it & 1) * tk.n_upd, bd.dlp + (it & 1) * tk.n[6], tk.n_upd, tk.n[6], red);
+    if (threadIdx.x == 0) {
+      if (border_wait<false>(ready, (count_t)it, done, d)) cg_scalars(d, bd, red[0], red[1], it, it + 1, ready, done);
+      else gave_up();
+    }
   }
 }
 
@@ -1407,7 +1420,7 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
   __shared__ double red[2];
   __shared__ double sc2[2], s_stop2;  // as in k_border_solve
   __shared__ CgState st2;
-  __shared__ int s_it, s_t, st_it, go, last;
+  __shared__ int s_it, s_t, st_it, go[2], last;
   __shared__ __align__(8) uint64_t bars[2 * kStages];
   DevScalars* S = d.sc;
   if (stopped_before(S)) return;
@@ -1436,36 +1449,43 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     double* const wout = q & 1 ? d.cg_w : bd.w2;
     // rounds 1 and 2 follow the last task's scalars, the later ones the tasks of
     // the round before: every CTA computes their scalars itself, with the last
-    // task's state from two rounds before where it has none of its own
-    if (threadIdx.x == 0) {
-      bool ok = true;
-      if (q < 3 || st_it < q) ok = border_wait<true>(ready, (count_t)(q < 3 ? q : q - 1), done, d);
-      if (ok && q >= 3 && st_it <= q) ok = border_wait<false>(cnt, (count_t)q * tasks, done, d);
-      go = ok;
-      if (!ok && (*(volatile int*)&S->solve_flags & 1)) {
+    // task's state from two rounds before where it has none of its own.  Another
+    // thread waits meanwhile for those scalars, which is nearly always over: the
+    // last task's CTA sums the parts after its task counts as done, and this
+    // round's tasks write the buffers it read.
+    auto gave_up = [&]() {  // a wait that ran out ends the CG for all CTAs
+      if (*(volatile int*)&S->solve_flags & 1) {
         *(volatile int*)&S->stop = 3;
         *(volatile count_t*)done = 1;
       }
+    };
+    const bool own_step = q >= 3 && st_it <= q;  // not its second task of the round
+    if (threadIdx.x == 0) {
+      go[0] = q < 3 ? border_wait<true>(ready, (count_t)q, done, d) : !own_step || border_wait<false>(cnt, (count_t)q * tasks, done, d);
+      if (!go[0]) gave_up();
       if (q < 3) {
         sc2[0] = *(volatile double*)&S->alpha;
         sc2[1] = *(volatile double*)&S->beta;
       }
+    } else if (threadIdx.x == 32) {
+      go[1] = !own_step || border_wait<false>(ready, (count_t)q - 1, done, d);
+      if (!go[1]) gave_up();
     }
     __syncthreads();
-    bool on = go != 0;
-    if (on && q >= 3 && st_it <= q) {  // not its second task of the round
+    bool on = go[0] && go[1];
+    if (on && own_step) {
       const int old = ((q - 1) & 1) * tasks;
       sum_parts(bd.rrp + old, bd.dlp + old, tasks, tasks, red);
       if (threadIdx.x == 0) {
         const bool late = st_it != q;
         CgState st = late ? cg_state(d, bd, q - 3) : st2;
         if (late) s_stop2 = q > 3 ? __ldcg(&bd.scal[0]) : cg_stop2(d);
-        go = !cg_step(d, st, s_stop2, red[0], red[1], q - 3, sc2);
+        go[0] = !cg_step(d, st, s_stop2, red[0], red[1], q - 3, sc2);
         st2 = st;
         st_it = q + 1;
       }
       __syncthreads();
-      on = go != 0;
+      on = go[0] != 0;
     }
     if (!on) {
       ring_drain(ring, S, false);
@@ -1533,7 +1553,9 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     sum_parts(bd.rrp + (q & 1) * tasks, bd.dlp + (q & 1) * tasks, tasks, tasks, red);
     if (threadIdx.x == 0) {
       if (q > 1) {
-        cg_scalars(d, bd, red[0], red[1], q - 2, q + 1, ready, done);
+        // after the previous round's step, whose state it starts from
+        if (border_wait<false>(ready, (count_t)q, done, d)) cg_scalars(d, bd, red[0], red[1], q - 2, q + 1, ready, done);
+        else gave_up();
       } else {
         if (q == 0) {
           S->gam = S->gam0 = red[0];

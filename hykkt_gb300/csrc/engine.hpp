@@ -198,7 +198,7 @@ struct DevBorder {
   double *r2, *s2, *w2;  // CG residual, direction and product of every second iteration
   double* S;             // Schur plans: S in panels of srb rows
   int srb;
-  double *rrp, *dlp;     // CG partial sums (r.r: of two iterations)
+  double *rrp, *dlp;     // CG partial sums of two iterations
   double* scal;          // CG: the squared residual that stops; 1/gamma, 1/alpha of two iterations
   unsigned long long* ctl;  // task counters of one launch
 };

@@ -34,3 +34,25 @@ def test_plans_in_flight_at_default_share(rtol):
             assert p.wait() == st
             assert p.info()["cg_iterations_total"] == its
             assert all(np.array_equal(a, b) for a, b in zip(sol, p.solution()))
+
+
+@pytest.mark.parametrize("n_bus", [60, 460, 900])
+def test_cg_hand_over_beside_factorizations(n_bus):
+    """The CTA that takes an iteration's last step, held up by another plan's
+    factorizations, hands its state to the next one's last step: the iterates
+    stay those of the lone run at every share of the GPU."""
+    s = H.small_grid_system(n_bus=n_bus, seed=9, dx=(1e-8, 1e4), ds=(1e-8, 1e8))
+    big = H.small_grid_system(n_bus=3000, seed=10)
+    p, q = hk.Plan(s), hk.Plan(big)
+    p.set_accuracy(2000, 1e-11, 0, 1e-10)
+    q.set_accuracy(1, 1e-1, 0, 1e-10)
+    st = p.solve(s)
+    its, sol = p.info()["cg_iterations_total"], p.solution()
+    for share in (1, 3, 40):
+        p.set_concurrency(share)
+        for _ in range(4):
+            q.solve(big, sync=False)
+            assert p.solve(s) == st
+            assert p.info()["cg_iterations_total"] == its
+            assert all(np.array_equal(a, b) for a, b in zip(sol, p.solution()))
+            q.wait()
