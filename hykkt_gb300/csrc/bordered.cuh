@@ -758,6 +758,8 @@ constexpr int kChunkVec = 512;              // a chunk's piece of the vector (fo
 constexpr int kSolveSmem = (kRed + kMaxVec + kStages * (kChunk + kChunkVec)) * 8;
 constexpr int kSchurMax = 2048;             // rows of a Schur plan, its vector in shared memory
 constexpr int kSchurSmem = (kRed + kSchurMax + kStages * kChunk) * 8;
+static_assert(kRed % 2 == 0 && kMaxVec % 2 == 0 && kSchurMax % 2 == 0 && kChunk % 2 == 0 && kChunkVec % 2 == 0,
+              "bulk copies go to 16-byte boundaries");
 
 // The CTA's chunk ring: barriers [chunk full, chunk read], chunks issued
 // (thread 0), vector pieces issued (thread 0) and chunks consumed since the
@@ -1193,7 +1195,7 @@ __device__ __forceinline__ bool stopped_before(const DevScalars* S) {
 
 template <bool kCg, int RB>
 __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd, const __grid_constant__ BorderTasks tk, const double* b, double* x, int use_stop) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(128) double sm[];  // destination of bulk copies
   __shared__ double red[2 * 32];
   __shared__ int s_it, s_t, go[2], last;
   // the CG's scalars as this CTA has them: alpha and beta of iteration sc_it,
@@ -1416,7 +1418,7 @@ __global__ void __launch_bounds__(256) k_schur_pack(DevBorder bd) {
 // r.r.  Vectors that other tasks read are double-buffered.
 template <int RB>
 __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, int tasks) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(128) double sm[];  // destination of bulk copies
   __shared__ double red[2];
   __shared__ double sc2[2], s_stop2;  // as in k_border_solve
   __shared__ CgState st2;
