@@ -1322,8 +1322,9 @@ extern "C" int hykkt_chol_create(hykkt_chol_t* c, int n, int nnz, const int* row
         if (it == end || *it != a) throw std::runtime_error("chol: entry not in pattern");
         src[it - S.lp_row.data()] = p;
       }
+    S.entry_src = std::move(src);
+    S.entry_n = nnz;
     h->eng = std::make_unique<Engine>(std::move(S), 0.0, opt);
-    h->eng->set_entry_map(src, nnz);
     HYKKT_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     *c = h.release();
     return HYKKT_OK;

@@ -220,8 +220,6 @@ Engine::~Engine() {
   if (cap_stream_) cudaStreamDestroy(cap_stream_);
   if (last_launch_) cudaEventDestroy(last_launch_);
   free_storage(allocs_);
-  if (entry_src_) cudaFree(entry_src_);
-  if (entry_vals_) cudaFree(entry_vals_);
   if (pin_in_) cudaFreeHost(pin_in_);
   if (pin_out_) cudaFreeHost(pin_out_);
   if (pin_sc_) cudaFreeHost(pin_sc_);
@@ -324,6 +322,13 @@ void Engine::upload_all() {
   d.lp_htsrc = dev_upload(A, B, S.lp_htsrc); d.lp_ccp = dev_upload(A, B, S.lp_ccp);
   d.lp_ca = dev_upload(A, B, S.lp_ca); d.lp_cb = dev_upload(A, B, S.lp_cb); d.lp_lrow = dev_upload(A, B, S.lp_lrow);
   d.lp_v = dev_alloc<double>(A, B, S.lp_cp[S.n_x]);
+  if (S.entry_n >= 0) {
+    entry_src_ = dev_upload(A, B, S.entry_src);
+    entry_vals_ = dev_alloc<double>(A, B, S.entry_n);
+    int dev = 0;
+    HYKKT_CUDA(cudaGetDevice(&dev));
+    HYKKT_CUDA(cudaDeviceGetAttribute(&reads_host_, cudaDevAttrPageableMemoryAccess, dev));
+  }
   d.perm = dev_upload(A, B, S.perm); d.rev_perm = dev_upload(A, B, S.rev_perm);
   d.jcp_ci = dev_upload(A, B, S.jcp_ci);
   d.jctp_rp = dev_upload(A, B, S.jctp_rp); d.jctp_ci = dev_upload(A, B, S.jctp_ci); d.jctp_src = dev_upload(A, B, S.jctp_src);
@@ -1550,22 +1555,12 @@ __global__ void k_gather_lower(DevPlan d, const int* __restrict__ src, const dou
     d.lp_v[q] = src[q] >= 0 ? vals[src[q]] : 0.0;
 }
 
-// Entry of the caller's array behind each permuted lower entry (-1: none, 0.0).
-void Engine::set_entry_map(const std::vector<int>& src, int64_t nnz) {
-  HYKKT_CUDA(cudaMalloc(&entry_src_, std::max<size_t>(src.size(), 1) * sizeof(int)));
-  HYKKT_CUDA(cudaMemcpy(entry_src_, src.data(), src.size() * sizeof(int), cudaMemcpyHostToDevice));
-  HYKKT_CUDA(cudaMalloc(&entry_vals_, std::max<int64_t>(nnz, 1) * sizeof(double)));
-  entry_n_ = nnz;
-  int dev = 0;
-  HYKKT_CUDA(cudaGetDevice(&dev));
-  HYKKT_CUDA(cudaDeviceGetAttribute(&reads_host_, cudaDevAttrPageableMemoryAccess, dev));
-}
-
 int Engine::factor_values(const double* vals_host, cudaStream_t st) {
   reload_device();
-  if (entry_n_ > 0) {
-    if (reads_host_) k_read_host<<<std::min(cdiv(entry_n_, 1024), 152 * 8), 256, 0, st>>>(vals_host, entry_vals_, entry_n_);
-    else HYKKT_CUDA(cudaMemcpyAsync(entry_vals_, vals_host, (size_t)entry_n_ * sizeof(double), cudaMemcpyHostToDevice, st));
+  const int64_t n = S_.entry_n;
+  if (n > 0) {
+    if (reads_host_) k_read_host<<<std::min(cdiv(n, 1024), 152 * 8), 256, 0, st>>>(vals_host, entry_vals_, n);
+    else HYKKT_CUDA(cudaMemcpyAsync(entry_vals_, vals_host, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st));
   }
   k_gather_lower<<<std::max(1, std::min(cdiv(dp.nnz_lo, 256), 152 * 16)), 256, 0, st>>>(dp, entry_src_, entry_vals_);
   HYKKT_CUDA(cudaGetLastError());

@@ -256,10 +256,8 @@ class Engine {
   // task (forward tasks, then backward) {claimed, dependencies met, done,
   // SM id} with times in ns of the GPU's global timer.
   void trace_trisolve(cudaStream_t stream, std::vector<unsigned long long>& out);
-  // Components: factor from a caller's host values, whose entry behind each
-  // permuted lower entry set_entry_map gives once; CG on S = Jc H^{-1} Jc^T
-  // with this factor.
-  void set_entry_map(const std::vector<int>& src, int64_t nnz);
+  // Components: factor from a caller's host values (Symbolic::entry_src says
+  // where they go); CG on S = Jc H^{-1} Jc^T with this factor.
   int factor_values(const double* vals_host, cudaStream_t stream);
   int schur_cg(int m, const std::vector<int>& jc_rp, const std::vector<int>& jc_ci, const double* jc_v_host,
                const double* b_host, double* x_host, int itmax, double tol, int* iters, double* err,
@@ -376,7 +374,6 @@ class Engine {
   DevScalars* pin_sc_ = nullptr;
   int* entry_src_ = nullptr;  // Cholesky component: entry map, device copy of the caller's values
   double* entry_vals_ = nullptr;
-  int64_t entry_n_ = 0;
   int reads_host_ = 0;        // the GPU reads pageable host memory
   cudaEvent_t last_launch_ = nullptr;  // recorded after each asynchronous graph launch
   int64_t pin_in_n_ = 0, pin_out_n_ = 0;

@@ -243,6 +243,11 @@ struct Symbolic {
   // fronts and solve items above are then not built
   Bordered border;
 
+  // Cholesky component: the caller's array (entry_n values, -1: none) behind
+  // each permuted lower entry (-1: none, the entry is 0.0)
+  std::vector<int> entry_src;
+  int64_t entry_n = -1;
+
   // Jc with permuted column indices (Jc_p = Jc P^T, values in Jc order)
   std::vector<int> jcp_ci;
   // Jc_p^T rows in permuted order: row i = Jc^T row perm[i]
