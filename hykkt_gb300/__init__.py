@@ -487,6 +487,8 @@ class Chol:
 
     def factor(self, vals) -> int:
         v = _f64(vals)
+        if v.size < int(self._rp[-1]):  # the GPU reads the array itself
+            raise HykktError(INVALID, f"{v.size} values for {int(self._rp[-1])} entries")
         return lib().hykkt_chol_factor(self.h, _p(v))
 
     def solve(self, b) -> np.ndarray:

@@ -1333,6 +1333,7 @@ extern "C" int hykkt_chol_create(hykkt_chol_t* c, int n, int nnz, const int* row
 
 extern "C" int hykkt_chol_factor(hykkt_chol_t c, const double* vals) {
   return guarded([&]() {
+    if (!vals && c->nnz > 0) return fail(HYKKT_INVALID, "NULL values");
     return c->eng->factor_values(vals, c->stream);
   });
 }

@@ -1557,10 +1557,23 @@ __global__ void k_gather_lower(DevPlan d, const int* __restrict__ src, const dou
 
 int Engine::factor_values(const double* vals_host, cudaStream_t st) {
   reload_device();
+  try {
+    return factor_values_on(vals_host, st);
+  } catch (...) {
+    cudaStreamSynchronize(st);  // whatever was enqueued has read the caller's array
+    throw;
+  }
+}
+
+int Engine::factor_values_on(const double* vals_host, cudaStream_t st) {
   const int64_t n = S_.entry_n;
   if (n > 0) {
-    if (reads_host_) k_read_host<<<std::min(cdiv(n, 1024), 152 * 8), 256, 0, st>>>(vals_host, entry_vals_, n);
-    else HYKKT_CUDA(cudaMemcpyAsync(entry_vals_, vals_host, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st));
+    // in place only from an array of whole doubles (a view into a byte buffer
+    // may start anywhere, which a kernel's loads cannot)
+    if (reads_host_ && reinterpret_cast<uintptr_t>(vals_host) % alignof(double) == 0)
+      k_read_host<<<std::min(cdiv(n, 1024), 152 * 8), 256, 0, st>>>(vals_host, entry_vals_, n);
+    else
+      HYKKT_CUDA(cudaMemcpyAsync(entry_vals_, vals_host, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st));
   }
   k_gather_lower<<<std::max(1, std::min(cdiv(dp.nnz_lo, 256), 152 * 16)), 256, 0, st>>>(dp, entry_src_, entry_vals_);
   HYKKT_CUDA(cudaGetLastError());

@@ -322,6 +322,7 @@ class Engine {
   cudaStream_t begin_upload();
   void upload_all();
   void upload_border();
+  int factor_values_on(const double* vals_host, cudaStream_t st);
   void record_border_factor(cudaStream_t st);
   void record_schur_cg(cudaStream_t st);
   void record_border_solve(cudaStream_t st, const double* b, double* x, int use_stop, bool cg);

@@ -490,7 +490,9 @@ int hykkt_ruiz_scale_noalloc_max_rows(void);
  * given order: HYKKT_ORDER_IDENTITY). */
 typedef struct hykkt_chol_s* hykkt_chol_t;
 int hykkt_chol_create(hykkt_chol_t* c, int n, int nnz, const int* rowptr, const int* colidx, int ordering);
-/* numerical_factorization on host values (nnz, CSR order) */
+/* numerical_factorization on host values (nnz, CSR order); complete when it
+ * returns.  Where the GPU reaches pageable host memory it reads the array in
+ * place, else (or where the array is not aligned to doubles) through a copy. */
 int hykkt_chol_factor(hykkt_chol_t c, const double* vals);
 /* solve(x, b) on host vectors (n) */
 int hykkt_chol_solve(hykkt_chol_t c, double* x, const double* b);

@@ -30,3 +30,34 @@ def test_first_factor_reads_the_whole_entry_map(n):
         assert ch.factor(A[r, ci]) == hk.OK
         assert np.linalg.norm(ch.solve(b) - want) <= 1e-12 * np.linalg.norm(want)
         ch.close()
+
+
+@pytest.mark.parametrize("n", [33, 400])
+def test_unaligned_values(n):
+    """A view into a byte buffer, whatever its offset, gives the same bits as an
+    aligned array."""
+    rng = np.random.default_rng(n)
+    A, rp, ci, r = _lower(n, rng)
+    v = np.ascontiguousarray(A[r, ci])
+    b = rng.standard_normal(n)
+    ch = hk.Chol(n, rp, ci)
+    assert ch.factor(v) == hk.OK
+    x = ch.solve(b)
+    for off in (1, 4, 7, 8):
+        buf = np.zeros(v.nbytes + 16, np.uint8)
+        at = (off - buf.ctypes.data) % 8 + (8 if off == 8 else 0)
+        u = buf[at:at + v.nbytes].view(np.float64)
+        assert u.ctypes.data % 8 == off % 8
+        u[:] = v
+        assert ch.factor(u) == hk.OK
+        assert np.array_equal(ch.solve(b), x)
+
+
+def test_missing_values_are_refused():
+    rng = np.random.default_rng(1)
+    A, rp, ci, r = _lower(50, rng)
+    ch = hk.Chol(50, rp, ci)
+    assert hk.lib().hykkt_chol_factor(ch.h, None) == hk.INVALID
+    with pytest.raises(hk.HykktError):
+        ch.factor(A[r, ci][:-1])
+    assert ch.factor(A[r, ci]) == hk.OK
