@@ -11,6 +11,7 @@
 #include <fstream>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <sstream>
 #include <thread>
 #include <stdexcept>
@@ -159,6 +160,8 @@ extern "C" const char* hykkt_version(void) { return "hykkt_gb300 0.1 (sm_103a, F
 struct hykkt_plan_s {
   std::unique_ptr<Engine> eng;
   cudaStream_t stream = nullptr;
+  std::mutex queue_mu;
+  std::unique_ptr<Symbolic> queue;  // a bordered plan's task-queue layout, for its arrays (plan_array)
   ~hykkt_plan_s() {
     eng.reset();
     if (stream) cudaStreamDestroy(stream);
@@ -426,6 +429,7 @@ extern "C" int hykkt_plan_autotune(hykkt_plan_t plan, const double* h_vals, cons
       auto e = engine_like(base, options_for(base_opt, chosen));
       e->set_concurrency(share);
       plan->eng = std::move(e);
+      plan->queue.reset();
       info->from_cache = 1;
     } else {
       const double* v[8] = {h_vals, ds_vals, jc_vals, jd_vals, rx, rs, ry, ryd};
@@ -474,6 +478,7 @@ extern "C" int hykkt_plan_autotune(hykkt_plan_t plan, const double* h_vals, cons
       }
       best_eng->set_concurrency(share);
       plan->eng = std::move(best_eng);
+      plan->queue.reset();
       cache_store(cache_path, key, share, chosen, best_rate);
       info->best_solves_per_s = best_rate;
     }
@@ -903,18 +908,40 @@ extern "C" int hykkt_symbolic_get(hykkt_symbolic_t sym, const char* what, int* o
   });
 }
 
+// An array of a plan's analysis.  A plan of the bordered layout has none of
+// the supernode rows, solve items and tasks: those are analysed for the plan's
+// patterns and ordering when one of them is first asked for.
+static const std::vector<int>* plan_array(hykkt_plan_t plan, std::vector<int>& cp, std::vector<int>& ri,
+                                          const char* what) {
+  static const std::set<std::string> common = {"perm",  "etree", "colcount", "ht_rp",  "ht_ci",    "hg_rp",
+                                               "hg_ci", "lp_cp", "lp_row",   "sn_first", "L_cp",     "L_ri"};
+  const Symbolic& S = plan->eng->sym();
+  const std::string w(what);
+  if (!S.border.on || common.count(w) || (w.rfind("bd_", 0) == 0 && w != "bd_need")) return sym_array(S, cp, ri, what);
+  std::lock_guard<std::mutex> lk(plan->queue_mu);
+  if (!plan->queue) {
+    SymbolicOptions o = plan->eng->options();
+    o.bordered = false;
+    plan->queue = std::make_unique<Symbolic>(build_symbolic(S.H, S.Ds, S.Jc, S.Jd, o, S.perm.data()));
+  }
+  return sym_array(*plan->queue, cp, ri, what);
+}
+
 extern "C" int64_t hykkt_plan_symbolic_size(hykkt_plan_t plan, const char* what) {
-  static thread_local std::vector<int> cp, ri;
-  cp.clear();
-  ri.clear();
-  const std::vector<int>* a = sym_array(plan->eng->sym(), cp, ri, what);
-  return a ? (int64_t)a->size() : -1;
+  int64_t n = -1;
+  const int rc = guarded([&]() {
+    std::vector<int> cp, ri;
+    const std::vector<int>* a = plan_array(plan, cp, ri, what);
+    if (a) n = (int64_t)a->size();
+    return HYKKT_OK;
+  });
+  return rc == HYKKT_OK ? n : -1;
 }
 
 extern "C" int hykkt_plan_symbolic_get(hykkt_plan_t plan, const char* what, int* out, int64_t n) {
   return guarded([&]() {
     std::vector<int> cp, ri;
-    const std::vector<int>* a = sym_array(plan->eng->sym(), cp, ri, what);
+    const std::vector<int>* a = plan_array(plan, cp, ri, what);
     if (!a || n > (int64_t)a->size()) return fail(HYKKT_INVALID, std::string("unknown array or size: ") + what);
     std::copy(a->begin(), a->begin() + n, out);
     return HYKKT_OK;

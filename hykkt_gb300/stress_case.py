@@ -102,10 +102,9 @@ def main() -> None:
     out["solve_piece"] = a.solve_piece
     sz = plan.sizes()
     out.update(nnz_L=sz["nnz_L"], front_arena_doubles=sz["front_arena"], n_supernodes=sz["n_supernodes"])
-    sq_c0, sq_c1 = plan.symbolic("sq_c0"), plan.symbolic("sq_c1")
-    if len(sq_c0):  # task queues
-        out["widest_solve_item"] = int((sq_c1 - sq_c0).max())
     out["border_columns"] = len(plan.symbolic("bd_col"))
+    if not out["border_columns"]:  # task queues
+        out["widest_solve_item"] = int((plan.symbolic("sq_c1") - plan.symbolic("sq_c0")).max())
     out["widest_supernode"] = int(np.diff(plan.symbolic("sn_first")).max())
     # accuracy-mode solve through the graph
     plan.set_accuracy(a.cg_itmax, a.cg_rtol, a.refine_max, 1e-8)

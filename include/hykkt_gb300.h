@@ -425,7 +425,11 @@ void hykkt_symbolic_destroy(hykkt_symbolic_t sym);
  * "sn_parent", "sn_nrows", "sn_rows".  Returns the length (or -1). */
 int64_t hykkt_symbolic_size(hykkt_symbolic_t sym, const char* what);
 int hykkt_symbolic_get(hykkt_symbolic_t sym, const char* what, int* out, int64_t n);
-/* Same getters on a plan's symbolic part. */
+/* Same getters on a plan's symbolic part.  A plan of the bordered layout
+ * solves without supernode rows ("sn_parent", "sn_nrows", "sn_rows", ...);
+ * they are analysed when they are first asked for, as hykkt_symbolic_create_ex
+ * gives them for the plan's ordering.  The columns of its border are "bd_col"
+ * (empty for a plan of the task-queue layout). */
 int64_t hykkt_plan_symbolic_size(hykkt_plan_t plan, const char* what);
 int hykkt_plan_symbolic_get(hykkt_plan_t plan, const char* what, int* out, int64_t n);
 
