@@ -273,9 +273,9 @@ extern "C" int hykkt_plan_clone(hykkt_plan_t src, hykkt_plan_t* plan) {
 
 // ===========================================================================
 // Autotuner of the triangular-solve layout (no counterpart in the reference,
-// which leaves the factor and its solves to cuSOLVER).  The layout of the
-// solve items decides the solve's critical path and its FP64 work: whole
-// supernodes (shortest dependency chain, most inversion work) or pieces of
+// which leaves the factor and its solves to cuSOLVER).  The layout decides the
+// solve's critical path and its FP64 work: the bordered layout, or solve items
+// of whole supernodes (shortest dependency chain, most inversion work) or pieces of
 // the widest supernodes (less inversion work per factorization, more solve
 // stages), with or without warp-subtree tasks, and the multiply-adds of one
 // product task.  Which is fastest depends on the pattern and on how many
@@ -310,7 +310,11 @@ uint64_t pattern_key(const Symbolic& S) {
 
 struct TuneChoice {
   int solve_piece = 0, warp_subtree = 16, chunk_fma = 4096;
+  // kByEstimate: what a plan of that solve_piece takes (cache entries without a
+  // layout); the bordered layout has no items, its three numbers are 0
+  enum Layout { kByEstimate, kBordered, kQueues } layout = kByEstimate;
 };
+const TuneChoice kTuneBordered{0, 0, 0, TuneChoice::kBordered};
 
 bool cache_lookup(const char* path, uint64_t key, int share, TuneChoice& c) {
   if (!path || !*path) return false;
@@ -324,6 +328,10 @@ bool cache_lookup(const char* path, uint64_t key, int share, TuneChoice& c) {
     TuneChoice t;
     if (in >> std::hex >> k >> std::dec >> sh >> t.solve_piece >> t.warp_subtree >> t.chunk_fma && k == key &&
         sh == share) {
+      std::string rate, layout;
+      in >> rate >> layout;
+      if (layout == "bordered") t = kTuneBordered;
+      else if (layout == "queues") t.layout = TuneChoice::kQueues;
       c = t;
       found = true;  // the last entry for the key wins
     }
@@ -334,16 +342,23 @@ bool cache_lookup(const char* path, uint64_t key, int share, TuneChoice& c) {
 void cache_store(const char* path, uint64_t key, int share, const TuneChoice& c, double rate) {
   if (!path || !*path) return;
   std::ofstream f(path, std::ios::app);
-  f << std::hex << (unsigned long long)key << std::dec << " " << share << " " << c.solve_piece << " "
-    << c.warp_subtree << " " << c.chunk_fma << " " << rate << "\n";
+  const bool bordered = c.layout == TuneChoice::kBordered;
+  const TuneChoice t = bordered ? TuneChoice() : c;  // numbers that a reader without the layout word can use
+  f << std::hex << (unsigned long long)key << std::dec << " " << share << " " << t.solve_piece << " "
+    << t.warp_subtree << " " << t.chunk_fma << " " << rate << (bordered ? " bordered" : " queues") << "\n";
 }
 
 SymbolicOptions options_for(const SymbolicOptions& base, const TuneChoice& c) {
   SymbolicOptions o = base;
+  if (c.layout == TuneChoice::kBordered) {
+    o.solve_piece = 1 << 30;
+    o.bordered = border_allowed(0);
+    return o;
+  }
   o.solve_piece = c.solve_piece > 0 ? c.solve_piece : (1 << 30);
   o.warp_subtree = c.warp_subtree;
   o.chunk_fma = c.chunk_fma;
-  o.bordered = border_allowed(c.solve_piece);
+  o.bordered = c.layout == TuneChoice::kByEstimate && border_allowed(c.solve_piece);
   return o;
 }
 
@@ -363,8 +378,8 @@ std::unique_ptr<Engine> engine_like(const Engine& base, const SymbolicOptions& o
 
 // solves/s of `share` engines of one layout solving the sample at once
 // (fewer when device memory runs short; *used receives how many); 0 when a
-// solve failed
-double measure_layout(std::unique_ptr<Engine>& first, const double* const v[8], int share, int* used) {
+// solve failed.  Two rounds, the second only from half of `best` on.
+double measure_layout(std::unique_ptr<Engine>& first, const double* const v[8], int share, double best, int* used) {
   std::vector<std::unique_ptr<Engine>> es;
   es.push_back(std::move(first));
   size_t free_b = 0, total_b = 0;
@@ -396,10 +411,11 @@ double measure_layout(std::unique_ptr<Engine>& first, const double* const v[8], 
     };
     bool ok = round();  // warm-up: captures each engine's graph
     const auto t0 = std::chrono::steady_clock::now();
-    const int rounds = 2;
-    for (int r = 0; r < rounds && ok; ++r) ok = round();
-    const double sec = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-    rate = ok ? rounds * (double)es.size() / sec : 0.0;
+    for (int r = 1; r <= 2 && ok && (r == 1 || rate >= 0.5 * best); ++r) {
+      ok = round();
+      const double sec = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+      rate = ok ? r * (double)es.size() / sec : 0.0;
+    }
   } catch (...) {
     for (auto& s : st) cudaStreamDestroy(s);
     first = std::move(es[0]);
@@ -439,19 +455,26 @@ extern "C" int hykkt_plan_autotune(hykkt_plan_t plan, const double* h_vals, cons
       int widest = 0;
       const Symbolic& S = base.sym();
       for (size_t J = 0; J + 1 < S.sn_first.size(); ++J) widest = std::max(widest, S.sn_first[J + 1] - S.sn_first[J]);
+      const auto kQueues = TuneChoice::kQueues;
       std::vector<TuneChoice> cands;
-      cands.push_back({0, 16, 4096});  // whole supernodes, warp subtrees
-      cands.push_back({0, 0, 4096});   // whole supernodes, warp items one per warp
+      cands.push_back({0, 16, 4096, kQueues});  // whole supernodes, warp subtrees
+      cands.push_back({0, 0, 4096, kQueues});   // whole supernodes, warp items one per warp
       for (int piece : {2048, 2800, 4096})
-        if (piece < widest) cands.push_back({piece, 0, 4096});
+        if (piece < widest) cands.push_back({piece, 0, 4096, kQueues});
       int best = -1;
-      double best_rate = 0.0;
+      double best_rate = 0.0, best_queue = -1.0;
+      TuneChoice queue;  // the best of the task queues
       std::unique_ptr<Engine> best_eng;
       auto evaluate = [&](const TuneChoice& c) {
-        const int slot = info->candidates;
         auto e = engine_like(base, options_for(base_opt, c));
+        if (c.layout == TuneChoice::kBordered && !e->sym().border.on) return;  // the estimate keeps the queues
+        const int slot = info->candidates;
         int used = 0;
-        const double r = measure_layout(e, v, share, &used);
+        const double r = measure_layout(e, v, share, best_rate, &used);
+        if (c.layout == kQueues && r > best_queue) {
+          best_queue = r;
+          queue = c;
+        }
         if (slot < 8) {
           info->cand_piece[slot] = c.solve_piece;
           info->cand_subtree[slot] = c.warp_subtree;
@@ -467,10 +490,11 @@ extern "C" int hykkt_plan_autotune(hykkt_plan_t plan, const double* h_vals, cons
           best_eng = std::move(e);
         }
       };
+      if (border_allowed(0)) evaluate(kTuneBordered);
       for (const TuneChoice& c : cands) evaluate(c);
       if (best < 0) return fail(HYKKT_NOT_SPD, "autotune: no candidate layout solved the sample system");
-      // product-task size on the best layout
-      const TuneChoice layout = chosen;
+      // product-task size on the best of the queues
+      const TuneChoice layout = queue;
       for (int fma : {2048, 8192}) {
         TuneChoice c = layout;
         c.chunk_fma = fma;

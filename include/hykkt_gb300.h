@@ -185,7 +185,8 @@ int hykkt_plan_residency(hykkt_plan_t plan, int* resident, int64_t* bytes);
  * so that several systems of one sequence can be solved at once. */
 int hykkt_plan_clone(hykkt_plan_t src, hykkt_plan_t* plan);
 /* No counterpart in the reference.  Autotuner of the triangular-solve
- * layout for the plan's pattern: candidate layouts (whole supernodes with
+ * layout for the plan's pattern: candidate layouts (the bordered layout where
+ * a plan of the pattern takes it; then task queues: whole supernodes with
  * and without warp-subtree tasks, pieces of 2048 / 2800 / 4096 columns of
  * the widest supernodes, then 2048 / 8192 multiply-adds per product task on
  * the best of those) are built from the plan's own patterns and ordering;
@@ -203,7 +204,7 @@ typedef struct hykkt_tune_info {
   int concurrent;            /* engines solving at once while timing */
   int solve_piece;           /* chosen: most columns of one solve item (0 = whole supernodes) */
   int warp_subtree;          /* chosen: most warp items per subtree task (0 = none) */
-  int chunk_fma;             /* chosen: multiply-adds per product task */
+  int chunk_fma;             /* chosen: multiply-adds per product task (0 = the bordered layout) */
   double best_solves_per_s;  /* measured throughput of the chosen layout */
   int cand_piece[8], cand_subtree[8], cand_chunk_fma[8];
   double solves_per_s[8];    /* measured throughput of each candidate (0: a solve failed) */
