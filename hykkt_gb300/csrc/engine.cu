@@ -820,17 +820,23 @@ void Engine::record_border_factor(cudaStream_t st) {
     if (p + 1 == b.npan && !b.mc) break;
     const int rb = (p + 1) / 4;  // row blocks below the panel
     const int tri = nrb * (nrb + 1) / 2 - rb * (rb + 1) / 2;
-    if (tri >= 8 * sms_) LAUNCH(k_border_update<4>, tri, 256, kUpdateSmem, st, d, b, p);
-    else if (2 * tri >= 4 * sms_) LAUNCH(k_border_update<2>, 2 * tri, 256, kUpdateSmem, st, d, b, p);
+    const int run = tri >= 8 * sms_ ? 4 : 2 * tri >= 4 * sms_ ? 2 : 1;
+    if (run == 4) LAUNCH(k_border_update<4>, tri, 256, kUpdateSmem, st, d, b, p);
+    else if (run == 2) LAUNCH(k_border_update<2>, 2 * tri, 256, kUpdateSmem, st, d, b, p);
     else LAUNCH(k_border_update<1>, 4 * tri, 256, kUpdateSmem, st, d, b, p);
+    if (prof_) {
+      // entries that the panel's update changes: of the border's rows below the
+      // panel all up to the diagonal but the panel's, of the constraint rows the
+      // columns right of the panel; 32 multiply-adds, a read and a write each
+      const double lo = std::min((p + 1) * kBorderPanel, b.k), k = b.k, mc = b.mc;
+      const double n = (k * (k + 1) - lo * (lo + 1)) / 2 - kBorderPanel * (k - lo) + mc * (k - lo) + mc * (mc + 1) / 2;
+      prof_work(run == 4 ? "k_border_update<4>" : run == 2 ? "k_border_update<2>" : "k_border_update<1>",
+                2.0 * kBorderPanel * n, 16.0 * n);
+    }
   }
   const int nt = cdiv(b.k, 64);
   LAUNCH(k_border_pack, nt * (nt + 1) / 2, 256, 0, st, b);
   if (b.mc) LAUNCH(k_schur_pack, cdiv(b.mc, 64) * (cdiv(b.mc, 64) + 1) / 2, 256, 0, st, b);
-  if (prof_) {
-    const double k = b.k;
-    prof_work("k_border_update<4>", 2.0 / 3.0 * k * k * k, 16.0 / 3.0 * k * (k + 1) * b.npan);
-  }
 }
 
 // The whole CG run of a Schur plan, from the vectors that k_cg_setup leaves.
