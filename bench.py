@@ -52,6 +52,42 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
+def kernel_bound(name, flops, nbytes, fp64_tflops, hbm_gbs):
+    """"fp64" or "hbm": which of a kernel's two floors is the longer.  The border
+    update's products are digit products on the tensor cores, no FP64 work."""
+    if name.startswith("k_border_update"):
+        return "hbm"
+    return "fp64" if flops / (fp64_tflops * 1e12) > nbytes / (hbm_gbs * 1e9) else "hbm"
+
+
+def solve_work(prof, its, runs, m_c):
+    """Algorithmic work of one solve with `its` CG iterations in `runs` CG runs
+    (the first and one per refinement step), from the profile of one: FP64
+    operations, the factorization's operations, solve pairs, and the bytes of
+    the factor that the solves read.  None without a solve in the profile."""
+    if "k_trsv_fwd" in prof:
+        # factorization and inversion kernels as profiled, plus one forward +
+        # backward triangular solve per CG iteration and four more per CG run
+        fact = sum(v[2] for k, v in prof.items() if k.startswith(("k_front", "k_panel", "k_trtri", "k_piece")))
+        pair, b_pair = (sum(prof[k][i] / prof[k][0] for k in ("k_trsv_fwd", "k_trsv_bwd")) for i in (2, 3))
+        pairs = its + 4.0 * runs
+        return {"fp64": fact + pairs * pair, "factor": fact, "pairs": pairs, "solve_bytes": pairs * b_pair,
+                "note": "batched value x algorithmic FP64 work per solve"}
+    if "k_border_once" not in prof:
+        return None
+    # bordered layout: the factorization is digit products on the tensor cores;
+    # an iteration does one solve's products, or one with S where that is formed
+    fact = sum(v[2] for k, v in prof.items() if k.startswith("k_border_update"))
+    launches, _, flops, nbytes = prof["k_border_once"]
+    schur = any(k.startswith("k_schur_cg") for k in prof)
+    pairs = 2.0 * runs if schur else its + 4.0 * runs
+    rounds = its + 2.0 * runs if schur else 0.0
+    return {"fp64": pairs * flops / launches + rounds * 2.0 * m_c ** 2, "factor": fact, "pairs": pairs,
+            "solve_bytes": pairs * nbytes / launches + rounds * 8.0 * m_c ** 2,
+            "note": "batched value x algorithmic FP64 work of the solves; the factorization's products are digit "
+                    "products on the tensor cores"}
+
+
 METRIC = "KKT solves/s + p50/p99 latency at rel. residual <=1e-8, batched vs plain"
 
 
@@ -802,12 +838,13 @@ def main():
         tname = "dram_traffic_grid10k.json" if piece == 0 else f"dram_traffic_grid10k_piece{piece}.json"
         tpath = os.path.join(ROOT, "profiles", tname)
         if os.path.exists(tpath) and cfg["n_bus"] == 10000:
+            # captures of the task queues' kernels: none of the bordered layout's names
             tk = json.load(open(tpath))["kernels"].get(name)
             traffic = tk["dram_bytes_per_launch"] if tk else None
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))) if os.path.exists(
             os.path.join(ROOT, "MEASURED_PEAKS.json")) else {}
         hbm = peaks.get("hbm_gbs", 6800.0)
-        if flops > 0 and flops / max(nbytes, 1) > 0.3:
+        if kernel_bound(name, flops, nbytes, fp64, hbm) == "fp64":
             ach = flops / (ms / 1e3) / 1e12
             roof = {"bound": "fp64", "kernel": name, "achieved": ach, "peak": fp64, "unit": "TFLOP/s",
                     "frac": ach / fp64, "traffic": traffic, "launches": launches, "avg_launch_ms": ms / launches,
@@ -820,26 +857,19 @@ def main():
                     "launches": launches, "avg_launch_ms": ms / launches, "plan": "plain (alone on the GPU)",
                     "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6800 GB/s"}
     # whole-solve FP64 roofline of the batched run: algorithmic FP64 work of
-    # one solve (factorization and inversion kernels as profiled, plus one
-    # forward + backward triangular solve per CG iteration and four more per
-    # CG run) times batched solves/s, against the measured DFMA peak
+    # one solve times batched solves/s, against the measured DFMA peak
     roof_solve = None
-    if prof and "k_trsv_fwd" in prof:
-        f_fact = sum(v[2] for k, v in prof.items() if k.startswith(("k_front", "k_panel", "k_trtri", "k_piece")))
-        f_pair = prof["k_trsv_fwd"][2] / prof["k_trsv_fwd"][0] + prof["k_trsv_bwd"][2] / prof["k_trsv_bwd"][0]
-        ref_steps = float(np.mean([inf["refine_steps"] for inf in infos]))
-        pairs = float(np.mean(its_total)) + 4.0 * (1.0 + ref_steps)
-        f_solve = f_fact + pairs * f_pair
-        ach_t = f_solve * value / 1e12
-        # the triangular solves' algorithmic bytes per second over all
-        # concurrent plans (every stored entry of L read once per direction)
-        b_pair = prof["k_trsv_fwd"][3] / prof["k_trsv_fwd"][0] + prof["k_trsv_bwd"][3] / prof["k_trsv_bwd"][0]
-        agg = pairs * b_pair * value / 1e9
+    work = solve_work(prof, float(np.mean(its_total)), 1.0 + float(np.mean([inf["refine_steps"] for inf in infos])),
+                      systems[0].m_c)
+    if work:
+        ach_t = work["fp64"] * value / 1e12
+        # algorithmic bytes per second of the solves over all concurrent plans
+        # (every stored entry of the factor read once per direction)
+        agg = work["solve_bytes"] * value / 1e9
         roof_solve = {"bound": "fp64", "achieved": ach_t, "peak": fp64, "unit": "TFLOP/s", "frac": ach_t / fp64,
-                      "fp64_gflop_per_solve": f_solve / 1e9, "factor_gflop": f_fact / 1e9,
-                      "solve_pairs_per_solve": pairs, "note": "batched value x algorithmic FP64 work per solve",
-                      "trisolve_gbs_all_plans": agg,
-                      "trisolve_hbm_frac": agg / (roof["peak"] if roof and roof["unit"] == "GB/s" else 6800.0)}
+                      "fp64_gflop_per_solve": work["fp64"] / 1e9, "factor_gflop": work["factor"] / 1e9,
+                      "solve_pairs_per_solve": work["pairs"], "note": work["note"],
+                      "trisolve_gbs_all_plans": agg, "trisolve_hbm_frac": agg / hbm}
     kernels_per_solve = (info["kernels_per_solve"] + info["kernels_per_cg_iteration"] * info["cg_iterations_total"]
                          + info["kernels_per_refine_step"] * info["refine_steps"])
     cpu = None
@@ -850,8 +880,8 @@ def main():
             "metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": tot_ms / args.steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded grid generator, hykkt_gb300/gridgen.py)",
-            "config": dict(cfg, l2="256 MB flush before the timed region; every solve rewrites ~2 GB of its plan's "
-                              "factor storage (> L2) before reading it", plan_build_s=plan_s,
+            "config": dict(cfg, l2="256 MB flush before the timed region; every solve rewrites its plan's factor storage "
+                              "(10k grid: ~0.8 GB, > L2) before reading it", plan_build_s=plan_s,
                            step=f"{B} solves, one per plan, the plans concurrent (batched); plain: 1 solve"),
             "p50_ms": float(np.percentile(solve_ms, 50)), "p99_ms": float(np.percentile(solve_ms, 99)),
             "plain": {"value": plain_value, "unit": "solves/s", "p50_ms": float(np.percentile(plain_solve, 50)),
