@@ -1134,18 +1134,34 @@ __device__ __forceinline__ void sum_parts(const double* rrp, const double* dlp, 
 // The CG's recurrence after iteration `it` with the sums r.r and w.r.  Every
 // iteration waits for it, and a division is 20 dependent FP64 instructions, so
 // the divisions by the previous iteration's gamma and alpha are products with
-// reciprocals formed beside one another then.
+// reciprocals formed beside one another then.  Where
+// gamma_0 is below 2^-700 the sums are taken times the power of four near its
+// reciprocal (which changes no bit of alpha and beta): the reciprocal of a sum
+// below 2^-1024, or the square of a threshold below 2^-537, would leave the
+// range where a quotient and the root do not.  (The two products in every run
+// took 0.3 us of an iteration.)
 struct CgState {
-  double inv_gam, inv_alpha;
+  double inv_gam, inv_alpha;  // of the scaled gamma
 };
-__device__ __forceinline__ double cg_stop2(const DevPlan& d) {  // threshold on r.r
+struct CgScale {
+  double q, stop2;  // the power of four, the scaled r.r that stops
+  int on;           // q is not 1
+};
+__device__ __forceinline__ CgScale cg_scale(const DevPlan& d) {
   const DevScalars* S = d.sc;
-  const double thr = S->rtol_cur > 0.0 ? S->rtol_cur * sqrt(S->gam0) : d.cg_tol;
-  return thr * thr;
+  const double gam0 = S->gam0;
+  const int e = (int)((unsigned long long)__double_as_longlong(gam0) >> 52) & 0x7ff;
+  const int h = gam0 == 0.0 || e > 1023 - 700 ? 0 : (e - 1023) / 2;  // -511 <= h <= 0
+  const double thr = (S->rtol_cur > 0.0 ? S->rtol_cur * sqrt(gam0) : d.cg_tol) * pow2_or_nan(-h);
+  return CgScale{pow2_or_nan(-2 * h), thr * thr, h != 0};
 }
 // 0 go on, 1 converged, 2 iteration limit; sc = alpha, beta of the next iteration
-__device__ __forceinline__ int cg_step(const DevPlan& d, CgState& st, double stop2, double rr, double wr, int it, double* sc) {
-  if (rr < stop2 || rr == 0.0) return 1;
+__device__ __forceinline__ int cg_step(const DevPlan& d, CgState& st, const CgScale& cs, double rr, double wr, int it, double* sc) {
+  if (cs.on) {
+    rr *= cs.q;
+    wr *= cs.q;
+  }
+  if (rr < cs.stop2 || rr == 0.0) return 1;
   if (it + 1 >= d.cg_itmax) return 2;
   const double beta = rr * st.inv_gam, den = fma(-(beta * rr), st.inv_alpha, wr), inv = 1.0 / rr;
   sc[0] = rr / den;
@@ -1154,23 +1170,29 @@ __device__ __forceinline__ int cg_step(const DevPlan& d, CgState& st, double sto
   st.inv_alpha = den * inv;
   return 0;
 }
-// bd.scal: the threshold, then the state for the iterations of each parity
-__device__ __forceinline__ CgState cg_state(const DevPlan& d, const DevBorder& bd, int it) {
-  if (it == 0) return CgState{1.0 / d.sc->gam, 1.0 / d.sc->alpha};
-  return CgState{__ldcg(&bd.scal[1 + 2 * (it & 1)]), __ldcg(&bd.scal[2 + 2 * (it & 1)])};
+// bd.scal: the state for the iterations of each parity, the scale
+__device__ __forceinline__ CgScale cg_scale(const DevPlan& d, const DevBorder& bd, int it) {
+  if (it == 0) return cg_scale(d);
+  const double q = __ldcg(&bd.scal[4]);
+  return CgScale{q, __ldcg(&bd.scal[5]), q != 1.0};
 }
-// one thread: the step for good, its state, and at the end what the loop leaves,
-// through `ready`
-__device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, double rr, double wr, int it, int round, count_t* ready, count_t* done) {
+__device__ __forceinline__ CgState cg_state(const DevPlan& d, const DevBorder& bd, const CgScale& cs, int it) {
+  if (it == 0) return CgState{1.0 / (d.sc->gam * cs.q), 1.0 / d.sc->alpha};
+  return CgState{__ldcg(&bd.scal[2 * (it & 1)]), __ldcg(&bd.scal[2 * (it & 1) + 1])};
+}
+// one thread: the step for good from the state `st`, the next state, and at the
+// end what the loop leaves, through `ready`
+__device__ void cg_scalars(const DevPlan& d, const DevBorder& bd, const CgScale& cs, CgState st, double rr, double wr, int it, int round, count_t* ready, count_t* done) {
   DevScalars* S = d.sc;
   double sc[2];
-  CgState st = cg_state(d, bd, it);
-  const double stop2 = it ? __ldcg(&bd.scal[0]) : cg_stop2(d);
-  const int stop = cg_step(d, st, stop2, rr, wr, it, sc);
+  const int stop = cg_step(d, st, cs, rr, wr, it, sc);
   if (!stop) {
-    if (it == 0) bd.scal[0] = stop2;
-    bd.scal[1 + 2 * ((it + 1) & 1)] = st.inv_gam;
-    bd.scal[2 + 2 * ((it + 1) & 1)] = st.inv_alpha;
+    if (it == 0) {
+      bd.scal[4] = cs.q;
+      bd.scal[5] = cs.stop2;
+    }
+    bd.scal[2 * ((it + 1) & 1)] = st.inv_gam;
+    bd.scal[2 * ((it + 1) & 1) + 1] = st.inv_alpha;
   } else {
     S->gam1 = rr;
     S->delta = wr;
@@ -1199,9 +1221,10 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
   __shared__ double red[2 * 32];
   __shared__ int s_it, s_t, go[2], last;
   // the CG's scalars as this CTA has them: alpha and beta of iteration sc_it,
-  // the recurrence's state for iteration st_it, the threshold
-  __shared__ double sc2[2], s_stop2;
-  __shared__ CgState st2;
+  // the recurrence's state for iteration st_it, its scale
+  __shared__ double sc2[2];
+  __shared__ CgScale s_scale, last_scale;
+  __shared__ CgState st2, last_st;
   __shared__ int sc_it, st_it;
   if ((kCg || use_stop) && stopped_before(d.sc)) return;
   count_t* head = bd.ctl;
@@ -1270,20 +1293,24 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     // thread waits meanwhile for the scalars that the CTA of the last
     // constraint task left two iterations ago, which is nearly always over:
     // that CTA sums the parts after its task counts as done, and this
-    // iteration's tasks write the buffers it read.
+    // iteration's tasks write the buffers it read.  A CTA without a state of its
+    // own takes that one.
     auto wait_scalars = [&]() {
       if (!kCg || sc_it == it) return true;
-      const bool late = st_it != it;  // no state of its own: the last constraint task's
       if (threadIdx.x == 32) {
         go[0] = border_wait<false>(ready, (count_t)it - 1, done, d);
-        if (!go[0]) gave_up();
+        if (!go[0]) {
+          gave_up();
+        } else if (st_it != it) {
+          s_scale = cg_scale(d, bd, it - 1);
+          st2 = cg_state(d, bd, s_scale, it - 1);
+        }
       }
       if (!wait_for(&cnt[6 * kCtlStep], (count_t)it * tk.n[6], 0, &go[1]) || !go[0]) return false;
       sum_parts(bd.rrp + ((it - 1) & 1) * tk.n_upd, bd.dlp + ((it - 1) & 1) * tk.n[6], tk.n_upd, tk.n[6], red);
       if (threadIdx.x == 0) {
-        CgState st = late ? cg_state(d, bd, it - 1) : st2;
-        if (late) s_stop2 = it > 1 ? __ldcg(&bd.scal[0]) : cg_stop2(d);
-        go[1] = !cg_step(d, st, s_stop2, red[0], red[1], it - 1, sc2);
+        CgState st = st2;
+        go[1] = !cg_step(d, st, s_scale, red[0], red[1], it - 1, sc2);
         st2 = st;
         st_it = it + 1;
         sc_it = it;
@@ -1362,13 +1389,20 @@ __global__ void __launch_bounds__(256, 3) k_border_solve(DevPlan d, DevBorder bd
     }
     __syncthreads();
     if (!last) continue;
-    // the last constraint task: the step for good (k_spmv_jcp, k_cg_update),
-    // after the previous iteration's, whose state it starts from
-    sum_parts(bd.rrp + (it & 1) * tk.n_upd, bd.dlp + (it & 1) * tk.n[6], tk.n_upd, tk.n[6], red);
-    if (threadIdx.x == 0) {
-      if (border_wait<false>(ready, (count_t)it, done, d)) cg_scalars(d, bd, red[0], red[1], it, it + 1, ready, done);
-      else gave_up();
+    // the last constraint task: the step for good (k_spmv_jcp, k_cg_update).  A
+    // thread beside the sums' fetches the state that it starts from, once the
+    // previous iteration's step has left it.
+    if (threadIdx.x == 64) {
+      go[1] = border_wait<false>(ready, (count_t)it, done, d);
+      if (go[1]) {
+        last_scale = cg_scale(d, bd, it);
+        last_st = cg_state(d, bd, last_scale, it);
+      } else {
+        gave_up();
+      }
     }
+    sum_parts(bd.rrp + (it & 1) * tk.n_upd, bd.dlp + (it & 1) * tk.n[6], tk.n_upd, tk.n[6], red);
+    if (threadIdx.x == 0 && go[1]) cg_scalars(d, bd, last_scale, last_st, red[0], red[1], it, it + 1, ready, done);
   }
 }
 
@@ -1420,8 +1454,9 @@ template <int RB>
 __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, int tasks) {
   extern __shared__ __align__(128) double sm[];  // destination of bulk copies
   __shared__ double red[2];
-  __shared__ double sc2[2], s_stop2;  // as in k_border_solve
-  __shared__ CgState st2;
+  __shared__ double sc2[2];  // as in k_border_solve
+  __shared__ CgScale s_scale, last_scale;
+  __shared__ CgState st2, last_st;
   __shared__ int s_it, s_t, st_it, go[2], last;
   __shared__ __align__(8) uint64_t bars[2 * kStages];
   DevScalars* S = d.sc;
@@ -1471,7 +1506,12 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
       }
     } else if (threadIdx.x == 32) {
       go[1] = !own_step || border_wait<false>(ready, (count_t)q - 1, done, d);
-      if (!go[1]) gave_up();
+      if (!go[1]) {
+        gave_up();
+      } else if (own_step && st_it != q) {
+        s_scale = cg_scale(d, bd, q - 3);
+        st2 = cg_state(d, bd, s_scale, q - 3);
+      }
     }
     __syncthreads();
     bool on = go[0] && go[1];
@@ -1479,10 +1519,8 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
       const int old = ((q - 1) & 1) * tasks;
       sum_parts(bd.rrp + old, bd.dlp + old, tasks, tasks, red);
       if (threadIdx.x == 0) {
-        const bool late = st_it != q;
-        CgState st = late ? cg_state(d, bd, q - 3) : st2;
-        if (late) s_stop2 = q > 3 ? __ldcg(&bd.scal[0]) : cg_stop2(d);
-        go[0] = !cg_step(d, st, s_stop2, red[0], red[1], q - 3, sc2);
+        CgState st = st2;
+        go[0] = !cg_step(d, st, s_scale, red[0], red[1], q - 3, sc2);
         st2 = st;
         st_it = q + 1;
       }
@@ -1552,12 +1590,19 @@ __global__ void __launch_bounds__(256, 3) k_schur_cg(DevPlan d, DevBorder bd, in
     }
     __syncthreads();
     if (!last) continue;
+    if (q > 1 && threadIdx.x == 64) {  // as in k_border_solve
+      go[1] = border_wait<false>(ready, (count_t)q, done, d);
+      if (go[1]) {
+        last_scale = cg_scale(d, bd, q - 2);
+        last_st = cg_state(d, bd, last_scale, q - 2);
+      } else {
+        gave_up();
+      }
+    }
     sum_parts(bd.rrp + (q & 1) * tasks, bd.dlp + (q & 1) * tasks, tasks, tasks, red);
     if (threadIdx.x == 0) {
       if (q > 1) {
-        // after the previous round's step, whose state it starts from
-        if (border_wait<false>(ready, (count_t)q, done, d)) cg_scalars(d, bd, red[0], red[1], q - 2, q + 1, ready, done);
-        else gave_up();
+        if (go[1]) cg_scalars(d, bd, last_scale, last_st, red[0], red[1], q - 2, q + 1, ready, done);
       } else {
         if (q == 0) {
           S->gam = S->gam0 = red[0];

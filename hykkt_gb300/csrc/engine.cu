@@ -660,7 +660,7 @@ void Engine::upload_border() {
   b.S = dev_alloc<double>(A, B, (int64_t)cdiv(b.mc, b.srb) * b.srb * b.mc);
   b.rrp = dev_alloc<double>(A, B, 2 * std::max(nm, cdiv(b.mc, b.srb)));
   b.dlp = dev_alloc<double>(A, B, 2 * std::max(cdiv(S_.m_c, kRowTask), cdiv(b.mc, b.srb)));
-  b.scal = dev_alloc<double>(A, B, 5);
+  b.scal = dev_alloc<double>(A, B, 6);
   b.ctl = dev_alloc<unsigned long long>(A, B, kCtlWords);
   // blocks by front size, so that small fronts share an SM
   blk_class_.assign(1, 0);

@@ -199,7 +199,7 @@ struct DevBorder {
   double* S;             // Schur plans: S in panels of srb rows
   int srb;
   double *rrp, *dlp;     // CG partial sums of two iterations
-  double* scal;          // CG: the squared residual that stops; 1/gamma, 1/alpha of two iterations
+  double* scal;          // CG: 1/gamma, 1/alpha of two iterations; their scale
   unsigned long long* ctl;  // task counters of one launch
 };
 
