@@ -4,7 +4,7 @@ Workload (default): 20 same-sparsity FP64 KKT systems on a synthetic
 10,000-bus grid (n_x = 24,000, m_c = 20,000, m_d = 28,000; gamma = 1e5;
 D_x, D_s log-uniform in [1e-10, 1e8]; seeded).  A solve = one full KKT
 solve of a system of the sequence (upload of the values, H~, Ruiz, Hgamma,
-multifrontal Cholesky, Schur CG, recovery, 4-block residual); the symbolic
+Cholesky, Schur CG, recovery, 4-block residual); the symbolic
 plan is built once before timing, as the reference does on its first
 execute().
 

@@ -654,7 +654,11 @@ void Engine::upload_border() {
   b.r2 = dev_alloc<double>(A, B, S_.m_c);
   b.s2 = dev_alloc<double>(A, B, S_.m_c);
   // Schur plans: four rows a task up to 640 constraints, else eight (a task
-  // forms the whole residual, which fewer rows repeat more often)
+  // forms the whole residual, which fewer rows repeat more often).  Solves with
+  // some 500 iterations, four and eight rows: 400 constraints 2.23 and 2.22 ms,
+  // 560 3.72 and 3.38, 640 4.65 and 4.45, 720 5.75 and 5.17, 840 7.08 and 7.03,
+  // 1,000 7.23 and 7.13, 1,200 11.7 and 10.8; with 140 iterations 400
+  // constraints 1.94 and 2.27, 200 1.48 either way.
   b.srb = S_.m_c <= 640 ? 4 : 8;
   b.w2 = dev_alloc<double>(A, B, b.mc);
   b.S = dev_alloc<double>(A, B, (int64_t)cdiv(b.mc, b.srb) * b.srb * b.mc);

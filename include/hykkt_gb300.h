@@ -213,8 +213,9 @@ int hykkt_plan_autotune(hykkt_plan_t plan, const double* h_vals, const double* d
                         const double* jd_vals, const double* rx, const double* rs, const double* ry,
                         const double* ryd, int share, const char* cache_path, hykkt_tune_info* info);
 /* No counterpart in the reference.  `share` = number of plans that solve
- * concurrently on this GPU: the plan's persistent triangular-solve kernels
- * take 1/share of the GPU's CTA slots (at least one per SM).  Default 1. */
+ * concurrently on this GPU: the plan's solve and CG kernels take 1/share of
+ * the GPU's CTA slots (at least 16 CTAs).  Default 1: plans that solve at once
+ * with it ask for the whole GPU each, and their CTAs start as others end. */
 int hykkt_plan_set_concurrency(hykkt_plan_t plan, int share);
 /* One numeric solve (the numeric phase of HykktSolver::execute,
  * HykktSolver.cpp:252-285).  values_on_device = 0: the ten arrays are host
